@@ -1,5 +1,6 @@
 // api.cu - context management and the C-ABI entry points of include/adda_gb300.h.
 #include "ctx.cuh"
+#include "fft_lines2.cuh"
 
 #include <cstdio>
 
@@ -60,6 +61,44 @@ FftPlan make_plan(int n, int max_radix)
 	return p;
 }
 
+// both radices at most RADIX_MAX, as equal as possible; the first pass skips the zero half of a padded line, which
+// an even radix does exactly
+Plan2 make_plan2(int n)
+{
+	Plan2 p{n, 0, 0};
+	int best = 1 << 30;
+	for (int a = 1; a <= RADIX_MAX; a++) {
+		if (n % a || n / a > RADIX_MAX) continue;
+		const int b = n / a, cost = 4 * (a + b) + (a % 2 ? 2 : 0) + (a < b ? 1 : 0);
+		if (cost < best) {
+			best = cost;
+			p.r1 = a;
+			p.r2 = b;
+		}
+	}
+	return p;
+}
+
+// tables that go to the device in one allocation and one copy
+struct Blob {
+	std::vector<unsigned char> bytes;
+	std::vector<std::pair<void **, size_t>> at;
+	template <typename T> void add(T **dev, const std::vector<T> &v)
+	{
+		at.emplace_back((void **)dev, bytes.size());
+		const size_t n = sizeof(T) * v.size();
+		bytes.resize(bytes.size() + (n + 255) / 256 * 256);
+		std::memcpy(bytes.data() + at.back().second, v.data(), n);
+	}
+	int upload(void **base)
+	{
+		ADDA_CUDA(cudaMalloc(base, bytes.size()));
+		ADDA_CUDA(cudaMemcpy(*base, bytes.data(), bytes.size(), cudaMemcpyHostToDevice));
+		for (auto &a : at) *a.first = (unsigned char *)*base + a.second;
+		return ADDA_GB300_OK;
+	}
+};
+
 } // namespace adda
 
 using namespace adda;
@@ -84,7 +123,7 @@ int adda_gb300_get_grid(const adda_gb300_ctx *c, int grid[3])
 // n-th roots of unity of one axis. The FP32 table has a second part of n entries for the register FFT of the y
 // transform (reg_fft, power-of-two n = T*E up to 512): W_n^(j1*k2) at k2*T + j1, so that the T lanes of a line read
 // their step-1 twiddles from consecutive addresses.
-static int upload_twiddles(adda_gb300_ctx *c, int which, int n)
+static void add_twiddles(adda_gb300_ctx *c, Blob &b, int which, int n)
 {
 	std::vector<double2> t64(n);
 	std::vector<float2> t32(2 * (size_t)n, make_float2(0.f, 0.f));
@@ -104,11 +143,41 @@ static int upload_twiddles(adda_gb300_ctx *c, int which, int n)
 	}
 	for (int k2 = 0; T && k2 < n / T; k2++)
 		for (int j1 = 0; j1 < T; j1++) t32[n + (size_t)k2 * T + j1] = t32[(size_t)j1 * k2 % n];
-	ADDA_CUDA(cudaMalloc(&c->tw64[which], sizeof(double2) * n));
-	ADDA_CUDA(cudaMalloc(&c->tw32[which], sizeof(float2) * 2 * (size_t)n));
-	ADDA_CUDA(cudaMemcpy(c->tw64[which], t64.data(), sizeof(double2) * n, cudaMemcpyHostToDevice));
-	ADDA_CUDA(cudaMemcpy(c->tw32[which], t32.data(), sizeof(float2) * 2 * (size_t)n, cudaMemcpyHostToDevice));
-	return ADDA_GB300_OK;
+	b.add(&c->tw64[which], t64);
+	b.add(&c->tw32[which], t32);
+}
+
+// twiddles of the two-pass transforms: W_n^(j*q) at [q*r2 + j], and for the y axis also at [j*r1 + q] (its inverse runs
+// the radices in the other order). Fixed point: scaled by 2^(64 - shift), as signed halves (low halves above -2^31, so
+// that they can be negated)
+static void add_twiddles2(adda_gb300_ctx *c, Blob &b, int which, bool fx)
+{
+	const Plan2 &p = c->p2[which];
+	const double scale = std::ldexp(1.0, 64 - fx_shift(p.n));
+	std::vector<float2> tf[2];
+	std::vector<int4> tx[2];
+	for (int o = 0; o < (which == 1 ? 2 : 1); o++) {
+		tf[o].resize(p.n);
+		tx[o].resize(p.n);
+		for (int q = 0; q < p.r1; q++)
+			for (int j = 0; j < p.r2; j++) {
+				double cs, sn;
+				unit_root((long)q * j, p.n, cs, sn);
+				const int at = o ? j * p.r1 + q : q * p.r2 + j;
+				tf[o][at] = make_float2((float)cs, (float)sn);
+				int h[4];
+				for (int k = 0; k < 2; k++) {
+					const long long v = std::llrint((k ? sn : cs) * scale);
+					const int lo = std::max((int)(unsigned)(v & 0xffffffffll), -0x7fffffff);
+					h[2 * k] = (int)((v - lo + 1) >> 32);
+					h[2 * k + 1] = lo;
+				}
+				tx[o][at] = make_int4(h[0], h[1], h[2], h[3]);
+			}
+		const int slot = o ? 3 : which;
+		b.add(&c->tw2f[slot], tf[o]);
+		if (fx) b.add(&c->tw2x[slot], tx[o]);
+	}
 }
 
 // one particle's lattice inside the context's box
@@ -192,6 +261,7 @@ static int create_impl(const adda_gb300_problem *p, adda_gb300_ctx *c, const std
 	}
 	const int g3[3] = {c->gX, c->gY, c->gZ};
 	FftPlan *pl[3] = {c->px, c->py, c->pz};
+	Blob tables;
 	for (int d = 0; d < 3; d++) {
 		pl[d][0] = make_plan(g3[d], 8);
 		pl[d][1] = make_plan(g3[d], 16);
@@ -199,9 +269,14 @@ static int create_impl(const adda_gb300_problem *p, adda_gb300_ctx *c, const std
 			set_error("FFT grid sizes must factor into 2,3,5,7,11,13");
 			return ADDA_GB300_EINVAL;
 		}
-		int rc = upload_twiddles(c, d, g3[d]);
-		if (rc) return rc;
+		add_twiddles(c, tables, d, g3[d]);
 	}
+	for (int d = 0; d < 3; d++) c->p2[d] = make_plan2(g3[d]);
+	c->fx = !c->surface && c->p2[0].r1 && c->p2[1].r1 && c->p2[2].r1;
+	for (int d = 0; d < 3; d++)
+		if (c->p2[d].r1) add_twiddles2(c, tables, d, c->fx);
+	int rc = tables.upload(&c->tables);
+	if (rc) return rc;
 	// lattices: check order (z, y, x ascending), build per-line dipole ranges. Particle q of a group occupies slot q
 	// of every lattice array: line starts [q][bZ*bY+1] (indices into its own dipoles), xy/material [q][N], positions
 	// [q][N][3], N the largest particle (the other slots padded with zeros)
@@ -262,6 +337,14 @@ static int create_impl(const adda_gb300_problem *p, adda_gb300_ctx *c, const std
 	const size_t dlen = (size_t)c->gX * c->DsZ * c->DsY * 6;
 	ADDA_CUDA(cudaMalloc(&c->D64, sizeof(double2) * dlen));
 	ADDA_CUDA(cudaMalloc(&c->D32, sizeof(float2) * dlen));
+	if (c->fx) {
+		ADDA_CUDA(cudaMalloc(&c->Dfx, sizeof(int4) * dlen));
+		// every top below every exponent (each byte 0x80: far below FX_LOW), as each matvec leaves them
+		const size_t ne = fx_exps_ints(c);
+		ADDA_CUDA(cudaMalloc(&c->fx_exps, sizeof(int) * (ne + (size_t)c->gX * c->DsZ)));
+		ADDA_CUDA(cudaMemset(c->fx_exps, 0x80, sizeof(int) * ne));
+		c->fx_eD = c->fx_exps + ne;
+	}
 	if (c->surface) {
 		const size_t rlen = (size_t)c->gX * c->gZ * (c->gY / 2 + 1) * 6;
 		ADDA_CUDA(cudaMalloc(&c->R64, sizeof(double2) * rlen));
@@ -304,8 +387,7 @@ static int create_impl(const adda_gb300_problem *p, adda_gb300_ctx *c, const std
 	}
 	c->cc_set.assign(R, 0);
 	c->nmat = 0;
-	int rc = matvec_setup(c);
-	if (rc) return rc;
+	if ((rc = matvec_setup(c))) return rc;
 	// ADDA_GB300_FFT_SHAPE="w1,w2,pairs,nt" fixes the FP32 tile shape (no tuning of it)
 	if (const char *e = getenv("ADDA_GB300_FFT_SHAPE")) {
 		int v[4];
@@ -323,7 +405,7 @@ int adda_gb300_destroy(adda_gb300_ctx *c)
 	solver_free(c);
 	void *bufs[] = {c->d_line_start, c->d_xy, c->d_mat, c->d_pos, c->D64, c->D32, c->cc64, c->ccs64, c->ccs32,
 		c->Xf, c->Tz, c->TzR, c->Tz2, c->TzR2, c->R64, c->R32, c->partial, c->d_red, c->vin, c->vout, c->pvec64,
-		c->tw64[0], c->tw64[1], c->tw64[2], c->tw32[0], c->tw32[1], c->tw32[2]};
+		c->tables, c->Dfx, c->fx_exps};
 	if (c->stream2) cudaStreamSynchronize(c->stream2);
 	for (void *b : bufs)
 		if (b) cudaFree(b);

@@ -360,6 +360,12 @@ struct FftPlan {
 	int r[ADDA_FFT_MAXPASS];
 };
 
+// n = r1*r2 of the two-pass line transforms (fft_lines2.cuh; make_plan2 in api.cu); r1 = 0: no such factors
+constexpr int RADIX_MAX = 16;
+struct Plan2 {
+	int n, r1, r2;
+};
+
 // multiply by exp(s*i*theta) given c=cos(theta), s_=s*sin(theta)
 template <typename C> __device__ __forceinline__ C crot(C v, double c, double s_)
 {

@@ -91,6 +91,16 @@ struct adda_gb300_ctx {
 	adda::FftPlan px[2], py[2], pz[2];
 	double2 *tw64[3] = {nullptr, nullptr, nullptr};
 	float2 *tw32[3] = {nullptr, nullptr, nullptr};
+	// two-pass transforms (fft_lines2.cuh): radices and twiddles per axis (x, y, z; [3] the y axis's inverse order)
+	adda::Plan2 p2[3] = {};
+	float2 *tw2f[4] = {nullptr, nullptr, nullptr, nullptr};
+	int4 *tw2x[4] = {nullptr, nullptr, nullptr, nullptr};
+	// FP64 matvec in 64-bit fixed point: all three axes have two-pass plans and there is no substrate
+	bool fx = false;
+	void *Dfx = nullptr;    // D in fixed point, [gX][DsZ][DsY][6]
+	int *fx_exps = nullptr; // exponents of the data between the kernels (matvec_lines2.cuh: FxExp)
+	int *fx_eD = nullptr;   // exponents of Dfx's rows [gX][DsZ] (behind them)
+	void *tables = nullptr; // the allocation behind the twiddle tables
 	// interaction matrix, reduced layout [gX][DsZ][DsY][6]
 	double2 *D64 = nullptr;
 	float2 *D32 = nullptr;
@@ -135,9 +145,14 @@ namespace adda {
 
 // plan.cpp-equivalent helpers (api.cu)
 FftPlan make_plan(int n, int max_radix);
+Plan2 make_plan2(int n);
 
 // dmatrix.cu
 int dmatrix_build(adda_gb300_ctx *c);
+
+// matvec_lines2.cu
+size_t fx_exps_ints(const adda_gb300_ctx *c); // ints of fx_exps
+int fx_dmatrix(adda_gb300_ctx *c);            // D64 -> Dfx, fx_eD
 
 // matvec.cu
 int matvec_setup(adda_gb300_ctx *c); // tile shapes, kernel attributes

@@ -5,6 +5,10 @@
 namespace adda {
 
 int matvec_setup_f32(adda_gb300_ctx *c); // matvec_f32.cu
+namespace mv {
+int l2_setup_yz(); // matvec_lines2.cu
+int l2_setup_x();  // matvec_lines2_x.cu
+} // namespace mv
 
 namespace {
 
@@ -27,7 +31,7 @@ __global__ void reduce_partials_k(const double *partial, size_t nblk, double *ou
 size_t matvec_partial_blocks(const adda_gb300_ctx *c, bool dbl)
 {
 	// K3 grid: ceil(bY/w1) x bZ blocks per RHS
-	const int w = c->shape[dbl ? 0 : 1].w1;
+	const int w = dbl && mv::use_fx(c) ? mv::FX_W1 : c->shape[dbl ? 0 : 1].w1;
 	return (size_t)((c->bY + w - 1) / w) * c->bZ;
 }
 
@@ -52,7 +56,9 @@ int matvec_setup(adda_gb300_ctx *c)
 		return ADDA_GB300_EINVAL;
 	}
 	int rc = mv::set_attrs_tv<double, double2>();
-	if (rc || (rc = mv::setup_yz<double>()) || (rc = mv::setup_yz<float>())) return rc;
+	if (rc || (rc = mv::setup_yz<double>()) || (rc = mv::setup_yz<float>()) || (rc = mv::l2_setup_yz()) ||
+		(rc = mv::l2_setup_x()))
+		return rc;
 	return matvec_setup_f32(c);
 }
 

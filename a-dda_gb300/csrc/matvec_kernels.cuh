@@ -29,6 +29,7 @@
 #include "ctx.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace adda {
 namespace mv {
@@ -617,6 +618,59 @@ __device__ __forceinline__ double block_sum(double v, double *sh)
 	return s; // valid in thread 0
 }
 
+// y = x + S.X for the dipoles of W x-lines (one z) whose X stands in a tile (element x of line comp*W + y is
+// o(x*LS + line)), with the epilogue reductions; every thread of the block calls it
+template <typename T, typename V, int W, typename P, typename O>
+__device__ __forceinline__ void gather_lines(const P &p, const MvEpi &e, O o, int LS, int r, int z, int y0, int wy, int NT,
+	double *red)
+{
+	typedef typename CxT<T>::type C;
+	// the lattice of RHS r's particle (a single-lattice context has one)
+	const size_t lq = (size_t)(r / p.rpp);
+	const uint32_t *lstart = p.line_start + lq * ((size_t)p.bZ * p.bY + 1), *lxy = p.xy + lq * p.lat_stride;
+	const uint8_t *lmat = p.mat + lq * p.lat_stride;
+	const size_t line = (size_t)z * p.bY + y0;
+	const uint32_t i0 = lstart[line], i1 = lstart[line + wy];
+	const V *arg = p.arg + (size_t)r * p.N * 3;
+	V *res = p.res + (size_t)r * p.N * 3;
+	const V *u = e.u ? reinterpret_cast<const V *>(e.u) + (size_t)r * p.N * 3 : nullptr;
+	typename AccOf<V>::T s0{}, s1r{}, s1i{};
+	for (uint32_t i = i0 + threadIdx.x; i < i1; i += NT) {
+		const uint32_t q = lxy[i];
+		const int x = q & 0xffff, y = q >> 16;
+		const uint8_t m = lmat[i];
+#pragma unroll
+		for (int comp = 0; comp < 3; comp++) {
+			const size_t j = (size_t)i * 3 + comp;
+			const V x0 = arg[j];
+			const V xv = p.her ? cconj(x0) : x0;
+			const C sx = cmul(ccs_of(p.ccs, p.per_dip, p.nmat, p.N, r, i, m, comp), o(x * LS + comp * W + (y - y0)));
+			V yv = cadd(xv, cvt<V>(sx));
+			if (p.her) yv = cconj(yv);
+			res[j] = yv;
+			if (e.mode) {
+				if (e.mode & EPI_NORM) acc_abs2(s0, yv);
+				if (e.mode & EPI_DOT_ARG) acc_cmul(s1r, s1i, x0, yv);      // x.y
+				if (e.mode & EPI_DOT_ARG_CONJ) acc_cmulc(s1r, s1i, x0, yv); // x.y*
+				if (e.mode & EPI_DOT_U_CONJ) acc_cmulc(s1r, s1i, yv, u[j]);  // y.u*
+			}
+		}
+	}
+	if (e.mode) {
+		const size_t nblk = (size_t)gridDim.x * gridDim.y;
+		const size_t blk = (size_t)blockIdx.y * gridDim.x + blockIdx.x;
+		double *out = e.partial + ((size_t)r * nblk + blk) * 4;
+		double v0 = block_sum(acc_val(s0), red);
+		double v1 = block_sum(acc_val(s1r), red);
+		double v2 = block_sum(acc_val(s1i), red);
+		if (threadIdx.x == 0) {
+			out[0] = v0;
+			out[1] = v1;
+			out[2] = v2;
+		}
+	}
+}
+
 // K3: inverse FFT along x of W y-lines (one z), then y = x + S.X for their dipoles, with the epilogue reductions.
 template <typename T, typename V, int W, int NS>
 __global__ void __launch_bounds__(col_threads<T, NS, 3 * W>(), (col_minblocks<T, NS, 3 * W>()))
@@ -632,10 +686,6 @@ __global__ void __launch_bounds__(col_threads<T, NS, 3 * W>(), (col_minblocks<T,
 	C *a = reinterpret_cast<C *>(smem_raw);
 	C *b = a + (size_t)n * LS;
 	const int r = blockIdx.z, z = blockIdx.y, y0 = blockIdx.x * W;
-	// the lattice of RHS r's particle (a single-lattice context has one)
-	const size_t lq = (size_t)(r / p.rpp);
-	const uint32_t *lstart = p.line_start + lq * ((size_t)p.bZ * p.bY + 1), *lxy = p.xy + lq * p.lat_stride;
-	const uint8_t *lmat = p.mat + lq * p.lat_stride;
 	const int wy = min(W, p.bY - y0);
 	const size_t plane = (size_t)p.bZ * p.bY;
 	const C *xf = p.Xf + (size_t)r * p.gX * 3 * plane + (size_t)z * p.bY + y0;
@@ -671,46 +721,7 @@ __global__ void __launch_bounds__(col_threads<T, NS, 3 * W>(), (col_minblocks<T,
 		__syncthreads();
 		o = tile_fft<C, NS, NL, LS, true>(a, b, p.px, p.twx);
 	}
-	const size_t line = (size_t)z * p.bY + y0;
-	const uint32_t i0 = lstart[line], i1 = lstart[line + wy];
-	const V *arg = p.arg + (size_t)r * p.N * 3;
-	V *res = p.res + (size_t)r * p.N * 3;
-	const V *u = e.u ? reinterpret_cast<const V *>(e.u) + (size_t)r * p.N * 3 : nullptr;
-	typename AccOf<V>::T s0{}, s1r{}, s1i{};
-	for (uint32_t i = i0 + threadIdx.x; i < i1; i += NT) {
-		const uint32_t q = lxy[i];
-		const int x = q & 0xffff, y = q >> 16;
-		const uint8_t m = lmat[i];
-#pragma unroll
-		for (int comp = 0; comp < 3; comp++) {
-			const size_t j = (size_t)i * 3 + comp;
-			const V x0 = arg[j];
-			const V xv = p.her ? cconj(x0) : x0;
-			const C sx = cmul(ccs_of(p.ccs, p.per_dip, p.nmat, p.N, r, i, m, comp), o[x * LS + comp * W + (y - y0)]);
-			V yv = cadd(xv, cvt<V>(sx));
-			if (p.her) yv = cconj(yv);
-			res[j] = yv;
-			if (e.mode) {
-				if (e.mode & EPI_NORM) acc_abs2(s0, yv);
-				if (e.mode & EPI_DOT_ARG) acc_cmul(s1r, s1i, x0, yv);      // x.y
-				if (e.mode & EPI_DOT_ARG_CONJ) acc_cmulc(s1r, s1i, x0, yv); // x.y*
-				if (e.mode & EPI_DOT_U_CONJ) acc_cmulc(s1r, s1i, yv, u[j]);  // y.u*
-			}
-		}
-	}
-	if (e.mode) {
-		const size_t nblk = (size_t)gridDim.x * gridDim.y;
-		const size_t blk = (size_t)blockIdx.y * gridDim.x + blockIdx.x;
-		double *out = e.partial + ((size_t)r * nblk + blk) * 4;
-		double v0 = block_sum(acc_val(s0), red);
-		double v1 = block_sum(acc_val(s1r), red);
-		double v2 = block_sum(acc_val(s1i), red);
-		if (threadIdx.x == 0) {
-			out[0] = v0;
-			out[1] = v1;
-			out[2] = v2;
-		}
-	}
+	gather_lines<T, V, W>(p, e, [&](int i) { return o[i]; }, LS, r, z, y0, wy, NT, red);
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -850,21 +861,62 @@ template <typename T> int setup_yz()
 	return ADDA_GB300_OK;
 }
 
+// the stages on two-pass transforms (matvec_lines2.cuh, compiled in matvec_lines2*.cu; measured there against the
+// kernels above, which stay for what they do not cover: axes without a two-pass plan, substrates in FP64, the narrow
+// widths of long axes).
+// FP64: all stages in fixed point when the context has the plans and the default tile widths, in place of which the
+// fixed-point kernels have their own: FX_W1 y-lines per K1/K3 block, FX_W2 per K2a/K2c block.
+constexpr int FX_W1 = 2, FX_W2 = 8;
+inline bool use_fx(const adda_gb300_ctx *c)
+{
+	return c->fx && c->shape[0].w1 == Tiles<double>::W1 && c->shape[0].w2 == Tiles<double>::W2;
+}
+// FP32: each stage whose axis has no compile-time kernel (those are faster: 256^3 0.68 ms) but a two-pass plan
+inline bool use_l2_f32(const adda_gb300_ctx *c, int axis, int n) { return static_len(n) == 0 && c->p2[axis].r1 > 0; }
+inline bool use_l2_x(const adda_gb300_ctx *c, const MvShape &s) { return use_l2_f32(c, 0, c->gX) && s.w1 >= 4; }
+inline bool use_l2_z(const adda_gb300_ctx *c, const MvShape &s) { return use_l2_f32(c, 2, c->gZ) && s.w2 >= 8; }
+inline bool use_l2_y(const adda_gb300_ctx *c) { return use_l2_f32(c, 1, c->gY) && !c->surface; }
+int l2_fftz_run(adda_gb300_ctx *c, const MvGeom<float> &p, int mode, int w2, dim3 g, cudaStream_t st);
+int l2_ffty_run(adda_gb300_ctx *c, const MvGeom<float> &p, int ck, int pairs, cudaStream_t st);
+template <typename V> int l2_scatter_run(adda_gb300_ctx *c, const MvP<float, V> &p, int w1, dim3 g, cudaStream_t st);
+template <typename V>
+int l2_gather_run(adda_gb300_ctx *c, const MvP<float, V> &p, int w1, dim3 g, const MvEpi &e, cudaStream_t st);
+int fx_scatter_run(adda_gb300_ctx *c, const MvP<double, double2> &p, cudaStream_t st);
+int fx_gather_run(adda_gb300_ctx *c, const MvP<double, double2> &p, const MvEpi &e, cudaStream_t st);
+int fx_yz_run(adda_gb300_ctx *c, const MvGeom<double> &p, int ck, cudaStream_t st);
+
 // the y/z stage of one chunk of x-slabs (K2a, [K2a surface], K2b, K2c) with the context's tile shape, on stream st
 template <typename T> int launch_yz(adda_gb300_ctx *c, MvGeom<T> p, int ck, const MvShape &sh, cudaStream_t st)
 {
 	const int R = p.R;
 	const bool surf = c->surface;
 	const dim3 g2((c->bY + sh.w2 - 1) / sh.w2, 3 * ck, R);
-	ADDA_NS_SWITCH(c->gZ, ADDA_W_SWITCH(has_w2, sh.w2, (mv_fftz<T, W, 0, NS><<<g2, col_threads<T, NS, W>(),
-		tile_smem<T>(c->gZ, W), st>>>(p))));
-	ADDA_LAUNCHED();
-	if (surf) {
-		ADDA_NS_SWITCH(c->gZ, ADDA_W_SWITCH(has_w2, sh.w2, (mv_fftz<T, W, 2, NS><<<g2, col_threads<T, NS, W>(),
+	bool l2z = false, l2y = false;
+	if constexpr (sizeof(T) == 8) {
+		if (use_fx(c)) return fx_yz_run(c, p, ck, st);
+	}
+	else {
+		l2z = use_l2_z(c, sh);
+		l2y = use_l2_y(c);
+	}
+	// the z transform of one mode (0: K2a, 2: K2a of the reflected transform, 1: K2c)
+	auto fftz = [&](auto mode) {
+		constexpr int MODE = decltype(mode)::value;
+		if constexpr (sizeof(T) == 4)
+			if (l2z) return l2_fftz_run(c, p, MODE, sh.w2, g2, st);
+		ADDA_NS_SWITCH(c->gZ, ADDA_W_SWITCH(has_w2, sh.w2, (mv_fftz<T, W, MODE, NS><<<g2, col_threads<T, NS, W>(),
 			tile_smem<T>(c->gZ, W), st>>>(p))));
 		ADDA_LAUNCHED();
+		return ADDA_GB300_OK;
+	};
+	int rc;
+	if ((rc = fftz(std::integral_constant<int, 0>()))) return rc;
+	if (surf && (rc = fftz(std::integral_constant<int, 2>()))) return rc;
+	if (l2y) {
+		if constexpr (sizeof(T) == 4)
+			if ((rc = l2_ffty_run(c, p, ck, sh.pairs, st))) return rc;
 	}
-	if (use_k2b_reg<T>(c->gY)) {
+	else if (use_k2b_reg<T>(c->gY)) {
 		if constexpr (sizeof(T) == 4) {
 			const int nt = sh.nt;
 			const int Tl = c->gY >= 256 ? 16 : 8; // lanes per line, RegShape<gY>::T
@@ -898,11 +950,8 @@ template <typename T> int launch_yz(adda_gb300_ctx *c, MvGeom<T> p, int ck, cons
 			ADDA_NS_SWITCH(c->gY, ADDA_W_SWITCH(has_pairs, sh.pairs, (mv_fft_y_dmul<T, NS, W><<<g2b, 256, sm, st>>>(q))));
 		}
 	}
-	ADDA_LAUNCHED();
-	ADDA_NS_SWITCH(c->gZ, ADDA_W_SWITCH(has_w2, sh.w2, (mv_fftz<T, W, 1, NS><<<g2, col_threads<T, NS, W>(),
-		tile_smem<T>(c->gZ, W), st>>>(p))));
-	ADDA_LAUNCHED();
-	return ADDA_GB300_OK;
+	if (!l2y) ADDA_LAUNCHED();
+	return fftz(std::integral_constant<int, 1>());
 }
 
 // the y/z stage and its set-up are compiled once per arithmetic, in matvec_yz.cu
@@ -953,13 +1002,24 @@ int launch_matvec(adda_gb300_ctx *c, int R, const V *arg, V *res, int her, const
 	p.lat_stride = c->lat_stride;
 	cudaStream_t st = c->stream;
 	const dim3 g1((c->bY + sh.w1 - 1) / sh.w1, c->bZ, R);
-	ADDA_NS_SWITCH(c->gX, ADDA_W_SWITCH(has_w1, sh.w1, (mv_scatter_fftx<T, V, W, NS><<<g1, col_threads<T, NS, 3 * W>(),
-		tile_smem<T>(c->gX, 3 * W), st>>>(p))));
-	ADDA_LAUNCHED();
+	int rc;
+	bool l2 = false; // K1 and K3 on two-pass transforms
+	if constexpr (dbl) {
+		l2 = use_fx(c);
+		if (l2 && (rc = fx_scatter_run(c, p, st))) return rc;
+	}
+	else {
+		l2 = use_l2_x(c, sh);
+		if (l2 && (rc = l2_scatter_run<V>(c, p, sh.w1, g1, st))) return rc;
+	}
+	if (!l2) {
+		ADDA_NS_SWITCH(c->gX, ADDA_W_SWITCH(has_w1, sh.w1, (mv_scatter_fftx<T, V, W, NS><<<g1,
+			col_threads<T, NS, 3 * W>(), tile_smem<T>(c->gX, 3 * W), st>>>(p))));
+		ADDA_LAUNCHED();
+	}
 	// the y/z stage chunk by chunk, even chunks on the context stream with Tz, odd ones on the second stream with Tz2
 	// (a chunk reuses its buffer only after the chunk two before it, on the same stream, has finished with it), so
 	// that one chunk's kernels fill the other's tail; joined before K3
-	int rc;
 	const bool two = c->gX > p.CK;
 	if (two) {
 		ADDA_CUDA(cudaEventRecord(c->ev_fork, st));
@@ -977,6 +1037,10 @@ int launch_matvec(adda_gb300_ctx *c, int R, const V *arg, V *res, int her, const
 	if (two) {
 		ADDA_CUDA(cudaEventRecord(c->ev_join, c->stream2));
 		ADDA_CUDA(cudaStreamWaitEvent(st, c->ev_join, 0));
+	}
+	if (l2) {
+		if constexpr (dbl) return fx_gather_run(c, p, epi, st);
+		else return l2_gather_run<V>(c, p, sh.w1, g1, epi, st);
 	}
 	ADDA_NS_SWITCH(c->gX, ADDA_W_SWITCH(has_w1, sh.w1, (mv_fftx_gather<T, V, W, NS><<<g1, col_threads<T, NS, 3 * W>(),
 		tile_smem<T>(c->gX, 3 * W), st>>>(p, epi))));

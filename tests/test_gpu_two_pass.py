@@ -1,0 +1,79 @@
+"""The matvec on two-pass transforms (axis lengths n = r1*r2 with radices up to 16): every FP64 matvec, in 64-bit fixed
+point, and the FP32 matvec of lengths without compile-time kernels.
+
+FP64 tolerance: a transform adds noise of about 2^-54 of its block's largest value, six transforms and the D product
+follow one another, and the largest value of these random data is below 16 times their rms: 7 * 16 * 2^-54 = 6e-15.
+FP32: the 5e-6 of the other parity tests."""
+import numpy as np
+import pytest
+
+from helpers import oracle_for, rel, setup_for
+from test_gpu_parity import context, cube_setup, random_vec
+
+pytestmark = pytest.mark.gpu
+TOL64, TOL32 = 6e-15, 5e-6
+
+# lengths whose plans hold every radix from 1 to 16 in the first and in the second pass
+LENGTHS = [2, 4, 6, 10, 14, 18, 22, 26, 32, 36, 44, 52, 70, 78, 80, 90, 96, 98, 110, 130, 132, 154, 156, 168, 180, 182,
+           196, 208, 210, 224, 240, 256]
+
+
+def check(s, x, her=False, precs=("fp64", "fp32")):
+    o, c = oracle_for(s), context(s, R=x.shape[0])
+    for prec in precs:
+        y, ip = c.matvec(x, prec, her)
+        for r in range(x.shape[0]):
+            o.set_cc(s.cc[r % 2].reshape(1, 3))
+            yr, ipr = o.matvec(x[r], her)
+            assert rel(y[r], yr) < (TOL64 if prec == "fp64" else TOL32), (prec, r)
+            assert abs(ip[r] / ipr - 1) < (1e-12 if prec == "fp64" else 1e-5)
+    o.close()
+    c.close()
+
+
+@pytest.mark.parametrize("n", LENGTHS)
+@pytest.mark.parametrize("axis", [0, 1, 2])
+def test_axis_length(axis, n):
+    """a thin box with the length along one axis (full to half of it, and with a ragged particle edge)"""
+    box, grid = [3, 2, 3], [6, 4, 6]
+    box[axis], grid[axis] = n // 2, n
+    s = cube_setup(box, grid)
+    check(s, random_vec(s.n, 2, n + axis), her=bool(n % 4))
+
+
+def test_scales_zeros_and_tiny_values():
+    """right-hand sides of very different magnitude, zeros and subnormal numbers keep their own exponents"""
+    s = setup_for(dict(grid=16, m=1.5, dpl=10))
+    x = random_vec(s.n, 1, 3)[0]
+    scales = [1.0, 1e-200, 1e200, 2.0 ** -1060]
+    c = context(s, R=6)
+    y, _ = c.matvec(np.stack([x * k for k in scales] + [np.zeros_like(x), x]), "fp64")
+    assert rel(y[1] * 1e200, y[0]) < TOL64 and rel(y[2] * 1e-200, y[0]) < TOL64
+    # spacing 2^-1074: the input itself has about 14 bits
+    assert rel(y[3] * 2.0 ** 1000 * 2.0 ** 60, y[0]) < 1e-3
+    assert not y[4].any() and np.array_equal(y[5], y[0])
+    c.close()
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+def test_non_finite_input_stays_with_its_rhs(bad):
+    s = setup_for(dict(grid=16, m=1.5, dpl=10))
+    x = random_vec(s.n, 2, 4)
+    c = context(s, R=2)
+    good, _ = c.matvec(x, "fp64")
+    x[1, 17] = bad
+    y, _ = c.matvec(x, "fp64")
+    assert np.array_equal(y[0], good[0]) and np.isnan(y[1]).all()
+    again, _ = c.matvec(np.stack([x[0], x[0]]), "fp64")
+    assert rel(again[0], good[0]) == 0 and np.isfinite(again[1]).all()
+    c.close()
+
+
+def test_concentrated_spectrum():
+    """a plane wave along an axis of a full cube puts the whole spectrum into a few elements: the transforms reach the
+    largest growth their range allows"""
+    s = cube_setup((32, 32, 32), (64, 64, 64))
+    k = 2 * np.pi / 64 * np.array([[0, 0, 0], [8, 0, 0], [16, 16, 0], [31, 31, 31]])
+    pol = np.array([1.0, 1.0j, -1.0])
+    x = np.stack([(np.exp(1j * s.pos @ kk)[:, None] * pol).reshape(-1) for kk in k])
+    check(s, x, precs=("fp64",))
