@@ -405,7 +405,7 @@ int adda_gb300_destroy(adda_gb300_ctx *c)
 	solver_free(c);
 	void *bufs[] = {c->d_line_start, c->d_xy, c->d_mat, c->d_pos, c->D64, c->D32, c->cc64, c->ccs64, c->ccs32,
 		c->Xf, c->Tz, c->TzR, c->Tz2, c->TzR2, c->R64, c->R32, c->partial, c->d_red, c->vin, c->vout, c->pvec64,
-		c->tables, c->Dfx, c->fx_exps};
+		c->tables, c->Dfx, c->fx_exps, c->fld};
 	if (c->stream2) cudaStreamSynchronize(c->stream2);
 	for (void *b : bufs)
 		if (b) cudaFree(b);

@@ -135,6 +135,9 @@ struct adda_gb300_ctx {
 	void *vin = nullptr, *vout = nullptr;
 	// solver
 	adda::SolverWork *sw = nullptr;
+	// workspace of scattered_fields (tables, partial sums, results), grown to the largest call
+	void *fld = nullptr;
+	size_t fld_bytes = 0;
 	// last solve leaves polarisations here (FP64) for the cross sections
 	double2 *pvec64 = nullptr;
 	int last_nrhs = 0;
@@ -165,6 +168,9 @@ template <typename T, typename V>
 int matvec_run(adda_gb300_ctx *c, int R, const V *arg, V *res, int her, const MvEpi &epi, const int *done);
 int reduce_partials(adda_gb300_ctx *c, int R, const double *partial, size_t nblk, double *out);
 
+// fields.cu
+int scattered_fields(adda_gb300_ctx *c, int nrhs, int ndir, const double *dirs, double *ebuff);
+
 // solver.cu
 int solver_solve(adda_gb300_ctx *c, const adda_gb300_solve_params *sp, int nrhs, const double *einc, double *xvec,
 	double *pvec, adda_gb300_rhs_stats *stats, double *resid_hist, int hist_cap);
@@ -177,7 +183,6 @@ int cross_sections_beam(adda_gb300_ctx *c, int nrhs, const double *einc, double 
 size_t solver_chpoint_size(const adda_gb300_ctx *c, int method);
 int solver_chpoint_save(adda_gb300_ctx *c, int rhs, void *buf, size_t size);
 int solver_chpoint_load(adda_gb300_ctx *c, int rhs, const void *buf, size_t size);
-int scattered_fields(adda_gb300_ctx *c, int nrhs, int ndir, const double *dirs, double *ebuff);
 int vjp_chi(adda_gb300_ctx *c, const adda_gb300_solve_params *sp, int rhs, const double prop[3], const double incpol[3],
 	const double *dinv_alpha, double *grad_cext, double *grad_cabs);
 

@@ -1,0 +1,275 @@
+// fields.cu - scattering amplitudes of the last solve in a set of directions (CalcFieldFree, crosssec.c:506-596):
+// E_r(n) = (-i k^3) exp(-i k r0.n) (I - nn) sum_j P_rj exp(-i kd n.pos_j).
+//
+// The sum is FP64-exact work on a chip whose FP64 pipe issues one instruction per 76 cycles and scheduler, so it runs on
+// the integer pipes:
+//   - the lattice makes the phase a product of three factors, one per axis: exp(-i kd n.pos) = X[x] Y[y] Z[z], taken from
+//     tables of (boxX + boxY + boxZ) values per direction instead of one sincos per dipole and direction;
+//   - along an x-line only X[x] changes: the dipoles of a line are summed with it, and the line's sum is multiplied by
+//     Y[y] Z[z];
+//   - P (relative to the largest |component| of the RHS) and X are 54-bit fixed point in two signed limbs of 27 bits.
+//     A complex product is 12 32x32+64-bit multiply-adds (2 cycles each); the limb products of up to FLD_RUN dipoles
+//     accumulate in 64 bits without carries.
+// One unit is 2^-54 of the largest P component (FP64 rounding of a typical term) and the tables are accurate to 2^-53;
+// the rounding of the phase's argument dominates both this and a direct FP64 sum (2e-15 at 64^3).
+// Measured: 64^3 sphere (137 k dipoles), 2 RHS, 2080 directions, with the host copies and the cross sections: 57.1 ms
+// with an FP64 sincos per dipole and direction -> 3.27 ms, of which fld_sum 3.1 ms (66 instructions a dipole and warp;
+// the multiply-add pipe's bound is 1.3 ms, the rest are the loads' latency at 20 warps an SM). One warp per block: with
+// blocks of four warps the last wave was half empty (5.4 ms, with a data-dependent loop over the dipoles).
+#include "fft_lines2.cuh"
+#include "ctx.cuh"
+
+#include <algorithm>
+#include <cstring>
+
+namespace adda {
+
+namespace {
+
+constexpr int FLD_RUN = 128;        // dipoles whose limb products fit 64-bit sums: 2^55 each
+constexpr int FLD_SPAN = 512;       // dipoles whose sums stay below 2^62 in fixed point
+constexpr int FLD_RESIDENT = 20;    // resident warps (blocks) an SM of the sum
+constexpr int FLD_FIN = 8;          // threads that add up a direction's partial sums
+constexpr size_t FLD_TABLE = 64u << 20; // bytes of phase tables per launch (bounds the directions of one)
+
+// largest high word of |P|'s components per RHS (hmax zeroed before)
+__global__ void __launch_bounds__(256) fld_max(const double2 *P, size_t n3, int *hmax)
+{
+	const int r = blockIdx.y;
+	int h = 0;
+	for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n3; i += (size_t)gridDim.x * blockDim.x) {
+		const double2 v = P[r * n3 + i];
+		h = max(h, max(__double2hiint(v.x) & 0x7fffffff, __double2hiint(v.y) & 0x7fffffff));
+	}
+	h = __reduce_max_sync(0xffffffffu, h);
+	if ((threadIdx.x & 31) == 0) atomicMax(hmax + r, h);
+}
+
+// two signed limbs of 27 bits of |v| < 2^54
+__device__ __forceinline__ void fld_limbs(long long v, int &h, int &l)
+{
+	l = (int)((unsigned)v << 5) >> 5;
+	h = (int)((v - l) >> 27);
+}
+// P in limbs: component i of RHS r at [r*n3 + i], (re high, re low, im high, im low)
+__global__ void __launch_bounds__(256) fld_split(const double2 *P, size_t n3, const int *hmax, int4 *out)
+{
+	const int r = blockIdx.y;
+	const int emax = max(1, hmax[r] >> 20);
+	for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n3; i += (size_t)gridDim.x * blockDim.x) {
+		const double2 v = P[r * n3 + i];
+		int4 o;
+		// fx_from_double gives |v| < 2^FX_TOP: down to 54 bits, value = v * 2^(emax - 1076)
+		fld_limbs(fx_rshift(fx_from_double(v.x, emax), FX_TOP - 54), o.x, o.y);
+		fld_limbs(fx_rshift(fx_from_double(v.y, emax), FX_TOP - 54), o.z, o.w);
+		out[r * n3 + i] = o;
+	}
+}
+
+// phase tables of nd directions (row length ld): x factors as limbs of 2^54, y and z factors as 2^62 split for fx_cmul
+__global__ void __launch_bounds__(256) fld_tables(const double *dirs, int nd, int ld, int bX, int bY, int bZ, double kd,
+	int4 *tab)
+{
+	const int d = blockIdx.x * blockDim.x + threadIdx.x;
+	int t = blockIdx.y; // table row: x, then y, then z
+	if (d >= nd) return;
+	const int axis = t < bX ? 0 : t < bX + bY ? 1 : 2;
+	const int i = t - (axis ? bX : 0) - (axis == 2 ? bY : 0);
+	double sn, cs;
+	sincos(-kd * (dirs[3 * d + axis] * i), &sn, &cs);
+	int4 o;
+	if (axis == 0) {
+		fld_limbs(__double2ll_rn(cs * 18014398509481984.0), o.x, o.y);
+		fld_limbs(__double2ll_rn(sn * 18014398509481984.0), o.z, o.w);
+	}
+	else {
+		const long long c = __double2ll_rn(cs * 4611686018427387904.0), s = __double2ll_rn(sn * 4611686018427387904.0);
+		fx_split(c, o.x, o.y);
+		fx_split(s, o.z, o.w);
+		o.y = max(o.y, -0x7fffffff); // negated in fx_cmul
+		o.w = max(o.w, -0x7fffffff);
+	}
+	tab[(size_t)t * ld + d] = o;
+}
+
+// partial sums over a range of dipoles for 32 directions, one per lane: grid (direction groups, ranges, RHS), one warp a
+// block, so that the neighbours in x read the same dipoles through L1. part: [range][R][6][ld]
+__global__ void __launch_bounds__(32, FLD_RESIDENT) fld_sum(const int4 *P, const uint16_t *pos, const uint32_t *xy,
+	const uint32_t *lstart, size_t N, const int4 *tab, const int *hmax, int nd, int ld, int bX, int bY, int bZ, size_t span,
+	double *part, int rpp, size_t lst)
+{
+	const int r = blockIdx.z, R = gridDim.z;
+	const int d = blockIdx.x * 32 + threadIdx.x;
+	const size_t lq = (size_t)(r / rpp); // RHS r's particle (group contexts)
+	pos += lq * lst * 3;
+	xy += lq * lst;
+	lstart += lq * ((size_t)bZ * bY + 1);
+	P += (size_t)r * 3 * N;
+	// the particle's own dipoles (a smaller particle of a group is padded to N)
+	const size_t i0 = (size_t)blockIdx.y * span, i1 = min((size_t)lstart[(size_t)bZ * bY], i0 + span);
+	const int4 *tx = tab + d, *ty = tx + (size_t)bX * ld, *tz = ty + (size_t)bY * ld;
+	const int e = max(1, hmax[r] >> 20) - 1074; // of S: a quarter of P's integers (fx_cmul)
+	double tot[6] = {0, 0, 0, 0, 0, 0};
+	size_t i = i0;
+	while (i < i1) {
+		const size_t iend = min(i1, i + FLD_SPAN);
+		long long S[6] = {0, 0, 0, 0, 0, 0};
+		while (i < iend) {
+			// one run: dipoles of one x-line, at most FLD_RUN of them
+			const int y = pos[3 * i + 1], z = pos[3 * i + 2];
+			const int n = (int)(min(min(iend, i + FLD_RUN), (size_t)lstart[(size_t)z * bY + y + 1]) - i);
+			const long long half = 1ll << 26; // rounds T >> 27
+			long long U[6] = {0, 0, 0, 0, 0, 0}, T[6] = {half, half, half, half, half, half};
+			const int4 *p = P + 3 * i;
+			const uint32_t *px = xy + i;
+#pragma unroll 2
+			for (int t = 0; t < n; t++) {
+				const int4 w = __ldg(tx + (size_t)(px[t] & 0xffff) * ld);
+				const int nsh = -w.z, nsl = -w.w;
+#pragma unroll
+				for (int c = 0; c < 3; c++) {
+					const int4 v = __ldg(p + 3 * t + c);
+					U[2 * c] = (long long)v.x * w.x + U[2 * c];
+					U[2 * c] = (long long)v.z * nsh + U[2 * c];
+					U[2 * c + 1] = (long long)v.x * w.z + U[2 * c + 1];
+					U[2 * c + 1] = (long long)v.z * w.x + U[2 * c + 1];
+					T[2 * c] = (long long)v.x * w.y + T[2 * c];
+					T[2 * c] = (long long)v.y * w.x + T[2 * c];
+					T[2 * c] = (long long)v.z * nsl + T[2 * c];
+					T[2 * c] = (long long)v.w * nsh + T[2 * c];
+					T[2 * c + 1] = (long long)v.x * w.w + T[2 * c + 1];
+					T[2 * c + 1] = (long long)v.y * w.z + T[2 * c + 1];
+					T[2 * c + 1] = (long long)v.z * w.y + T[2 * c + 1];
+					T[2 * c + 1] = (long long)v.w * w.x + T[2 * c + 1];
+				}
+			}
+			i += n;
+			// the line's sum times Y Z (2^60 after the product of the two, back to 2^62)
+			const int4 yv = __ldg(ty + (size_t)y * ld), zv = __ldg(tz + (size_t)z * ld);
+			const fx2 yy{((long long)yv.x << 32) + yv.y, ((long long)yv.z << 32) + yv.w};
+			const fx2 q = fx_cmul(yy, zv, false);
+			int4 yz;
+			fx_split(q.x << 2, yz.x, yz.y);
+			fx_split(q.y << 2, yz.z, yz.w);
+			yz.y = max(yz.y, -0x7fffffff); // negated in fx_cmul
+			yz.w = max(yz.w, -0x7fffffff);
+#pragma unroll
+			for (int c = 0; c < 3; c++) {
+				// (U * 2^54 + T * 2^27) / 2^54
+				const fx2 s = fx_cmul(fx2{U[2 * c] + (T[2 * c] >> 27), U[2 * c + 1] + (T[2 * c + 1] >> 27)}, yz, false);
+				S[2 * c] += s.x;
+				S[2 * c + 1] += s.y;
+			}
+		}
+#pragma unroll
+		for (int c = 0; c < 6; c++) tot[c] += fx_to_double(S[c], e);
+	}
+	if (d < nd) {
+		double *o = part + ((size_t)blockIdx.y * R + r) * 6 * ld + d;
+#pragma unroll
+		for (int c = 0; c < 6; c++) o[(size_t)c * ld] = hmax[r] >= 0x7ff00000 ? __hiloint2double(0x7ff80000, 0) : tot[c];
+	}
+}
+
+__device__ __forceinline__ double2 cmuld(double2 a, double2 b)
+{
+	return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+}
+// 32 directions of one RHS per block: fixed-order sum of the partials (FLD_FIN threads a direction), (I - nn), and the
+// factor (-i k^3) exp(-i k r0.n) with r0 the centre offset of the box's first dipole (make_particle.c:2305-2308).
+// out [R][ndir][3], directions d0...
+__global__ void __launch_bounds__(32 * FLD_FIN) fld_finish(const double *part, int slices, int nd, int ld, int R,
+	const double *dirs, double k, double gs, int bX, int bY, int bZ, double2 *out, int ndir, int d0)
+{
+	__shared__ double sh[FLD_FIN][6][32];
+	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, r = blockIdx.y, d = blockIdx.x * 32 + lane;
+	double s[6] = {0, 0, 0, 0, 0, 0};
+	if (d < nd)
+		for (int b = w; b < slices; b += FLD_FIN)
+#pragma unroll
+			for (int c = 0; c < 6; c++) s[c] += part[(((size_t)b * R + r) * 6 + c) * ld + d];
+#pragma unroll
+	for (int c = 0; c < 6; c++) sh[w][c][lane] = s[c];
+	__syncthreads();
+	if (w || d >= nd) return;
+#pragma unroll
+	for (int c = 0; c < 6; c++)
+		for (int b = 1; b < FLD_FIN; b++) s[c] += sh[b][c][lane];
+	const double n[3] = {dirs[3 * d], dirs[3 * d + 1], dirs[3 * d + 2]};
+	double2 dpr = make_double2(0, 0);
+	for (int c = 0; c < 3; c++) {
+		dpr.x += s[2 * c] * n[c];
+		dpr.y += s[2 * c + 1] * n[c];
+	}
+	const double r0[3] = {-gs * (bX - 1) / 2.0, -gs * (bY - 1) / 2.0, -gs * (bZ - 1) / 2.0};
+	double sn, cs;
+	sincos(-k * (r0[0] * n[0] + r0[1] * n[1] + r0[2] * n[2]), &sn, &cs);
+	const double k3 = k * k * k;
+	const double2 amp = make_double2(sn * k3, -cs * k3); // -i k^3 (cs + i sn)
+	for (int c = 0; c < 3; c++)
+		out[((size_t)r * ndir + d0 + d) * 3 + c] = cmuld(amp, make_double2(s[2 * c] - dpr.x * n[c],
+			s[2 * c + 1] - dpr.y * n[c]));
+}
+
+} // namespace
+
+int scattered_fields(adda_gb300_ctx *c, int R, int ndir, const double *dirs, double *ebuff)
+{
+	const size_t N = c->N, n3 = 3 * N;
+	cudaStream_t s = c->stream;
+	const size_t rows = (size_t)c->bX + c->bY + c->bZ;
+	// directions per launch: the tables' budget, a multiple of 32 within the grid's limit
+	const int per = (int)std::max<size_t>(32, std::min<size_t>(32768, FLD_TABLE / (rows * sizeof(int4)) / 32 * 32));
+	const int ld = std::min(per, (ndir + 31) / 32 * 32), groups = ld / 32;
+	// ranges of dipoles: three waves of resident warps (lines of different length even out), at least 256 dipoles each
+	const size_t warps = (size_t)152 * FLD_RESIDENT * 3, per_slice = (size_t)groups * R;
+	const size_t slices = std::max<size_t>(1, std::min<size_t>((N + 255) / 256, warps / per_slice));
+	const size_t span = std::max<size_t>(1, (N + slices - 1) / slices);
+	const auto up = [](size_t v) { return (v + 255) / 256 * 256; };
+	const size_t b_dirs = up(sizeof(double) * 3 * ndir), b_out = up(sizeof(double2) * 3 * (size_t)ndir * R),
+				 b_max = up(sizeof(int) * R), b_tab = up(sizeof(int4) * rows * ld), b_part = up(sizeof(double) * slices * R * 6 * ld);
+	const size_t need = b_dirs + b_out + b_max + b_tab + b_part;
+	if (need > c->fld_bytes) {
+		if (c->fld) cudaFree(c->fld);
+		c->fld = nullptr;
+		c->fld_bytes = 0;
+		ADDA_CUDA(cudaMalloc(&c->fld, need));
+		c->fld_bytes = need;
+	}
+	unsigned char *at = (unsigned char *)c->fld;
+	const auto take = [&](size_t n) {
+		unsigned char *q = at;
+		at += n;
+		return q;
+	};
+	double *d_dirs = (double *)take(b_dirs);
+	double2 *d_out = (double2 *)take(b_out);
+	int *d_max = (int *)take(b_max);
+	int4 *d_tab = (int4 *)take(b_tab);
+	int4 *d_p = (int4 *)c->vin; // the staging buffer of the host-pointer matvec: R*3N complex doubles
+	double *d_part = (double *)take(b_part);
+	ADDA_CUDA(cudaMemcpyAsync(d_dirs, dirs, sizeof(double) * 3 * ndir, cudaMemcpyHostToDevice, s));
+	ADDA_CUDA(cudaMemsetAsync(d_max, 0, sizeof(int) * R, s));
+	const dim3 gp((unsigned)std::max<size_t>(1, std::min<size_t>((n3 + 255) / 256, 152 * 8)), R);
+	fld_max<<<gp, 256, 0, s>>>(c->pvec64, n3, d_max);
+	ADDA_LAUNCHED();
+	fld_split<<<gp, 256, 0, s>>>(c->pvec64, n3, d_max, d_p);
+	ADDA_LAUNCHED();
+	for (int d0 = 0; d0 < ndir; d0 += ld) {
+		const int nd = std::min(ld, ndir - d0);
+		fld_tables<<<dim3((nd + 255) / 256, (unsigned)rows), 256, 0, s>>>(d_dirs + 3 * (size_t)d0, nd, ld, c->bX, c->bY, c->bZ,
+			c->k * c->gridspace, d_tab);
+		ADDA_LAUNCHED();
+		fld_sum<<<dim3(groups, (unsigned)slices, R), 32, 0, s>>>(d_p, c->d_pos, c->d_xy, c->d_line_start, N, d_tab, d_max, nd,
+			ld, c->bX, c->bY, c->bZ, span, d_part, c->rpp, c->lat_stride);
+		ADDA_LAUNCHED();
+		fld_finish<<<dim3(groups, R), 32 * FLD_FIN, 0, s>>>(d_part, (int)slices, nd, ld, R, d_dirs + 3 * (size_t)d0, c->k,
+			c->gridspace, c->bX, c->bY, c->bZ, d_out, ndir, d0);
+		ADDA_LAUNCHED();
+	}
+	ADDA_CUDA(cudaMemcpyAsync(ebuff, d_out, sizeof(double2) * 3 * (size_t)ndir * R, cudaMemcpyDeviceToHost, s));
+	ADDA_CUDA(cudaStreamSynchronize(s));
+	return ADDA_GB300_OK;
+}
+
+} // namespace adda
