@@ -42,10 +42,17 @@ enum MvEpiMode {
 	EPI_DOT_ARG_CONJ = 8 // s1 = sum x*conj(y)  (x = argument)                 -- BiCGStab s.t (iterative.c:712)
 };
 
+struct RhsState; // krylov.cuh
+
 struct MvEpi {
 	int mode;
 	const void *u;     // vector for EPI_DOT_U_CONJ (same precision as the matvec)
 	double *partial;   // per-block partial sums
+	// the solver's scalar step on the sums (MvTail, krylov.cuh), in the last block of a RHS
+	int tail = 0;
+	RhsState *st = nullptr;
+	int *done = nullptr;
+	unsigned *cnt = nullptr; // [R], zero
 };
 
 struct SolverWork; // solver.cu

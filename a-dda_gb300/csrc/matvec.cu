@@ -15,15 +15,11 @@ namespace {
 // sum per-RHS partials (fixed order): out[r*4 + 0..2]
 __global__ void reduce_partials_k(const double *partial, size_t nblk, double *out)
 {
-	__shared__ double red[32];
 	const int r = blockIdx.x;
-	double s[3] = {0, 0, 0};
-	for (size_t b = threadIdx.x; b < nblk; b += blockDim.x)
-		for (int j = 0; j < 3; j++) s[j] += partial[((size_t)r * nblk + b) * 4 + j];
-	for (int j = 0; j < 3; j++) {
-		double v = mv::block_sum(s[j], red);
-		if (threadIdx.x == 0) out[r * 4 + j] = v;
-	}
+	double s[3];
+	sum_parts<3>(partial, nblk, r, s);
+	if (threadIdx.x == 0)
+		for (int j = 0; j < 3; j++) out[r * 4 + j] = s[j];
 }
 
 } // namespace

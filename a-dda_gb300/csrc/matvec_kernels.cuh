@@ -27,6 +27,7 @@
 #pragma once
 
 #include "ctx.cuh"
+#include "krylov.cuh"
 
 #include <algorithm>
 #include <type_traits>
@@ -605,24 +606,10 @@ __global__ void __launch_bounds__(NT, NS >= 512 ? (NT >= 256 ? 1 : 256 / NT) : (
 	}
 }
 
-__device__ __forceinline__ double block_sum(double v, double *sh)
-{
-	for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-	const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-	__syncthreads();
-	if (lane == 0) sh[wid] = v;
-	__syncthreads();
-	double s = 0;
-	if (threadIdx.x == 0)
-		for (int w = 0; w < (int)(blockDim.x >> 5); w++) s += sh[w];
-	return s; // valid in thread 0
-}
-
 // y = x + S.X for the dipoles of W x-lines (one z) whose X stands in a tile (element x of line comp*W + y is
 // o(x*LS + line)), with the epilogue reductions; every thread of the block calls it
 template <typename T, typename V, int W, typename P, typename O>
-__device__ __forceinline__ void gather_lines(const P &p, const MvEpi &e, O o, int LS, int r, int z, int y0, int wy, int NT,
-	double *red)
+__device__ __forceinline__ void gather_lines(const P &p, const MvEpi &e, O o, int LS, int r, int z, int y0, int wy, int NT)
 {
 	typedef typename CxT<T>::type C;
 	// the lattice of RHS r's particle (a single-lattice context has one)
@@ -660,14 +647,15 @@ __device__ __forceinline__ void gather_lines(const P &p, const MvEpi &e, O o, in
 		const size_t nblk = (size_t)gridDim.x * gridDim.y;
 		const size_t blk = (size_t)blockIdx.y * gridDim.x + blockIdx.x;
 		double *out = e.partial + ((size_t)r * nblk + blk) * 4;
-		double v0 = block_sum(acc_val(s0), red);
-		double v1 = block_sum(acc_val(s1r), red);
-		double v2 = block_sum(acc_val(s1i), red);
+		const typename AccOf<V>::T sums[3] = {s0, s1r, s1i};
+		double tot[3];
+		block_totals<3>(sums, tot);
 		if (threadIdx.x == 0) {
-			out[0] = v0;
-			out[1] = v1;
-			out[2] = v2;
+			out[0] = tot[0];
+			out[1] = tot[1];
+			out[2] = tot[2];
 		}
+		if (e.tail && last_block(e.cnt + r, (unsigned)nblk)) matvec_tail(e.tail, e.st, e.done, e.partial, nblk, r);
 	}
 }
 
@@ -678,7 +666,6 @@ __global__ void __launch_bounds__(col_threads<T, NS, 3 * W>(), (col_minblocks<T,
 {
 	typedef typename CxT<T>::type C;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
-	__shared__ double red[32];
 	if (rhs_done(p, blockIdx.z)) return; // blockIdx.z = RHS
 	constexpr int NL = 3 * W, LS = tile_ls(3 * W), NT = col_threads<T, NS, 3 * W>();
 	constexpr bool RC = reg_cols<T, NS>();
@@ -721,7 +708,7 @@ __global__ void __launch_bounds__(col_threads<T, NS, 3 * W>(), (col_minblocks<T,
 		__syncthreads();
 		o = tile_fft<C, NS, NL, LS, true>(a, b, p.px, p.twx);
 	}
-	gather_lines<T, V, W>(p, e, [&](int i) { return o[i]; }, LS, r, z, y0, wy, NT, red);
+	gather_lines<T, V, W>(p, e, [&](int i) { return o[i]; }, LS, r, z, y0, wy, NT);
 }
 
 // ---------------------------------------------------------------------------------------------------------------

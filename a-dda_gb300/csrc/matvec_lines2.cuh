@@ -473,7 +473,6 @@ __global__ void __launch_bounds__(32 * ((3 * W * RADIX_MAX + 31) / 32), A::FX ? 
 {
 	typedef typename A::C C;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
-	__shared__ double red[32];
 	if (rhs_done(p, blockIdx.z)) return; // blockIdx.z = RHS
 	constexpr int NL = 3 * W, LS = tile_ls(3 * W);
 	C *a = reinterpret_cast<C *>(smem_raw); // bX x LS
@@ -524,7 +523,7 @@ __global__ void __launch_bounds__(32 * ((3 * W * RADIX_MAX + 31) / 32), A::FX ? 
 		}
 		else return v;
 	};
-	gather_lines<typename A::T, V, W>(p, e, get, LS, r, z, y0, wy, blockDim.x, red);
+	gather_lines<typename A::T, V, W>(p, e, get, LS, r, z, y0, wy, blockDim.x);
 }
 
 // ---------------------------------------------------------------------------------------------------------------

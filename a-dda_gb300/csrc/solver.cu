@@ -1,14 +1,14 @@
 // solver.cu - device-resident Krylov solvers (IterativeSolver, src/iterative.c:1398-1530) and cross sections.
 //
 // Every vector, scalar and reduction stays on the GPU. One iteration is a fixed kernel sequence:
-//   QMR_CS (iterative.c:956-1029):   matvec(v) + [alpha = v.Av fused in its epilogue] -> qmr_s1 -> qmr_v1
-//                                    [v~ update + |v~|^2, v~.v~] -> qmr_s2 -> qmr_v2 [p, x, v, r updates + |r|^2]
-//                                    -> progress
-//   BiCGStab (iterative.c:673-720):  bs_s0 -> bs_v1 [p] -> matvec(p) [v.r~*] -> bs_s1 -> bs_v2 [s, |s|^2] -> bs_s2
-//                                    -> matvec(s) [|t|^2, s.t*] -> bs_s3 -> bs_v3 [x, r, |r|^2, r.r~*] -> progress
-// Scalar kernels run one block per right-hand side: they sum the deterministic per-block partials of the previous
-// kernel in a fixed order and update that RHS's FP64 recurrence scalars (including the breakdown tests and the
-// stagnation counter of ProgressReport, iterative.c:282-318). Several RHS iterate in lockstep; a converged RHS is
+//   QMR_CS (iterative.c:956-1029):   matvec(v) [alpha = v.Av] -> qmr_v1 [v~ update + |v~|^2, v~.v~; Givens rotation]
+//                                    -> qmr_v2 [p, x, v, r updates + |r|^2; progress]
+//   BiCGStab (iterative.c:673-720):  bs_s0 -> bs_v1 [p] -> matvec(p) [v.r~*; alpha] -> bs_v2 [s, |s|^2; half step]
+//                                    -> matvec(s) [|t|^2, s.t*; omega] -> bs_v3 [x, r, |r|^2, r.r~*; progress]
+// The scalar steps run in the last block of the kernel whose sums they need (krylov.cuh), or as kernels of one block
+// per right-hand side: the deterministic per-block partials are summed in a fixed order and update that RHS's FP64
+// recurrence scalars (including the breakdown tests and the stagnation counter of ProgressReport,
+// iterative.c:282-318). Several RHS iterate in lockstep; a converged RHS is
 // frozen by its done flag. check_every iterations are captured once as a CUDA graph and replayed; the host reads
 // the done flags only between graph launches.
 //
@@ -22,6 +22,7 @@
 // initial-field test for the first iteration (matvec_ready, iterative.c:962-965, 691); here the first iteration
 // always computes its matvec. The iterates agree to rounding.
 #include "ctx.cuh"
+#include "krylov.cuh"
 
 #include <algorithm>
 #include <chrono>
@@ -32,30 +33,6 @@
 
 namespace adda {
 
-struct RhsState {
-	double inprodR, inprodRp1, epsB, resid_scale;
-	int niter, counter, done, status, half, mc, maxiter, x0zero;
-	int it0;  // niter when the current Krylov run started (role parity of the swapped QMR_CS / CSYM buffers)
-	double prev_err; // last reported relative residual (ProgressReport's prev_err, kept in checkpoints)
-	int full; // BiCGStab: no half-step exit
-	// QMR_CS
-	double c_old, c_new, om_old, om_new;
-	double2 beta, tautilda, s_old, s_new, alpha, theta, eta, zetat;
-	// BiCGStab, BiCG_CS (ro, balpha), CGNR (real parts of ro, balpha)
-	double2 ro_old, ro_new, omega, balpha;
-	// CSYM: beta_(k+1) = |w| (real); tau, c, s, theta, eta share the QMR_CS fields, gamma is kept in zetat
-	double cs_beta;
-	// QMR_CS_2: ro_k, theta_(k-1), c_(k-1); eps_(k-1), eta_(k-1), beta_k; delta_k = v_k.v_k
-	double q2_ro, q2_theta, q2_c;
-	double2 q2_eps, q2_eta, q2_beta, q2_delta;
-	// BCGS2: rho_0, rho_1, alpha; the convex-combination coefficients y0[1], y0[2]
-	double2 b2_rho0, b2_rho1, b2_alpha, b2_y1, b2_y2;
-	// coefficients for the vector kernels
-	double2 k0, k1, k2, k3, kib, kr;
-	double d0;
-	double temp; // |b|^2
-};
-
 struct SolverWork {
 	int R = 0;
 	size_t n3 = 0;
@@ -65,6 +42,7 @@ struct SolverWork {
 	double2 *kv[8] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
 	RhsState *st = nullptr;
 	int *done = nullptr;   // mirror of st[r].done for the matvec early exit
+	unsigned *cnt = nullptr; // blocks done per RHS (last_block), zero between kernels
 	double *hist = nullptr;
 	int hist_cap = 0;
 	double *vpart = nullptr; // vector-kernel partials [R][nbv][4]
@@ -84,91 +62,56 @@ namespace {
 
 constexpr int NT = 256;
 
-__device__ __forceinline__ double2 dc(double a, double b) { return make_double2(a, b); }
-__device__ __forceinline__ double2 dmul(double2 a, double2 b) { return dc(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); }
-__device__ __forceinline__ double2 dadd(double2 a, double2 b) { return dc(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ double2 dsub(double2 a, double2 b) { return dc(a.x - b.x, a.y - b.y); }
-__device__ __forceinline__ double2 dscal(double2 a, double s) { return dc(a.x * s, a.y * s); }
-__device__ __forceinline__ double2 dconj(double2 a) { return dc(a.x, -a.y); }
-__device__ __forceinline__ double dabs(double2 a) { return hypot(a.x, a.y); }
-__device__ __forceinline__ double2 ddiv(double2 a, double2 b)
-{
-	// a/b with scaling against overflow (Smith's method)
-	if (fabs(b.x) >= fabs(b.y)) {
-		const double r = b.y / b.x, d = b.x + b.y * r;
-		return dc((a.x + a.y * r) / d, (a.y - a.x * r) / d);
-	}
-	const double r = b.x / b.y, d = b.x * r + b.y;
-	return dc((a.x * r + a.y) / d, (a.y * r - a.x) / d);
-}
-__device__ __forceinline__ double2 dinv(double2 b) { return ddiv(dc(1, 0), b); }
-__device__ __forceinline__ double2 dsqrt(double2 z)
-{
-	const double a = z.x, b = z.y;
-	const double t = sqrt(0.5 * (hypot(a, b) + fabs(a)));
-	if (t == 0) return dc(0, 0);
-	if (a >= 0) return dc(t, b / (2 * t));
-	return dc(fabs(b) / (2 * t), copysign(t, b));
-}
-
-// a loop-invariant complex coefficient in the arithmetic of the vector type C (prepared for the packed double-float
-// products when C is dd2)
-template <typename C> struct CoefOf {
-	typedef C T;
-	static __device__ __forceinline__ C make(double2 k) { return from_d2<C>(k); }
+// loop-invariant coefficients of a vector kernel in the arithmetic of the vector type C: k[i] as a complex factor, re(i)
+// as a real one. For dd2 one warp converts them (a conversion is four FP64 instructions per number) and the block shares
+// the result. Every thread of the block constructs it.
+template <typename C, int N> struct Coefs {
+	double2 v[N];
+	template <typename... A> __device__ __forceinline__ explicit Coefs(A... a) : v{a...} {}
+	__device__ __forceinline__ C operator[](int i) const { return from_d2<C>(v[i]); }
+	__device__ __forceinline__ decltype(C::x) re(int i) const { return (decltype(C::x))v[i].x; }
 };
-template <> struct CoefOf<dd2> {
-	typedef dd2k T;
-	static __device__ __forceinline__ dd2k make(double2 k) { return make_dd2k(from_d2<dd2>(k)); }
-};
-template <typename C> __device__ __forceinline__ typename CoefOf<C>::T cof(double2 k) { return CoefOf<C>::make(k); }
-
-// block sum of up to 4 values; result valid in thread 0
-__device__ __forceinline__ void block_sum4(double v[4], int nv)
-{
-	__shared__ double sh[4][NT / 32];
-	const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-	for (int j = 0; j < nv; j++) {
-		double s = v[j];
-		for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-		if (lane == 0) sh[j][wid] = s;
-	}
-	__syncthreads();
-	if (threadIdx.x == 0)
-		for (int j = 0; j < nv; j++) {
-			double s = 0;
-			for (int w = 0; w < NT / 32; w++) s += sh[j][w];
-			v[j] = s;
+template <int N> struct Coefs<dd2, N> {
+	DF v[2 * N];
+	template <typename... A> __device__ __forceinline__ explicit Coefs(A... a)
+	{
+		__shared__ DF sh[2 * N];
+		const double2 k[N] = {a...};
+		double mine = 0;
+#pragma unroll
+		for (int i = 0; i < 2 * N; i++)
+			if ((int)threadIdx.x == i) mine = i & 1 ? k[i / 2].y : k[i / 2].x;
+		if (threadIdx.x < 32) {
+			const DF d = df_of(mine);
+			if (threadIdx.x < 2 * N) sh[threadIdx.x] = d;
 		}
-	__syncthreads();
-}
+		__syncthreads();
+#pragma unroll
+		for (int i = 0; i < 2 * N; i++) v[i] = sh[i];
+	}
+	__device__ __forceinline__ dd2k operator[](int i) const { return make_dd2k(make_dd2(v[2 * i], v[2 * i + 1])); }
+	__device__ __forceinline__ DF re(int i) const { return v[2 * i]; }
+};
 
-__device__ __forceinline__ void write_part(double *part, int nbv, double v[4], int nv)
+// NV block sums (double or double-float accumulators) as the block's partial sums
+template <int NV, typename T> __device__ __forceinline__ void write_part(double *part, int nbv, const T *v)
 {
-	block_sum4(v, nv);
+	double s[NV];
+	block_totals<NV>(v, s);
 	if (threadIdx.x == 0) {
 		double *o = part + ((size_t)blockIdx.y * nbv + blockIdx.x) * 4;
-		for (int j = 0; j < nv; j++) o[j] = v[j];
+#pragma unroll
+		for (int j = 0; j < NV; j++) o[j] = s[j];
 	}
 }
 
-// the same from double-float accumulators
-__device__ __forceinline__ void write_part(double *part, int nbv, DF a[4], int nv)
-{
-	double v[4];
-	for (int j = 0; j < 4; j++) v[j] = acc_val(a[j]);
-	write_part(part, nbv, v, nv);
-}
-
-// sum partials of RHS r in a fixed order (all threads participate); result in thread 0
-__device__ __forceinline__ void sum_part(const double *part, size_t nblk, int r, double out[4], int nv)
-{
-	double v[4] = {0, 0, 0, 0};
-	for (size_t b = threadIdx.x; b < nblk; b += blockDim.x)
-		for (int j = 0; j < nv; j++) v[j] += part[((size_t)r * nblk + b) * 4 + j];
-	block_sum4(v, nv);
-	for (int j = 0; j < nv; j++) out[j] = v[j];
-}
+// what the last block of a RHS needs for the scalar step after a vector kernel
+struct Tail {
+	int *done;
+	double *hist;
+	int hist_cap;
+	unsigned *cnt; // [R], zero
+};
 
 #define VLOOP(n3) for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < (n3); i += (size_t)gridDim.x * blockDim.x)
 
@@ -191,7 +134,7 @@ __global__ void __launch_bounds__(NT) k_mult_cc(const double2 *E, double2 *b, co
 		b[(size_t)r * n3 + i] = y;
 		v[0] += y.x * y.x + y.y * y.y;
 	}
-	write_part(part, nbv, v, 1);
+	write_part<1>(part, nbv, v);
 }
 
 __global__ void s_init(RhsState *st, int *done, const double *part, int nbv, double eps, int maxiter, int mc,
@@ -199,7 +142,7 @@ __global__ void s_init(RhsState *st, int *done, const double *part, int nbv, dou
 {
 	const int r = blockIdx.x;
 	double s[4];
-	sum_part(part, nbv, r, s, 1);
+	sum_parts<1>(part, nbv, r, s);
 	if (threadIdx.x) return;
 	RhsState &S = st[r];
 	memset(&S, 0, sizeof(S));
@@ -235,7 +178,7 @@ __global__ void __launch_bounds__(NT) k_init_field(RhsState *st, int *done, cons
 			r[rr * n3 + i] = d;
 			acc_abs2(v[0], d);
 		}
-		write_part(part, nbv, v, 1);
+		write_part<1>(part, nbv, v);
 	}
 	else { // choose x0 per RHS: st.x0zero holds 1 for x0=0
 		const bool zero = st[rr].x0zero != 0;
@@ -254,7 +197,7 @@ __global__ void s_init_choose(RhsState *st, int *done, const double *part, int n
 {
 	const int r = blockIdx.x;
 	double s[4];
-	sum_part(part, nbv, r, s, 1);
+	sum_parts<1>(part, nbv, r, s);
 	if (threadIdx.x) return;
 	RhsState &S = st[r];
 	S.inprodR = s[0];
@@ -282,7 +225,7 @@ __global__ void __launch_bounds__(NT) k_dot(const C *a, const C *u, size_t n3, i
 		if (mode == 0) acc_cmul(v[1], v[2], x, y);
 		else acc_cmulc(v[1], v[2], x, y);
 	}
-	write_part(part, nbv, v, 3);
+	write_part<3>(part, nbv, v);
 }
 
 template <typename C> __global__ void __launch_bounds__(NT) k_copy(C *dst, const C *src, size_t n3, const int *done)
@@ -297,7 +240,7 @@ __global__ void qmr_s_init(RhsState *st, const double *part, int nbv)
 {
 	const int r = blockIdx.x;
 	double s[4];
-	sum_part(part, nbv, r, s, 3);
+	sum_parts<3>(part, nbv, r, s);
 	if (threadIdx.x) return;
 	RhsState &S = st[r];
 	S.om_old = 0;
@@ -313,44 +256,21 @@ template <typename C> __global__ void __launch_bounds__(NT) qmr_v_init(const Rhs
 {
 	const int rr = blockIdx.y;
 	if (st[rr].done) return;
-	const auto k = cof<C>(st[rr].kib);
-	VLOOP(n3) v[rr * n3 + i] = cmul(k, r[rr * n3 + i]);
+	const Coefs<C, 1> k(st[rr].kib);
+	VLOOP(n3) v[rr * n3 + i] = cmul(k[0], r[rr * n3 + i]);
 }
 
 // ---------------- QMR_CS iteration ----------------
 
-__global__ void qmr_s1(RhsState *st, int *done, const double *part, size_t nblk)
-{
-	const int r = blockIdx.x;
-	if (st[r].done) return;
-	double s[4];
-	sum_part(part, nblk, r, s, 3);
-	if (threadIdx.x) return;
-	RhsState &S = st[r];
-	if (1 / (S.om_new * S.om_new) < 1e-10) { // iterative.c:958-960
-		S.status = ADDA_GB300_EBREAKDOWN;
-		S.done = 1;
-		done[r] = 1;
-		return;
-	}
-	const double2 alpha = dc(s[1], s[2]);
-	S.alpha = alpha;
-	S.theta = dscal(dmul(dconj(S.s_old), S.beta), S.om_old);
-	S.eta = dadd(dscal(S.beta, S.c_old * S.c_new * S.om_old), dscal(dmul(alpha, dconj(S.s_new)), S.om_new));
-	S.zetat = dsub(dscal(alpha, S.c_new * S.om_new), dscal(dmul(S.s_new, S.beta), S.c_old * S.om_old));
-	S.k0 = (S.niter == 1) ? dc(0, 0) : dc(-S.beta.x, -S.beta.y);
-	S.k1 = dc(-alpha.x, -alpha.y);
-	S.om_old = S.om_new;
-}
-
 // v~ = k0*v~ + k1*v + A.v ; partials sum re^2, im^2, re*im (nDotProdSelf_conj_Norm2, linalg.c:127)
 template <typename C>
-__global__ void __launch_bounds__(NT) qmr_v1(const RhsState *st, C *vt, const C *v, const C *Av, size_t n3,
-	double *part, int nbv)
+__global__ void __launch_bounds__(NT) qmr_v1(RhsState *st, C *vt, const C *v, const C *Av, size_t n3,
+	double *part, int nbv, Tail t)
 {
 	const int r = blockIdx.y;
 	if (st[r].done) return;
-	const auto k0 = cof<C>(st[r].k0), k1 = cof<C>(st[r].k1);
+	const Coefs<C, 2> K(st[r].k0, st[r].k1);
+	const auto k0 = K[0], k1 = K[1];
 	typename AccOf<C>::T s[4] = {};
 	VLOOP(n3) {
 		const size_t j = r * n3 + i;
@@ -358,59 +278,26 @@ __global__ void __launch_bounds__(NT) qmr_v1(const RhsState *st, C *vt, const C 
 		vt[j] = y;
 		acc_sq3(s, y);
 	}
-	write_part(part, nbv, s, 3);
-}
-
-__global__ void qmr_s2(RhsState *st, const double *part, int nbv)
-{
-	const int r = blockIdx.x;
-	if (st[r].done) return;
-	double s[4];
-	sum_part(part, nbv, r, s, 3);
-	if (threadIdx.x) return;
-	RhsState &S = st[r];
-	const double nrm = s[0] + s[1];
-	S.beta = dsqrt(dc(s[0] - s[1], 2 * s[2]));
-	S.om_new = sqrt(nrm) / dabs(S.beta);
-	const double zt2 = S.zetat.x * S.zetat.x + S.zetat.y * S.zetat.y;
-	const double zabs = sqrt(zt2 + nrm);
-	const double zt = sqrt(zt2);
-	const double2 zeta = (zt < 1e-40) ? dc(zabs, 0) : dscal(S.zetat, zabs / zt);
-	S.c_old = S.c_new;
-	S.c_new = zt / zabs;
-	S.s_old = S.s_new;
-	S.s_new = ddiv(dscal(S.beta, S.om_new), zeta);
-	const double2 t4 = dinv(zeta);
-	if (S.niter == 1) {
-		S.k0 = dc(0, 0);
-		S.k1 = dc(0, 0);
+	write_part<3>(part, nbv, s);
+	if (last_block(t.cnt + r, gridDim.x)) {
+		double tot[3];
+		sum_parts<3>(part, nbv, r, tot);
+		if (threadIdx.x < 32) qmr_after_v1(st[r], tot);
 	}
-	else {
-		const double2 t2 = dmul(dc(-S.eta.x, -S.eta.y), t4);
-		S.k1 = t2;
-		S.k0 = (S.niter == 2) ? dc(0, 0) : dmul(dc(-S.theta.x, -S.theta.y), t4);
-	}
-	S.k2 = t4;
-	const double2 tau = dscal(S.tautilda, S.c_new);
-	S.tautilda = dmul(dc(-S.s_new.x, -S.s_new.y), S.tautilda);
-	S.k3 = tau;
-	S.kib = dinv(S.beta);
-	S.d0 = S.s_new.x * S.s_new.x + S.s_new.y * S.s_new.y;
-	S.kr = dscal(S.tautilda, S.c_new / S.om_new);
 }
 
 // p_old = k0*p_old + k1*p_new + k2*v (becomes p_new); x += k3*p; v~ *= 1/beta (becomes v); r = d0*r + kr*v;
 // partial |r|^2
 template <typename C>
-__global__ void __launch_bounds__(NT) qmr_v2(const RhsState *st, C *po, const C *pn, const C *v, C *vt, C *x, C *rv,
-	size_t n3, double *part, int nbv)
+__global__ void __launch_bounds__(NT) qmr_v2(RhsState *st, C *po, const C *pn, const C *v, C *vt, C *x, C *rv,
+	size_t n3, double *part, int nbv, Tail t)
 {
 	const int r = blockIdx.y;
 	if (st[r].done) return;
 	const RhsState &S = st[r];
-	const auto k0 = cof<C>(S.k0), k1 = cof<C>(S.k1), k2 = cof<C>(S.k2), k3 = cof<C>(S.k3), kib = cof<C>(S.kib),
-		kr = cof<C>(S.kr);
-	const auto d0 = rof<C>(S.d0);
+	const Coefs<C, 7> K(S.k0, S.k1, S.k2, S.k3, S.kib, S.kr, dc(S.d0, 0));
+	const auto k0 = K[0], k1 = K[1], k2 = K[2], k3 = K[3], kib = K[4], kr = K[5];
+	const auto d0 = K.re(6);
 	typename AccOf<C>::T s[4] = {};
 	VLOOP(n3) {
 		const size_t j = r * n3 + i;
@@ -423,33 +310,21 @@ __global__ void __launch_bounds__(NT) qmr_v2(const RhsState *st, C *po, const C 
 		rv[j] = rn;
 		acc_abs2(s[0], rn);
 	}
-	write_part(part, nbv, s, 1);
+	write_part<1>(part, nbv, s);
+	// progress in the last block
+	if (last_block(t.cnt + r, gridDim.x)) {
+		double tot[3];
+		sum_parts<1>(part, nbv, r, tot);
+		if (threadIdx.x == 0) progress(st[r], t.done + r, tot, t.hist + (size_t)r * t.hist_cap, t.hist_cap, 0);
+	}
 }
 
-// ProgressReport (iterative.c:282-306) + loop condition (iterative.c:1467); partial |r|^2 in slot 0 unless half
-// mode 0: |r|^2 from partial slot 0; 1: BiCGStab (also the next ro, half-step exit); 2: inprodRp1 already set by the
-// method's scalar kernel (CSYM's |tau|^2)
-__global__ void s_progress(RhsState *st, int *done, const double *part, int nbv, double *hist, int hist_cap, int mode)
+// the progress step as a kernel of its own (methods whose last vector kernel has no sums)
+__global__ void s_progress(RhsState *st, int *done, double *hist, int hist_cap)
 {
 	const int r = blockIdx.x;
-	if (st[r].done) return;
-	double s[4];
-	sum_part(part, nbv, r, s, 2);
-	if (threadIdx.x) return;
-	RhsState &S = st[r];
-	const bool bcgs = mode == 1;
-	if (!S.half && mode != 2) S.inprodRp1 = s[0];
-	if (bcgs && !S.half) S.ro_old = S.ro_new; // the next bs_s0 sums the r.r~* partials of bs_v3 itself
-	if (S.inprodRp1 <= S.inprodR) {
-		S.inprodR = S.inprodRp1;
-		S.counter = 0;
-	}
-	else S.counter++;
-	S.prev_err = sqrt(S.resid_scale * S.inprodRp1);
-	if (S.niter < hist_cap) hist[(size_t)r * hist_cap + S.niter] = S.prev_err;
-	S.niter++;
-	S.done = !(S.inprodR > S.epsB && S.niter <= S.maxiter && S.counter <= S.mc);
-	done[r] = S.done;
+	if (threadIdx.x || st[r].done) return;
+	progress(st[r], done + r, nullptr, hist + (size_t)r * hist_cap, hist_cap, 2);
 }
 
 // ---------------- BiCGStab iteration ----------------
@@ -460,7 +335,7 @@ __global__ void bs_s0(RhsState *st, int *done, const double *part, int nbv)
 	const int r = blockIdx.x;
 	if (st[r].done) return;
 	double s[4];
-	sum_part(part, nbv, r, s, 3);
+	sum_parts<3>(part, nbv, r, s);
 	if (threadIdx.x) return;
 	RhsState &S = st[r];
 	const double2 ro = dc(s[1], s[2]);
@@ -489,41 +364,23 @@ __global__ void __launch_bounds__(NT) bs_v1(const RhsState *st, C *p, const C *v
 {
 	const int r = blockIdx.y;
 	if (st[r].done) return;
-	const auto k0 = cof<C>(st[r].k0), k1 = cof<C>(st[r].k1);
+	const Coefs<C, 2> K(st[r].k0, st[r].k1);
+	const auto k0 = K[0], k1 = K[1];
 	VLOOP(n3) {
 		const size_t j = r * n3 + i;
 		p[j] = cadd(cadd(cmul(k0, p[j]), cmul(k1, v[j])), rv[j]);
 	}
 }
 
-// alpha = ro_new / (v.r~*) (matvec epilogue slot 1,2)
-__global__ void bs_s1(RhsState *st, int *done, const double *part, size_t nblk)
-{
-	const int r = blockIdx.x;
-	if (st[r].done) return;
-	double s[4];
-	sum_part(part, nblk, r, s, 3);
-	if (threadIdx.x) return;
-	RhsState &S = st[r];
-	const double2 t = dc(s[1], s[2]);
-	if (dabs(t) / dabs(S.ro_new) < 1e-10) { // iterative.c:695-697
-		S.status = ADDA_GB300_EBREAKDOWN;
-		S.done = 1;
-		done[r] = 1;
-		return;
-	}
-	S.balpha = ddiv(S.ro_new, t);
-	S.k0 = dc(-S.balpha.x, -S.balpha.y);
-}
-
 // s = k0*v + r ; partial |s|^2
 template <typename C>
-__global__ void __launch_bounds__(NT) bs_v2(const RhsState *st, C *sv, const C *v, const C *rv, size_t n3,
-	double *part, int nbv)
+__global__ void __launch_bounds__(NT) bs_v2(RhsState *st, C *sv, const C *v, const C *rv, size_t n3,
+	double *part, int nbv, Tail t)
 {
 	const int r = blockIdx.y;
 	if (st[r].done) return;
-	const auto k0 = cof<C>(st[r].k0);
+	const Coefs<C, 1> K(st[r].k0);
+	const auto k0 = K[0];
 	typename AccOf<C>::T s[4] = {};
 	VLOOP(n3) {
 		const size_t j = r * n3 + i;
@@ -531,42 +388,24 @@ __global__ void __launch_bounds__(NT) bs_v2(const RhsState *st, C *sv, const C *
 		sv[j] = y;
 		acc_abs2(s[0], y);
 	}
-	write_part(part, nbv, s, 1);
-}
-
-__global__ void bs_s2(RhsState *st, const double *part, int nbv)
-{
-	const int r = blockIdx.x;
-	if (st[r].done) return;
-	double s[4];
-	sum_part(part, nbv, r, s, 1);
-	if (threadIdx.x) return;
-	RhsState &S = st[r];
-	S.inprodRp1 = s[0];
-	S.half = (S.inprodRp1 < S.epsB && !S.full) ? 1 : 0; // converged at the half step (iterative.c:703-707)
-}
-
-// omega = s.t* / |t|^2 (matvec epilogue: slot 0 = |t|^2, slots 1,2 = s.t*)
-__global__ void bs_s3(RhsState *st, const double *part, size_t nblk)
-{
-	const int r = blockIdx.x;
-	if (st[r].done) return;
-	double s[4];
-	sum_part(part, nblk, r, s, 3);
-	if (threadIdx.x) return;
-	RhsState &S = st[r];
-	if (!S.half) S.omega = dscal(dc(s[1], s[2]), 1 / s[0]);
+	write_part<1>(part, nbv, s);
+	if (last_block(t.cnt + r, gridDim.x)) {
+		double tot[1];
+		sum_parts<1>(part, nbv, r, tot);
+		if (threadIdx.x == 0) bs_after_s(st[r], tot);
+	}
 }
 
 // x += alpha*p (+ omega*s); r = -omega*t + s; partials |r|^2, r.r~*
 template <typename C>
-__global__ void __launch_bounds__(NT) bs_v3(const RhsState *st, C *x, const C *p, const C *sv, const C *t, C *rv,
-	const C *rt, size_t n3, double *part, int nbv)
+__global__ void __launch_bounds__(NT) bs_v3(RhsState *st, C *x, const C *p, const C *sv, const C *tv, C *rv,
+	const C *rt, size_t n3, double *part, int nbv, Tail t)
 {
 	const int r = blockIdx.y;
 	if (st[r].done) return;
 	const RhsState &S = st[r];
-	const auto a = cof<C>(S.balpha), om = cof<C>(S.omega), mom = cof<C>(dc(-S.omega.x, -S.omega.y));
+	const Coefs<C, 3> K(S.balpha, S.omega, dneg(S.omega));
+	const auto a = K[0], om = K[1], mom = K[2];
 	const bool half = S.half != 0;
 	typename AccOf<C>::T s[4] = {};
 	VLOOP(n3) {
@@ -576,12 +415,18 @@ __global__ void __launch_bounds__(NT) bs_v3(const RhsState *st, C *x, const C *p
 			continue;
 		}
 		x[j] = cadd(x[j], cadd(cmul(a, p[j]), cmul(om, sv[j])));
-		const C y = cadd(cmul(mom, t[j]), sv[j]);
+		const C y = cadd(cmul(mom, tv[j]), sv[j]);
 		rv[j] = y;
 		acc_abs2(s[0], y);
 		acc_cmulc(s[1], s[2], y, rt[j]);
 	}
-	write_part(part, nbv, s, 3);
+	write_part<3>(part, nbv, s);
+	// progress in the last block
+	if (last_block(t.cnt + r, gridDim.x)) {
+		double tot[3];
+		sum_parts<1>(part, nbv, r, tot);
+		if (threadIdx.x == 0) progress(st[r], t.done + r, tot, t.hist + (size_t)r * t.hist_cap, t.hist_cap, 1);
+	}
 }
 
 // ---------------- BiCG_CS (COCG), iterative.c:490-637 ----------------
@@ -593,7 +438,7 @@ __global__ void bg_s0(RhsState *st, int *done, const double *part, int nbv)
 	const int r = blockIdx.x;
 	if (st[r].done) return;
 	double s[4];
-	sum_part(part, nbv, r, s, 3);
+	sum_parts<3>(part, nbv, r, s);
 	if (threadIdx.x) return;
 	RhsState &S = st[r];
 	S.ro_new = dc(s[1], s[2]);
@@ -612,7 +457,8 @@ template <typename C> __global__ void __launch_bounds__(NT) bg_v1(const RhsState
 	const int r = blockIdx.y;
 	if (st[r].done) return;
 	const bool first = st[r].niter == 1;
-	const auto k0 = cof<C>(st[r].k0);
+	const Coefs<C, 1> K(st[r].k0);
+	const auto k0 = K[0];
 	VLOOP(n3) {
 		const size_t j = r * n3 + i;
 		p[j] = first ? rv[j] : cadd(cmul(k0, p[j]), rv[j]);
@@ -625,7 +471,7 @@ __global__ void bg_s1(RhsState *st, int *done, const double *part, size_t nblk)
 	const int r = blockIdx.x;
 	if (st[r].done) return;
 	double s[4];
-	sum_part(part, nblk, r, s, 3);
+	sum_parts<3>(part, nblk, r, s);
 	if (threadIdx.x) return;
 	RhsState &S = st[r];
 	const double2 mu = dc(s[1], s[2]);
@@ -641,12 +487,13 @@ __global__ void bg_s1(RhsState *st, int *done, const double *part, size_t nblk)
 
 // x += alpha*p; r -= alpha*Ap; partials |r|^2 and r.r
 template <typename C>
-__global__ void __launch_bounds__(NT) bg_v2(const RhsState *st, C *x, const C *p, C *rv, const C *Av, size_t n3,
-	double *part, int nbv)
+__global__ void __launch_bounds__(NT) bg_v2(RhsState *st, C *x, const C *p, C *rv, const C *Av, size_t n3,
+	double *part, int nbv, Tail t)
 {
 	const int r = blockIdx.y;
 	if (st[r].done) return;
-	const auto a = cof<C>(st[r].balpha), ma = cof<C>(dc(-st[r].balpha.x, -st[r].balpha.y));
+	const Coefs<C, 2> K(st[r].balpha, dneg(st[r].balpha));
+	const auto a = K[0], ma = K[1];
 	typename AccOf<C>::T s[4] = {};
 	VLOOP(n3) {
 		const size_t j = r * n3 + i;
@@ -656,7 +503,13 @@ __global__ void __launch_bounds__(NT) bg_v2(const RhsState *st, C *x, const C *p
 		acc_abs2(s[0], y);
 		acc_cmul(s[1], s[2], y, y);
 	}
-	write_part(part, nbv, s, 3);
+	write_part<3>(part, nbv, s);
+	// progress in the last block
+	if (last_block(t.cnt + r, gridDim.x)) {
+		double tot[3];
+		sum_parts<1>(part, nbv, r, tot);
+		if (threadIdx.x == 0) progress(st[r], t.done + r, tot, t.hist + (size_t)r * t.hist_cap, t.hist_cap, 0);
+	}
 }
 
 // ---------------- CGNR, iterative.c:729-769 ----------------
@@ -667,7 +520,7 @@ __global__ void cg_s0(RhsState *st, const double *part, size_t nblk)
 	const int r = blockIdx.x;
 	if (st[r].done) return;
 	double s[4];
-	sum_part(part, nblk, r, s, 1);
+	sum_parts<1>(part, nblk, r, s);
 	if (threadIdx.x) return;
 	RhsState &S = st[r];
 	S.ro_new = dc(s[0], 0);
@@ -680,7 +533,8 @@ template <typename C> __global__ void __launch_bounds__(NT) cg_v1(const RhsState
 	const int r = blockIdx.y;
 	if (st[r].done) return;
 	const bool first = st[r].niter == 1;
-	const auto beta = rof<C>(st[r].k0.x);
+	const Coefs<C, 1> K(dc(st[r].k0.x, 0));
+	const auto beta = K.re(0);
 	VLOOP(n3) {
 		const size_t j = r * n3 + i;
 		p[j] = first ? ahr[j] : cadd(cscale(p[j], beta), ahr[j]);
@@ -693,7 +547,7 @@ __global__ void cg_s1(RhsState *st, const double *part, size_t nblk)
 	const int r = blockIdx.x;
 	if (st[r].done) return;
 	double s[4];
-	sum_part(part, nblk, r, s, 1);
+	sum_parts<1>(part, nblk, r, s);
 	if (threadIdx.x) return;
 	RhsState &S = st[r];
 	S.balpha = dc(S.ro_new.x / s[0], 0);
@@ -702,12 +556,13 @@ __global__ void cg_s1(RhsState *st, const double *part, size_t nblk)
 
 // x += alpha*p; r -= alpha*Ap (real alpha); partial |r|^2
 template <typename C>
-__global__ void __launch_bounds__(NT) cg_v2(const RhsState *st, C *x, const C *p, C *rv, const C *Av, size_t n3,
-	double *part, int nbv)
+__global__ void __launch_bounds__(NT) cg_v2(RhsState *st, C *x, const C *p, C *rv, const C *Av, size_t n3,
+	double *part, int nbv, Tail t)
 {
 	const int r = blockIdx.y;
 	if (st[r].done) return;
-	const auto a = rof<C>(st[r].balpha.x), ma = rof<C>(-st[r].balpha.x);
+	const Coefs<C, 2> K(dc(st[r].balpha.x, 0), dc(-st[r].balpha.x, 0));
+	const auto a = K.re(0), ma = K.re(1);
 	typename AccOf<C>::T s[4] = {};
 	VLOOP(n3) {
 		const size_t j = r * n3 + i;
@@ -716,7 +571,13 @@ __global__ void __launch_bounds__(NT) cg_v2(const RhsState *st, C *x, const C *p
 		rv[j] = y;
 		acc_abs2(s[0], y);
 	}
-	write_part(part, nbv, s, 1);
+	write_part<1>(part, nbv, s);
+	// progress in the last block
+	if (last_block(t.cnt + r, gridDim.x)) {
+		double tot[3];
+		sum_parts<1>(part, nbv, r, tot);
+		if (threadIdx.x == 0) progress(st[r], t.done + r, tot, t.hist + (size_t)r * t.hist_cap, t.hist_cap, 0);
+	}
 }
 
 // ---------------- CSYM, iterative.c:773-892 ----------------
@@ -741,7 +602,8 @@ template <typename C> __global__ void __launch_bounds__(NT) cs_conj_scale(const 
 {
 	const int r = blockIdx.y;
 	if (st[r].done) return;
-	const auto k = rof<C>(st[r].kib.x);
+	const Coefs<C, 1> K(dc(st[r].kib.x, 0));
+	const auto k = K.re(0);
 	VLOOP(n3) {
 		const size_t j = r * n3 + i;
 		a[j] = cscale(cconj(a[j]), k);
@@ -754,7 +616,7 @@ __global__ void cs_s1(RhsState *st, const double *part, size_t nblk)
 	const int r = blockIdx.x;
 	if (st[r].done) return;
 	double s[4];
-	sum_part(part, nblk, r, s, 3);
+	sum_parts<3>(part, nblk, r, s);
 	if (threadIdx.x) return;
 	RhsState &S = st[r];
 	const double2 alpha = dc(s[1], s[2]);
@@ -774,8 +636,9 @@ __global__ void __launch_bounds__(NT) cs_v1(const RhsState *st, C *qo, const C *
 	const int r = blockIdx.y;
 	if (st[r].done) return;
 	const bool first = st[r].niter == 1;
-	const auto k0 = cof<C>(st[r].k0);
-	const auto k1 = rof<C>(st[r].k1.x);
+	const Coefs<C, 2> K(st[r].k0, dc(st[r].k1.x, 0));
+	const auto k0 = K[0];
+	const auto k1 = K.re(1);
 	typename AccOf<C>::T s[4] = {};
 	VLOOP(n3) {
 		const size_t j = r * n3 + i;
@@ -784,7 +647,7 @@ __global__ void __launch_bounds__(NT) cs_v1(const RhsState *st, C *qo, const C *
 		qo[j] = w;
 		acc_abs2(s[0], w);
 	}
-	write_part(part, nbv, s, 1);
+	write_part<1>(part, nbv, s);
 }
 
 // beta_(k+1) = |w|; Givens rotation c_k, s_k, 1/ksi_k (:832-862); p and x coefficients; tau_(k+1) = -s_k*tau_k and
@@ -794,7 +657,7 @@ __global__ void cs_s2(RhsState *st, int *done, const double *part, int nbv)
 	const int r = blockIdx.x;
 	if (st[r].done) return;
 	double s[4];
-	sum_part(part, nbv, r, s, 1);
+	sum_parts<1>(part, nbv, r, s);
 	if (threadIdx.x) return;
 	RhsState &S = st[r];
 	const double beta = sqrt(s[0]);
@@ -845,8 +708,9 @@ __global__ void __launch_bounds__(NT) cs_v2(const RhsState *st, C *po, const C *
 	if (st[r].done) return;
 	const RhsState &S = st[r];
 	const int it = S.niter;
-	const auto k1 = cof<C>(S.k1), k2 = cof<C>(S.k2), k3 = cof<C>(S.k3), kr = cof<C>(S.kr);
-	const auto kib = rof<C>(S.kib.x);
+	const Coefs<C, 5> K(S.k1, S.k2, S.k3, S.kr, dc(S.kib.x, 0));
+	const auto k1 = K[0], k2 = K[1], k3 = K[2], kr = K[3];
+	const auto kib = K.re(4);
 	VLOOP(n3) {
 		const size_t j = r * n3 + i;
 		C pv = cmul(k3, qn[j]);
@@ -866,7 +730,7 @@ __global__ void q2_init_s(RhsState *st, const double *part, int nbv)
 {
 	const int r = blockIdx.x;
 	double s[4];
-	sum_part(part, nbv, r, s, 3);
+	sum_parts<3>(part, nbv, r, s);
 	if (threadIdx.x || st[r].done) return;
 	RhsState &S = st[r];
 	S.q2_ro = sqrt(S.inprodR);
@@ -882,7 +746,7 @@ __global__ void q2_resume_s(RhsState *st, const double *part, int nbv)
 {
 	const int r = blockIdx.x;
 	double s[4];
-	sum_part(part, nbv, r, s, 3);
+	sum_parts<3>(part, nbv, r, s);
 	if (threadIdx.x || st[r].done) return;
 	RhsState &S = st[r];
 	S.q2_delta = dscal(dc(s[1], s[2]), 1 / (S.q2_ro * S.q2_ro));
@@ -910,8 +774,9 @@ template <typename C> __global__ void __launch_bounds__(NT) q2_v1(const RhsState
 	const int r = blockIdx.y;
 	if (st[r].done) return;
 	const bool first = st[r].niter == 1;
-	const auto ir = rof<C>(st[r].kib.x);
-	const auto k0 = cof<C>(st[r].k0);
+	const Coefs<C, 2> K(dc(st[r].kib.x, 0), st[r].k0);
+	const auto k0 = K[1];
+	const auto ir = K.re(0);
 	VLOOP(n3) {
 		const size_t j = r * n3 + i;
 		const C vv = cscale(v[j], ir);
@@ -926,7 +791,7 @@ __global__ void q2_s1(RhsState *st, int *done, const double *part, size_t nblk)
 	const int r = blockIdx.x;
 	if (st[r].done) return;
 	double s[4];
-	sum_part(part, nblk, r, s, 3);
+	sum_parts<3>(part, nblk, r, s);
 	if (threadIdx.x) return;
 	RhsState &S = st[r];
 	S.q2_eps = dc(s[1], s[2]);
@@ -946,7 +811,8 @@ __global__ void __launch_bounds__(NT) q2_v2(const RhsState *st, C *v, const C *A
 {
 	const int r = blockIdx.y;
 	if (st[r].done) return;
-	const auto k1 = cof<C>(st[r].k1);
+	const Coefs<C, 1> K(st[r].k1);
+	const auto k1 = K[0];
 	typename AccOf<C>::T s[4] = {};
 	VLOOP(n3) {
 		const size_t j = r * n3 + i;
@@ -955,7 +821,7 @@ __global__ void __launch_bounds__(NT) q2_v2(const RhsState *st, C *v, const C *A
 		acc_abs2(s[0], y);
 		acc_cmul(s[1], s[2], y, y);
 	}
-	write_part(part, nbv, s, 3);
+	write_part<3>(part, nbv, s);
 }
 
 // ro_(k+1) = |v~_(k+1)|; theta_k, c_k, |s_k|^2, eta_k (:1111-1120); coefficients of d, x, r; delta_(k+1)
@@ -964,7 +830,7 @@ __global__ void q2_s2(RhsState *st, const double *part, int nbv)
 	const int r = blockIdx.x;
 	if (st[r].done) return;
 	double s[4];
-	sum_part(part, nbv, r, s, 3);
+	sum_parts<3>(part, nbv, r, s);
 	if (threadIdx.x) return;
 	RhsState &S = st[r];
 	const double ro_new = sqrt(s[0]);
@@ -987,15 +853,16 @@ __global__ void q2_s2(RhsState *st, const double *part, int nbv)
 
 // d = eta*p (first iteration) or d0*d + eta*p; x += d; r = sabs2*r - eta*v~; partial |r|^2
 template <typename C>
-__global__ void __launch_bounds__(NT) q2_v3(const RhsState *st, C *d, const C *p, C *x, C *rv, const C *v, size_t n3,
-	double *part, int nbv)
+__global__ void __launch_bounds__(NT) q2_v3(RhsState *st, C *d, const C *p, C *x, C *rv, const C *v, size_t n3,
+	double *part, int nbv, Tail t)
 {
 	const int r = blockIdx.y;
 	if (st[r].done) return;
 	const RhsState &S = st[r];
 	const bool first = S.niter == 1;
-	const auto eta = cof<C>(S.k2), me = cof<C>(S.kr);
-	const auto d0 = rof<C>(S.d0), sa = rof<C>(S.k3.x);
+	const Coefs<C, 4> K(S.k2, S.kr, dc(S.d0, 0), dc(S.k3.x, 0));
+	const auto eta = K[0], me = K[1];
+	const auto d0 = K.re(2), sa = K.re(3);
 	typename AccOf<C>::T s[4] = {};
 	VLOOP(n3) {
 		const size_t j = r * n3 + i;
@@ -1006,7 +873,13 @@ __global__ void __launch_bounds__(NT) q2_v3(const RhsState *st, C *d, const C *p
 		rv[j] = y;
 		acc_abs2(s[0], y);
 	}
-	write_part(part, nbv, s, 1);
+	write_part<1>(part, nbv, s);
+	// progress in the last block
+	if (last_block(t.cnt + r, gridDim.x)) {
+		double tot[3];
+		sum_parts<1>(part, nbv, r, tot);
+		if (threadIdx.x == 0) progress(st[r], t.done + r, tot, t.hist + (size_t)r * t.hist_cap, t.hist_cap, 0);
+	}
 }
 
 // ---------------- BCGS2 = BiCGstab(2), iterative.c:340-487 ----------------
@@ -1026,7 +899,7 @@ __global__ void b2_s_beta(RhsState *st, int *done, const double *part, size_t nb
 	const int r = blockIdx.x;
 	if (st[r].done) return;
 	double s[4];
-	sum_part(part, nblk, r, s, 3);
+	sum_parts<3>(part, nblk, r, s);
 	if (threadIdx.x) return;
 	RhsState &S = st[r];
 	const double2 rho1 = dc(s[1], s[2]);
@@ -1052,7 +925,8 @@ __global__ void __launch_bounds__(NT) b2_vu(const RhsState *st, C *u0, const C *
 	const int r = blockIdx.y;
 	if (st[r].done) return;
 	const bool copy = st[r].niter == 1 && j == 0;
-	const auto k0 = cof<C>(st[r].k0);
+	const Coefs<C, 1> K(st[r].k0);
+	const auto k0 = K[0];
 	VLOOP(n3) {
 		const size_t q = r * n3 + i;
 		u0[q] = copy ? r0[q] : cadd(cmul(k0, u0[q]), r0[q]);
@@ -1066,7 +940,7 @@ __global__ void b2_s_alpha(RhsState *st, int *done, const double *part, size_t n
 	const int r = blockIdx.x;
 	if (st[r].done) return;
 	double s[4];
-	sum_part(part, nblk, r, s, 3);
+	sum_parts<3>(part, nblk, r, s);
 	if (threadIdx.x) return;
 	RhsState &S = st[r];
 	const double2 sigma = dc(s[1], s[2]);
@@ -1086,7 +960,8 @@ __global__ void __launch_bounds__(NT) b2_vx(const RhsState *st, C *x, const C *u
 {
 	const int r = blockIdx.y;
 	if (st[r].done) return;
-	const auto a = cof<C>(st[r].b2_alpha), ma = cof<C>(dc(-st[r].b2_alpha.x, -st[r].b2_alpha.y));
+	const Coefs<C, 2> K(st[r].b2_alpha, dneg(st[r].b2_alpha));
+	const auto a = K[0], ma = K[1];
 	typename AccOf<C>::T s[4] = {};
 	VLOOP(n3) {
 		const size_t q = r * n3 + i;
@@ -1098,7 +973,7 @@ __global__ void __launch_bounds__(NT) b2_vx(const RhsState *st, C *x, const C *u
 			acc_abs2(s[0], y);
 		}
 	}
-	if (j == 1) write_part(part, nbv, s, 1);
+	if (j == 1) write_part<1>(part, nbv, s);
 }
 
 // Gram entries Z_11, Z_22, Z_10 = r_0.r_1*, Z_20 = r_0.r_2*, Z_21 = r_1.r_2* (8 slots of xpart)
@@ -1118,13 +993,11 @@ __global__ void __launch_bounds__(NT) b2_gram(const RhsState *st, const C *r0, c
 		acc_cmulc(s[4], s[5], a, c);
 		acc_cmulc(s[6], s[7], b, c);
 	}
-	double v[8];
-	for (int k = 0; k < 8; k++) v[k] = acc_val(s[k]);
-	block_sum4(v, 4);
-	block_sum4(v + 4, 4);
+	double tot[8];
+	block_totals<8>(s, tot);
 	if (threadIdx.x == 0) {
 		double *o = xpart + ((size_t)blockIdx.y * nbv + blockIdx.x) * 8;
-		for (int k = 0; k < 8; k++) o[k] = v[k];
+		for (int k = 0; k < 8; k++) o[k] = tot[k];
 	}
 }
 
@@ -1205,8 +1078,8 @@ __global__ void __launch_bounds__(NT) b2_vfinal(const RhsState *st, C *u0, const
 {
 	const int r = blockIdx.y;
 	if (st[r].done) return;
-	const auto y1 = cof<C>(st[r].b2_y1), y2 = cof<C>(st[r].b2_y2);
-	const auto my1 = cof<C>(dc(-st[r].b2_y1.x, -st[r].b2_y1.y)), my2 = cof<C>(dc(-st[r].b2_y2.x, -st[r].b2_y2.y));
+	const Coefs<C, 4> K(st[r].b2_y1, st[r].b2_y2, dneg(st[r].b2_y1), dneg(st[r].b2_y2));
+	const auto y1 = K[0], y2 = K[1], my1 = K[2], my2 = K[3];
 	typename AccOf<C>::T s[4] = {};
 	VLOOP(n3) {
 		const size_t q = r * n3 + i;
@@ -1217,7 +1090,7 @@ __global__ void __launch_bounds__(NT) b2_vfinal(const RhsState *st, C *u0, const
 		r0[q] = y;
 		acc_cmulc(s[1], s[2], y, rt[q]);
 	}
-	write_part(part, nbv, s, 3);
+	write_part<3>(part, nbv, s);
 }
 
 // ---------------- FP64 helpers for the refinement loop and the results ----------------
@@ -1248,7 +1121,7 @@ __global__ void __launch_bounds__(NT) k_resid64(const double2 *b, const double2 
 		rf[j] = from_d2<C>(d);
 		s[0] += d.x * d.x + d.y * d.y;
 	}
-	write_part(part, nbv, s, 1);
+	write_part<1>(part, nbv, s);
 }
 
 template <typename C> __global__ void __launch_bounds__(NT) k_from64(C *dst, const double2 *src, size_t n)
@@ -1423,9 +1296,11 @@ static int ensure_work(adda_gb300_ctx *c, int R, int hist_cap)
 		ADDA_CUDA(cudaMalloc(&w->av64, vb));
 		for (int i = 0; i < 8; i++) ADDA_CUDA(cudaMalloc(&w->kv[i], vb));
 		ADDA_CUDA(cudaMalloc(&w->st, sizeof(RhsState) * Rm));
-		ADDA_CUDA(cudaMalloc(&w->done, sizeof(int) * Rm));
+		ADDA_CUDA(cudaMalloc(&w->done, sizeof(int) * 2 * Rm));
+		w->cnt = (unsigned *)(w->done + Rm);
+		ADDA_CUDA(cudaMemset(w->cnt, 0, sizeof(unsigned) * Rm));
 		ADDA_CUDA(cudaMallocHost(&w->h_done, sizeof(int) * Rm));
-		w->nbv = (int)std::max<size_t>(1, std::min<size_t>(152 * 8, (n3 + 4 * NT - 1) / (4 * NT)));
+		w->nbv = (int)std::max<size_t>(1, std::min<size_t>(152 * 4, (n3 + NT - 1) / NT)); // the most of vector_blocks
 		ADDA_CUDA(cudaMalloc(&w->vpart, sizeof(double) * Rm * w->nbv * 4));
 		ADDA_CUDA(cudaMalloc(&w->xpart, sizeof(double) * Rm * w->nbv * 8));
 		if (!c->pvec64) ADDA_CUDA(cudaMalloc(&c->pvec64, vb));
@@ -1451,6 +1326,16 @@ static int ensure_work(adda_gb300_ctx *c, int R, int hist_cap)
 	}
 	w->R = R;
 	return ADDA_GB300_OK;
+}
+
+// blocks per RHS of the vector kernels of one solve: FP64 vectors of small particles are bound by the FP64 pipes of the
+// SMs they reach, so they spread out, one element a thread (16^3 sphere, 2 RHS: an iteration 79 -> 68 us); the others
+// take four elements a thread, which amortises the block's coefficients and sums (32^3 cube adjoint solve: 25.0 ms
+// against 26.7)
+static int vector_blocks(size_t n3, bool fp64)
+{
+	const size_t per = fp64 ? NT : 4 * NT;
+	return (int)std::max<size_t>(1, std::min<size_t>(152 * 4, (n3 + per - 1) / per));
 }
 
 void solver_free(adda_gb300_ctx *c)
@@ -1503,21 +1388,16 @@ static int enqueue_iter(adda_gb300_ctx *c, SolverWork *w, int method, int R, int
 	const dim3 gv(w->nbv, R);
 	const size_t nblk = matvec_partial_blocks(c, dbl);
 	cudaStream_t s = c->stream;
+	const Tail tl{w->done, w->hist, w->hist_cap, w->cnt};
 	int rc;
 	if (method == ADDA_ITER_QMR_CS) {
 		C *v = parity ? k.v2 : k.v1, *vt = parity ? k.v1 : k.v2;
 		C *pn = parity ? k.v3 : k.p, *po = parity ? k.p : k.v3;
-		MvEpi e{EPI_DOT_ARG, nullptr, c->partial};
+		const MvEpi e{EPI_DOT_ARG, nullptr, c->partial, TAIL_QMR, w->st, w->done, w->cnt};
 		if ((rc = matvec_run<T>(c, R, v, k.Av, 0, e, w->done))) return rc;
-		qmr_s1<<<R, NT, 0, s>>>(w->st, w->done, c->partial, nblk);
+		qmr_v1<C><<<gv, NT, 0, s>>>(w->st, vt, v, k.Av, n3, w->vpart, w->nbv, tl);
 		ADDA_LAUNCHED();
-		qmr_v1<C><<<gv, NT, 0, s>>>(w->st, vt, v, k.Av, n3, w->vpart, w->nbv);
-		ADDA_LAUNCHED();
-		qmr_s2<<<R, NT, 0, s>>>(w->st, w->vpart, w->nbv);
-		ADDA_LAUNCHED();
-		qmr_v2<C><<<gv, NT, 0, s>>>(w->st, po, pn, v, vt, k.x, k.r, n3, w->vpart, w->nbv);
-		ADDA_LAUNCHED();
-		s_progress<<<R, NT, 0, s>>>(w->st, w->done, w->vpart, w->nbv, w->hist, w->hist_cap, 0);
+		qmr_v2<C><<<gv, NT, 0, s>>>(w->st, po, pn, v, vt, k.x, k.r, n3, w->vpart, w->nbv, tl);
 		ADDA_LAUNCHED();
 	}
 	else if (method == ADDA_ITER_BICG_CS) {
@@ -1529,9 +1409,7 @@ static int enqueue_iter(adda_gb300_ctx *c, SolverWork *w, int method, int R, int
 		if ((rc = matvec_run<T>(c, R, k.p, k.Av, 0, e, w->done))) return rc;
 		bg_s1<<<R, NT, 0, s>>>(w->st, w->done, c->partial, nblk);
 		ADDA_LAUNCHED();
-		bg_v2<C><<<gv, NT, 0, s>>>(w->st, k.x, k.p, k.r, k.Av, n3, w->vpart, w->nbv);
-		ADDA_LAUNCHED();
-		s_progress<<<R, NT, 0, s>>>(w->st, w->done, w->vpart, w->nbv, w->hist, w->hist_cap, 0);
+		bg_v2<C><<<gv, NT, 0, s>>>(w->st, k.x, k.p, k.r, k.Av, n3, w->vpart, w->nbv, tl);
 		ADDA_LAUNCHED();
 	}
 	else if (method == ADDA_ITER_CGNR) {
@@ -1545,9 +1423,7 @@ static int enqueue_iter(adda_gb300_ctx *c, SolverWork *w, int method, int R, int
 		if ((rc = matvec_run<T>(c, R, k.p, k.Av, 0, e2, w->done))) return rc;
 		cg_s1<<<R, NT, 0, s>>>(w->st, c->partial, nblk);
 		ADDA_LAUNCHED();
-		cg_v2<C><<<gv, NT, 0, s>>>(w->st, k.x, k.p, k.r, k.Av, n3, w->vpart, w->nbv);
-		ADDA_LAUNCHED();
-		s_progress<<<R, NT, 0, s>>>(w->st, w->done, w->vpart, w->nbv, w->hist, w->hist_cap, 0);
+		cg_v2<C><<<gv, NT, 0, s>>>(w->st, k.x, k.p, k.r, k.Av, n3, w->vpart, w->nbv, tl);
 		ADDA_LAUNCHED();
 	}
 	else if (method == ADDA_ITER_BCGS2) {
@@ -1574,7 +1450,7 @@ static int enqueue_iter(adda_gb300_ctx *c, SolverWork *w, int method, int R, int
 		ADDA_LAUNCHED();
 		b2_vfinal<C><<<gv, NT, 0, s>>>(w->st, u0, u1, u2, k.x, r0, r1, r2, rt, n3, w->vpart, w->nbv);
 		ADDA_LAUNCHED();
-		s_progress<<<R, NT, 0, s>>>(w->st, w->done, w->vpart, w->nbv, w->hist, w->hist_cap, 2);
+		s_progress<<<R, 32, 0, s>>>(w->st, w->done, w->hist, w->hist_cap);
 		ADDA_LAUNCHED();
 	}
 	else if (method == ADDA_ITER_QMR_CS_2) {
@@ -1591,9 +1467,7 @@ static int enqueue_iter(adda_gb300_ctx *c, SolverWork *w, int method, int R, int
 		ADDA_LAUNCHED();
 		q2_s2<<<R, NT, 0, s>>>(w->st, w->vpart, w->nbv);
 		ADDA_LAUNCHED();
-		q2_v3<C><<<gv, NT, 0, s>>>(w->st, k.v2, k.p, k.x, k.r, k.v1, n3, w->vpart, w->nbv);
-		ADDA_LAUNCHED();
-		s_progress<<<R, NT, 0, s>>>(w->st, w->done, w->vpart, w->nbv, w->hist, w->hist_cap, 0);
+		q2_v3<C><<<gv, NT, 0, s>>>(w->st, k.v2, k.p, k.x, k.r, k.v1, n3, w->vpart, w->nbv, tl);
 		ADDA_LAUNCHED();
 	}
 	else if (method == ADDA_ITER_CSYM) {
@@ -1610,7 +1484,7 @@ static int enqueue_iter(adda_gb300_ctx *c, SolverWork *w, int method, int R, int
 		ADDA_LAUNCHED();
 		cs_v2<C><<<gv, NT, 0, s>>>(w->st, po, pn, qn, qo, k.x, n3);
 		ADDA_LAUNCHED();
-		s_progress<<<R, NT, 0, s>>>(w->st, w->done, w->vpart, w->nbv, w->hist, w->hist_cap, 2);
+		s_progress<<<R, 32, 0, s>>>(w->st, w->done, w->hist, w->hist_cap);
 		ADDA_LAUNCHED();
 	}
 	else {
@@ -1619,21 +1493,13 @@ static int enqueue_iter(adda_gb300_ctx *c, SolverWork *w, int method, int R, int
 		ADDA_LAUNCHED();
 		bs_v1<C><<<gv, NT, 0, s>>>(w->st, k.p, v, k.r, n3);
 		ADDA_LAUNCHED();
-		MvEpi e1{EPI_DOT_U_CONJ, rt, c->partial};
+		const MvEpi e1{EPI_DOT_U_CONJ, rt, c->partial, TAIL_BS_V, w->st, w->done, w->cnt};
 		if ((rc = matvec_run<T>(c, R, k.p, v, 0, e1, w->done))) return rc;
-		bs_s1<<<R, NT, 0, s>>>(w->st, w->done, c->partial, nblk);
+		bs_v2<C><<<gv, NT, 0, s>>>(w->st, sv, v, k.r, n3, w->vpart, w->nbv, tl);
 		ADDA_LAUNCHED();
-		bs_v2<C><<<gv, NT, 0, s>>>(w->st, sv, v, k.r, n3, w->vpart, w->nbv);
-		ADDA_LAUNCHED();
-		bs_s2<<<R, NT, 0, s>>>(w->st, w->vpart, w->nbv);
-		ADDA_LAUNCHED();
-		MvEpi e2{EPI_NORM | EPI_DOT_ARG_CONJ, nullptr, c->partial};
+		const MvEpi e2{EPI_NORM | EPI_DOT_ARG_CONJ, nullptr, c->partial, TAIL_BS_T, w->st, w->done, w->cnt};
 		if ((rc = matvec_run<T>(c, R, sv, k.Av, 0, e2, w->done))) return rc;
-		bs_s3<<<R, NT, 0, s>>>(w->st, c->partial, nblk);
-		ADDA_LAUNCHED();
-		bs_v3<C><<<gv, NT, 0, s>>>(w->st, k.x, k.p, sv, k.Av, k.r, rt, n3, w->vpart, w->nbv);
-		ADDA_LAUNCHED();
-		s_progress<<<R, NT, 0, s>>>(w->st, w->done, w->vpart, w->nbv, w->hist, w->hist_cap, 1);
+		bs_v3<C><<<gv, NT, 0, s>>>(w->st, k.x, k.p, sv, k.Av, k.r, rt, n3, w->vpart, w->nbv, tl);
 		ADDA_LAUNCHED();
 	}
 	return ADDA_GB300_OK;
@@ -2068,6 +1934,7 @@ static int solve_core_impl(adda_gb300_ctx *c, const adda_gb300_solve_params *sp,
 	int rc;
 	const size_t n3 = w->n3;
 	cudaStream_t s = c->stream;
+	w->nbv = vector_blocks(n3, sp->precision == ADDA_PREC_FP64);
 	const dim3 gv(w->nbv, R);
 	const auto t0 = std::chrono::steady_clock::now();
 	const bool resume = sp->init_field == ADDA_IF_CHPOINT;

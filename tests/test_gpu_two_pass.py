@@ -77,3 +77,45 @@ def test_concentrated_spectrum():
     pol = np.array([1.0, 1.0j, -1.0])
     x = np.stack([(np.exp(1j * s.pos @ kk)[:, None] * pol).reshape(-1) for kk in k])
     check(s, x, precs=("fp64",))
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+def test_block_sums_of_extreme_values(prec):
+    """|y|^2 (block sums in fixed point relative to a warp's largest value) of vectors of very different magnitude, of a
+    vector with one large element among tiny ones, of zeros, and of vectors with NaN and infinity"""
+    s = setup_for(dict(grid=16, m=1.5, dpl=10))
+    x = random_vec(s.n, 1, 8)[0]
+    big = 1e15 if prec == "fp32" else 1e100
+    spike = x * (1e-12 / big)
+    spike[5] = big
+    bad = [x.copy(), x.copy()]
+    bad[0][3], bad[1][4] = np.nan, np.inf
+    c = context(s, R=7)
+    y, ip = c.matvec(np.stack([x, x * big, x / big, spike, np.zeros_like(x)] + bad), prec)
+    for r in range(4):
+        # the FP32 sums are of the rounded results in double: both to rounding
+        assert abs(ip[r] / np.sum(np.abs(y[r]) ** 2) - 1) < 1e-12
+    assert ip[4] == 0 and not np.isfinite(ip[5:]).any()
+    c.close()
+
+
+@pytest.mark.parametrize("method", ["qmr", "bicgstab"])
+@pytest.mark.parametrize("grid", [2, 4, 6, 10])
+def test_scalar_steps_in_the_last_block(method, grid):
+    """solves whose vector kernels have one block, and a few, per right-hand side; several right-hand sides of different
+    scale converge independently to the oracle's solution"""
+    from oracle import oracle as O
+    s = setup_for(dict(grid=grid, m=1.3 + 0.1j, dpl=10))
+    o, c = oracle_for(s), context(s, R=3)
+    scale = [1.0, 1e-30, 1e30]
+    e = np.stack([s.einc[0] * k for k in scale])
+    for r in range(3):
+        c.set_cc(r, s.cc[0].reshape(1, 3))
+    o.set_cc(s.cc[0].reshape(1, 3))
+    want = o.solve(s.einc[0], method={"qmr": O.QMR_CS, "bicgstab": O.BICGSTAB}[method], eps=1e-11)["p"]
+    res = c.solve(e, method=method, prec="fp64", eps=1e-11)
+    for r in range(3):
+        assert res["stats"][r]["status"] == "ok"
+        assert rel(res["p"][r] / scale[r], want) < 1e-9
+    o.close()
+    c.close()
