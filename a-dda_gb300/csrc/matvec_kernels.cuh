@@ -111,6 +111,7 @@ template <typename T, typename V, int W, int NS>
 __global__ void __launch_bounds__(col_threads<T, NS, 3 * W>(), (col_minblocks<T, NS, 3 * W>()))
 	mv_scatter_fftx(MvP<T, V> p)
 {
+	chain_entry();
 	typedef typename CxT<T>::type C;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	if (rhs_done(p, blockIdx.z)) return; // blockIdx.z = RHS
@@ -188,6 +189,7 @@ __global__ void __launch_bounds__(col_threads<T, NS, 3 * W>(), (col_minblocks<T,
 template <typename T, int W, int MODE, int NS>
 __global__ void __launch_bounds__(col_threads<T, NS, W>(), (col_minblocks<T, NS, W>())) mv_fftz(MvGeom<T> p)
 {
+	chain_entry();
 	constexpr bool INV = MODE == 1, SGN = MODE != 0;
 	typedef typename CxT<T>::type C;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -276,6 +278,7 @@ __global__ void __launch_bounds__(col_threads<T, NS, W>(), (col_minblocks<T, NS,
 // with its 32 lanes along y (coalesced rows of Tz, odd tile stride: conflict-free).
 template <typename T, int NS, int P> __global__ void __launch_bounds__(256) mv_fft_y_dmul(MvGeom<T> p)
 {
+	chain_entry();
 	typedef typename CxT<T>::type C;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	if (all_done(p)) return;
@@ -352,6 +355,7 @@ template <typename T, int NS, int P> __global__ void __launch_bounds__(256) mv_f
 // transform into Tz. Line l = pair*6 + c6, c6 < 3 from Tz, c6 >= 3 from TzR.
 template <typename T, int NS, int P> __global__ void __launch_bounds__(256) mv_fft_y_surf(MvGeom<T> p)
 {
+	chain_entry();
 	typedef typename CxT<T>::type C;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	if (all_done(p)) return;
@@ -446,6 +450,7 @@ template <int NS, int NT, bool SURF = false>
 __global__ void __launch_bounds__(NT, NS >= 512 ? (NT >= 256 ? 1 : 256 / NT) : (SURF ? 3 : 4) * 128 / NT)
 	mv_fft_y_reg(MvGeom<float> p)
 {
+	chain_entry();
 	typedef float2 C;
 	constexpr int T = RegShape<NS>::T, E = RegShape<NS>::E, BUF = RegShape<NS>::BUF, G = NT / T;
 	constexpr int NSLOT = SURF ? 4 : 3;
@@ -664,6 +669,7 @@ template <typename T, typename V, int W, int NS>
 __global__ void __launch_bounds__(col_threads<T, NS, 3 * W>(), (col_minblocks<T, NS, 3 * W>()))
 	mv_fftx_gather(MvP<T, V> p, MvEpi e)
 {
+	chain_entry();
 	typedef typename CxT<T>::type C;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	if (rhs_done(p, blockIdx.z)) return; // blockIdx.z = RHS
@@ -891,8 +897,8 @@ template <typename T> int launch_yz(adda_gb300_ctx *c, MvGeom<T> p, int ck, cons
 		constexpr int MODE = decltype(mode)::value;
 		if constexpr (sizeof(T) == 4)
 			if (l2z) return l2_fftz_run(c, p, MODE, sh.w2, g2, st);
-		ADDA_NS_SWITCH(c->gZ, ADDA_W_SWITCH(has_w2, sh.w2, (mv_fftz<T, W, MODE, NS><<<g2, col_threads<T, NS, W>(),
-			tile_smem<T>(c->gZ, W), st>>>(p))));
+		ADDA_NS_SWITCH(c->gZ, ADDA_W_SWITCH(has_w2, sh.w2, (launch_next((mv_fftz<T, W, MODE, NS>), g2, col_threads<T, NS, W>(),
+			tile_smem<T>(c->gZ, W), st, p))));
 		ADDA_LAUNCHED();
 		return ADDA_GB300_OK;
 	};
@@ -912,8 +918,8 @@ template <typename T> int launch_yz(adda_gb300_ctx *c, MvGeom<T> p, int ck, cons
 			const size_t sm = k2b_reg_smem(c->gY, nt, surf);
 #define ADDA_K2B_REG(NS_, NT_)                                                                                      \
 	if (c->gY == NS_ && nt == NT_) {                                                                                \
-		if (surf) mv_fft_y_reg<NS_, NT_, true><<<g, NT_, sm, st>>>(p);                                            \
-		else mv_fft_y_reg<NS_, NT_><<<g, NT_, sm, st>>>(p);                                                       \
+		if (surf) launch_next((mv_fft_y_reg<NS_, NT_, true>), g, NT_, sm, st, p);                                            \
+		else launch_next((mv_fft_y_reg<NS_, NT_>), g, NT_, sm, st, p);                                                       \
 	}
 			ADDA_K2B_REG(64, 64) ADDA_K2B_REG(64, 128) ADDA_K2B_REG(64, 256)
 			ADDA_K2B_REG(128, 64) ADDA_K2B_REG(128, 128) ADDA_K2B_REG(128, 256)
@@ -931,10 +937,10 @@ template <typename T> int launch_yz(adda_gb300_ctx *c, MvGeom<T> p, int ck, cons
 		const dim3 g2b((c->gZ + q.KB - 1) / q.KB, ck, (R + q.RG - 1) / q.RG);
 		const size_t sm = 2 * sizeof(typename CxT<T>::type) * (size_t)c->gY * tile_ls(3 * sh.pairs);
 		if (surf) {
-			ADDA_NS_SWITCH(c->gY, ADDA_W_SWITCH(has_pairs, sh.pairs, (mv_fft_y_surf<T, NS, W><<<g2b, 256, sm, st>>>(q))));
+			ADDA_NS_SWITCH(c->gY, ADDA_W_SWITCH(has_pairs, sh.pairs, (launch_next((mv_fft_y_surf<T, NS, W>), g2b, 256, sm, st, q))));
 		}
 		else {
-			ADDA_NS_SWITCH(c->gY, ADDA_W_SWITCH(has_pairs, sh.pairs, (mv_fft_y_dmul<T, NS, W><<<g2b, 256, sm, st>>>(q))));
+			ADDA_NS_SWITCH(c->gY, ADDA_W_SWITCH(has_pairs, sh.pairs, (launch_next((mv_fft_y_dmul<T, NS, W>), g2b, 256, sm, st, q))));
 		}
 	}
 	if (!l2y) ADDA_LAUNCHED();
@@ -1000,8 +1006,8 @@ int launch_matvec(adda_gb300_ctx *c, int R, const V *arg, V *res, int her, const
 		if (l2 && (rc = l2_scatter_run<V>(c, p, sh.w1, g1, st))) return rc;
 	}
 	if (!l2) {
-		ADDA_NS_SWITCH(c->gX, ADDA_W_SWITCH(has_w1, sh.w1, (mv_scatter_fftx<T, V, W, NS><<<g1,
-			col_threads<T, NS, 3 * W>(), tile_smem<T>(c->gX, 3 * W), st>>>(p))));
+		ADDA_NS_SWITCH(c->gX, ADDA_W_SWITCH(has_w1, sh.w1, (launch_next((mv_scatter_fftx<T, V, W, NS>), g1,
+			col_threads<T, NS, 3 * W>(), tile_smem<T>(c->gX, 3 * W), st, p))));
 		ADDA_LAUNCHED();
 	}
 	// the y/z stage chunk by chunk, even chunks on the context stream with Tz, odd ones on the second stream with Tz2
@@ -1029,8 +1035,8 @@ int launch_matvec(adda_gb300_ctx *c, int R, const V *arg, V *res, int her, const
 		if constexpr (dbl) return fx_gather_run(c, p, epi, st);
 		else return l2_gather_run<V>(c, p, sh.w1, g1, epi, st);
 	}
-	ADDA_NS_SWITCH(c->gX, ADDA_W_SWITCH(has_w1, sh.w1, (mv_fftx_gather<T, V, W, NS><<<g1, col_threads<T, NS, 3 * W>(),
-		tile_smem<T>(c->gX, 3 * W), st>>>(p, epi))));
+	ADDA_NS_SWITCH(c->gX, ADDA_W_SWITCH(has_w1, sh.w1, (launch_next((mv_fftx_gather<T, V, W, NS>), g1, col_threads<T, NS, 3 * W>(),
+		tile_smem<T>(c->gX, 3 * W), st, p, epi))));
 	ADDA_LAUNCHED();
 	return ADDA_GB300_OK;
 }

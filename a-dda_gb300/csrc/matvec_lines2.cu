@@ -55,7 +55,7 @@ int l2_fftz_run(adda_gb300_ctx *c, const MvGeom<float> &p, int mode, int w2, dim
 	const int nt = l2_threads(w2, c->p2[2]);
 	const size_t sm = l2_z_smem<Ar32>(c->p2[2], w2);
 #define ADDA_L2Z(W, MODE)                                                                                            \
-	if (w2 == W && mode == MODE) l2_fftz<Ar32, W, MODE, 8><<<g, nt, sm, st>>>(p, q);
+	if (w2 == W && mode == MODE) launch_next((l2_fftz<Ar32, W, MODE, 8>), g, nt, sm, st, p, q);
 	ADDA_L2Z(8, 0) ADDA_L2Z(8, 1) ADDA_L2Z(8, 2) ADDA_L2Z(16, 0) ADDA_L2Z(16, 1) ADDA_L2Z(16, 2)
 	ADDA_L2Z(32, 0) ADDA_L2Z(32, 1) ADDA_L2Z(32, 2)
 #undef ADDA_L2Z
@@ -68,7 +68,7 @@ int l2_ffty_run(adda_gb300_ctx *c, const MvGeom<float> &p, int ck, int pairs, cu
 	const Lines2<Ar32> q = make_lines2<Ar32>(c);
 	const int P = std::max(c->p2[1].r1, c->p2[1].r2), G = pairs;
 	const dim3 g((c->gZ * p.R + G - 1) / G, ck);
-	l2_fft_y<Ar32, 16><<<g, (3 * G * P + 31) / 32 * 32, l2_y_smem<Ar32>(c->p2[1], G), st>>>(p, q, G, P);
+	launch_next((l2_fft_y<Ar32, 16>), g, (3 * G * P + 31) / 32 * 32, l2_y_smem<Ar32>(c->p2[1], G), st, p, q, G, P);
 	ADDA_LAUNCHED();
 	return ADDA_GB300_OK;
 }
@@ -80,13 +80,13 @@ int fx_yz_run(adda_gb300_ctx *c, const MvGeom<double> &p, int ck, cudaStream_t s
 	const dim3 g2((c->bY + W2 - 1) / W2, 3 * ck, p.R);
 	const int ntz = l2_threads(W2, c->p2[2]);
 	const size_t smz = l2_z_smem<ArFx>(c->p2[2], W2);
-	l2_fftz<ArFx, W2, 0, W1><<<g2, ntz, smz, st>>>(p, q);
+	launch_next((l2_fftz<ArFx, W2, 0, W1>), g2, ntz, smz, st, p, q);
 	ADDA_LAUNCHED();
 	const int P = std::max(c->p2[1].r1, c->p2[1].r2), G = std::min(8, 128 / (3 * P));
 	const dim3 g((c->gZ * p.R + G - 1) / G, ck);
-	l2_fft_y<ArFx, W2><<<g, (3 * G * P + 31) / 32 * 32, l2_y_smem<ArFx>(c->p2[1], G), st>>>(p, q, G, P);
+	launch_next((l2_fft_y<ArFx, W2>), g, (3 * G * P + 31) / 32 * 32, l2_y_smem<ArFx>(c->p2[1], G), st, p, q, G, P);
 	ADDA_LAUNCHED();
-	l2_fftz<ArFx, W2, 1, W1><<<g2, ntz, smz, st>>>(p, q);
+	launch_next((l2_fftz<ArFx, W2, 1, W1>), g2, ntz, smz, st, p, q);
 	ADDA_LAUNCHED();
 	return ADDA_GB300_OK;
 }

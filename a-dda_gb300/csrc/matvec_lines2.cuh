@@ -84,6 +84,7 @@ template <class A, typename V, int W, int W2>
 __global__ void __launch_bounds__(32 * ((3 * W * RADIX_MAX + 31) / 32), A::FX ? 512 / (3 * W * RADIX_MAX) : 1)
 	l2_scatter_x(MvP<typename A::T, V> p, Lines2<A> q)
 {
+	chain_entry<!A::FX>();
 	typedef typename A::C C;
 	typedef TileC<A> TC;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -180,6 +181,7 @@ __global__ void __launch_bounds__(32 * ((3 * W * RADIX_MAX + 31) / 32), A::FX ? 
 template <class A, int W, int MODE, int W1>
 __global__ void __launch_bounds__(W * RADIX_MAX, A::FX ? 512 / (W * RADIX_MAX) : 1) l2_fftz(MvGeom<typename A::T> p, Lines2<A> q)
 {
+	chain_entry<!A::FX>();
 	typedef typename A::C C;
 	constexpr bool INV = MODE == 1, SGN = MODE != 0;
 	static_assert(MODE != 2 || !A::FX, "no fixed-point surface mode");
@@ -310,6 +312,7 @@ template <class A, int W2>
 __global__ void __launch_bounds__(A::FX ? 128 : 384, A::FX ? 4 : 2)
 	l2_fft_y(MvGeom<typename A::T> p, Lines2<A> q, int G, int P)
 {
+	chain_entry<!A::FX>();
 	typedef typename A::C C;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	__shared__ unsigned sor[3][8];
@@ -471,6 +474,7 @@ template <class A, typename V, int W, int W2>
 __global__ void __launch_bounds__(32 * ((3 * W * RADIX_MAX + 31) / 32), A::FX ? 512 / (3 * W * RADIX_MAX) : 1)
 	l2_gather_x(MvP<typename A::T, V> p, Lines2<A> q, MvEpi e)
 {
+	chain_entry<!A::FX>();
 	typedef typename A::C C;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	if (rhs_done(p, blockIdx.z)) return; // blockIdx.z = RHS

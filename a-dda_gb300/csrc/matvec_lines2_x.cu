@@ -11,8 +11,8 @@ template <typename V> int l2_scatter_run(adda_gb300_ctx *c, const MvP<float, V> 
 	const Lines2<Ar32> q = make_lines2<Ar32>(c);
 	const int nt = l2_threads(3 * w1, c->p2[0]);
 	const size_t sm = l2_xtile_smem<Ar32>(c->bX, c->p2[0], w1);
-	if (w1 == 4) l2_scatter_x<Ar32, V, 4, 16><<<g, nt, sm, st>>>(p, q);
-	else l2_scatter_x<Ar32, V, 8, 16><<<g, nt, sm, st>>>(p, q);
+	if (w1 == 4) launch_next((l2_scatter_x<Ar32, V, 4, 16>), g, nt, sm, st, p, q);
+	else launch_next((l2_scatter_x<Ar32, V, 8, 16>), g, nt, sm, st, p, q);
 	ADDA_LAUNCHED();
 	return ADDA_GB300_OK;
 }
@@ -23,8 +23,8 @@ int l2_gather_run(adda_gb300_ctx *c, const MvP<float, V> &p, int w1, dim3 g, con
 	const Lines2<Ar32> q = make_lines2<Ar32>(c);
 	const int nt = l2_threads(3 * w1, c->p2[0]);
 	const size_t sm = l2_xtile_smem<Ar32>(c->bX, c->p2[0], w1);
-	if (w1 == 4) l2_gather_x<Ar32, V, 4, 16><<<g, nt, sm, st>>>(p, q, e);
-	else l2_gather_x<Ar32, V, 8, 16><<<g, nt, sm, st>>>(p, q, e);
+	if (w1 == 4) launch_next((l2_gather_x<Ar32, V, 4, 16>), g, nt, sm, st, p, q, e);
+	else launch_next((l2_gather_x<Ar32, V, 8, 16>), g, nt, sm, st, p, q, e);
 	ADDA_LAUNCHED();
 	return ADDA_GB300_OK;
 }
@@ -40,7 +40,7 @@ int fx_scatter_run(adda_gb300_ctx *c, const MvP<double, double2> &p, cudaStream_
 {
 	constexpr int W1 = FX_W1, W2 = FX_W2;
 	const dim3 g((c->bY + W1 - 1) / W1, c->bZ, p.R);
-	l2_scatter_x<ArFx, double2, W1, W2><<<g, l2_threads(3 * W1, c->p2[0]), l2_xtile_smem<ArFx>(c->bX, c->p2[0], W1), st>>>(p,
+	launch_next((l2_scatter_x<ArFx, double2, W1, W2>), g, l2_threads(3 * W1, c->p2[0]), l2_xtile_smem<ArFx>(c->bX, c->p2[0], W1), st, p,
 		make_lines2<ArFx>(c));
 	ADDA_LAUNCHED();
 	return ADDA_GB300_OK;
@@ -50,7 +50,7 @@ int fx_gather_run(adda_gb300_ctx *c, const MvP<double, double2> &p, const MvEpi 
 {
 	constexpr int W1 = FX_W1, W2 = FX_W2;
 	const dim3 g((c->bY + W1 - 1) / W1, c->bZ, p.R);
-	l2_gather_x<ArFx, double2, W1, W2><<<g, l2_threads(3 * W1, c->p2[0]), l2_xtile_smem<ArFx>(c->bX, c->p2[0], W1), st>>>(p,
+	launch_next((l2_gather_x<ArFx, double2, W1, W2>), g, l2_threads(3 * W1, c->p2[0]), l2_xtile_smem<ArFx>(c->bX, c->p2[0], W1), st, p,
 		make_lines2<ArFx>(c), e);
 	ADDA_LAUNCHED();
 	return ADDA_GB300_OK;

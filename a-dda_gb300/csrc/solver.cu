@@ -267,6 +267,7 @@ template <typename C>
 __global__ void __launch_bounds__(NT) qmr_v1(RhsState *st, C *vt, const C *v, const C *Av, size_t n3,
 	double *part, int nbv, Tail t)
 {
+	chain_entry();
 	const int r = blockIdx.y;
 	if (st[r].done) return;
 	const Coefs<C, 2> K(st[r].k0, st[r].k1);
@@ -292,6 +293,7 @@ template <typename C>
 __global__ void __launch_bounds__(NT) qmr_v2(RhsState *st, C *po, const C *pn, const C *v, C *vt, C *x, C *rv,
 	size_t n3, double *part, int nbv, Tail t)
 {
+	chain_entry();
 	const int r = blockIdx.y;
 	if (st[r].done) return;
 	const RhsState &S = st[r];
@@ -332,6 +334,7 @@ __global__ void s_progress(RhsState *st, int *done, double *hist, int hist_cap)
 // ro_new = r.r~* (partial slots 1,2 of the previous bs_v3, or of the initial k_dot for the first iteration)
 __global__ void bs_s0(RhsState *st, int *done, const double *part, int nbv)
 {
+	chain_entry();
 	const int r = blockIdx.x;
 	if (st[r].done) return;
 	double s[4];
@@ -362,6 +365,7 @@ __global__ void bs_s0(RhsState *st, int *done, const double *part, int nbv)
 template <typename C>
 __global__ void __launch_bounds__(NT) bs_v1(const RhsState *st, C *p, const C *v, const C *rv, size_t n3)
 {
+	chain_entry();
 	const int r = blockIdx.y;
 	if (st[r].done) return;
 	const Coefs<C, 2> K(st[r].k0, st[r].k1);
@@ -377,6 +381,7 @@ template <typename C>
 __global__ void __launch_bounds__(NT) bs_v2(RhsState *st, C *sv, const C *v, const C *rv, size_t n3,
 	double *part, int nbv, Tail t)
 {
+	chain_entry();
 	const int r = blockIdx.y;
 	if (st[r].done) return;
 	const Coefs<C, 1> K(st[r].k0);
@@ -401,6 +406,7 @@ template <typename C>
 __global__ void __launch_bounds__(NT) bs_v3(RhsState *st, C *x, const C *p, const C *sv, const C *tv, C *rv,
 	const C *rt, size_t n3, double *part, int nbv, Tail t)
 {
+	chain_entry();
 	const int r = blockIdx.y;
 	if (st[r].done) return;
 	const RhsState &S = st[r];
@@ -1395,9 +1401,9 @@ static int enqueue_iter(adda_gb300_ctx *c, SolverWork *w, int method, int R, int
 		C *pn = parity ? k.v3 : k.p, *po = parity ? k.p : k.v3;
 		const MvEpi e{EPI_DOT_ARG, nullptr, c->partial, TAIL_QMR, w->st, w->done, w->cnt};
 		if ((rc = matvec_run<T>(c, R, v, k.Av, 0, e, w->done))) return rc;
-		qmr_v1<C><<<gv, NT, 0, s>>>(w->st, vt, v, k.Av, n3, w->vpart, w->nbv, tl);
+		launch_next((qmr_v1<C>), gv, NT, 0, s, w->st, vt, v, k.Av, n3, w->vpart, w->nbv, tl);
 		ADDA_LAUNCHED();
-		qmr_v2<C><<<gv, NT, 0, s>>>(w->st, po, pn, v, vt, k.x, k.r, n3, w->vpart, w->nbv, tl);
+		launch_next((qmr_v2<C>), gv, NT, 0, s, w->st, po, pn, v, vt, k.x, k.r, n3, w->vpart, w->nbv, tl);
 		ADDA_LAUNCHED();
 	}
 	else if (method == ADDA_ITER_BICG_CS) {
@@ -1489,17 +1495,17 @@ static int enqueue_iter(adda_gb300_ctx *c, SolverWork *w, int method, int R, int
 	}
 	else {
 		C *v = k.v1, *sv = k.v2, *rt = k.v3;
-		bs_s0<<<R, NT, 0, s>>>(w->st, w->done, w->vpart, w->nbv);
+		launch_next((bs_s0), R, NT, 0, s, w->st, w->done, w->vpart, w->nbv);
 		ADDA_LAUNCHED();
-		bs_v1<C><<<gv, NT, 0, s>>>(w->st, k.p, v, k.r, n3);
+		launch_next((bs_v1<C>), gv, NT, 0, s, w->st, k.p, v, k.r, n3);
 		ADDA_LAUNCHED();
 		const MvEpi e1{EPI_DOT_U_CONJ, rt, c->partial, TAIL_BS_V, w->st, w->done, w->cnt};
 		if ((rc = matvec_run<T>(c, R, k.p, v, 0, e1, w->done))) return rc;
-		bs_v2<C><<<gv, NT, 0, s>>>(w->st, sv, v, k.r, n3, w->vpart, w->nbv, tl);
+		launch_next((bs_v2<C>), gv, NT, 0, s, w->st, sv, v, k.r, n3, w->vpart, w->nbv, tl);
 		ADDA_LAUNCHED();
 		const MvEpi e2{EPI_NORM | EPI_DOT_ARG_CONJ, nullptr, c->partial, TAIL_BS_T, w->st, w->done, w->cnt};
 		if ((rc = matvec_run<T>(c, R, sv, k.Av, 0, e2, w->done))) return rc;
-		bs_v3<C><<<gv, NT, 0, s>>>(w->st, k.x, k.p, sv, k.Av, k.r, rt, n3, w->vpart, w->nbv, tl);
+		launch_next((bs_v3<C>), gv, NT, 0, s, w->st, k.x, k.p, sv, k.Av, k.r, rt, n3, w->vpart, w->nbv, tl);
 		ADDA_LAUNCHED();
 	}
 	return ADDA_GB300_OK;
