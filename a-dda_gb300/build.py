@@ -17,7 +17,8 @@ OUT = os.path.join(HERE, "_build")
 LIB = os.path.join(OUT, "libadda_gb300.so")
 INCLUDE = os.path.join(ROOT, "include")
 
-CU = ["api.cu", "matvec.cu", "matvec_f32.cu", "matvec_yz.cu", "matvec_lines2.cu", "matvec_lines2_x.cu", "dmatrix.cu", "solver.cu", "fields.cu", "noalloc.cu"]
+CU = ["api.cu", "matvec.cu", "matvec_f32.cu", "matvec_yz.cu", "matvec_lines2.cu", "matvec_lines2_x.cu", "matvec_lines2_big.cu",
+      "matvec_lines2_bigfx.cu", "dmatrix.cu", "solver.cu", "fields.cu", "noalloc.cu"]
 C = ["host_setup.c", "integrate.c"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 

@@ -61,19 +61,22 @@ FftPlan make_plan(int n, int max_radix)
 	return p;
 }
 
-// both radices at most RADIX_MAX, as equal as possible; the first pass skips the zero half of a padded line, which
-// an even radix does exactly
-Plan2 make_plan2(int n)
+// the two radices as equal as possible, both at most RADIX_MAX if that can be; the first pass skips the zero half of a
+// padded line, which an even radix does exactly. Up to 512: longer axes take the narrow tiles of the run-time plan
+Plan2 make_plan2(int n, bool fx)
 {
-	Plan2 p{n, 0, 0};
+	Plan2 p{n, 0, 0, false};
 	int best = 1 << 30;
-	for (int a = 1; a <= RADIX_MAX; a++) {
-		if (n % a || n / a > RADIX_MAX) continue;
-		const int b = n / a, cost = 4 * (a + b) + (a % 2 ? 2 : 0) + (a < b ? 1 : 0);
+	for (int a = 1; a <= RADIX_BIG && n <= 512; a++) {
+		if (n % a || n / a > RADIX_BIG || !radix_built(a, fx) || !radix_built(n / a, fx)) continue;
+		const int b = n / a, big = a > RADIX_MAX || b > RADIX_MAX;
+		if (big && std::min(a, b) < 9) continue;
+		const int cost = 4 * (a + b) + (a % 2 ? 2 : 0) + (a < b ? 1 : 0) + (big ? 10000 : 0);
 		if (cost < best) {
 			best = cost;
 			p.r1 = a;
 			p.r2 = b;
+			p.big = big;
 		}
 	}
 	return p;
@@ -152,7 +155,7 @@ static void add_twiddles(adda_gb300_ctx *c, Blob &b, int which, int n)
 // that they can be negated)
 static void add_twiddles2(adda_gb300_ctx *c, Blob &b, int which, bool fx)
 {
-	const Plan2 &p = c->p2[which];
+	const Plan2 &p = fx ? c->p2x[which] : c->p2[which];
 	const double scale = std::ldexp(1.0, 64 - fx_shift(p.n));
 	std::vector<float2> tf[2];
 	std::vector<int4> tx[2];
@@ -175,8 +178,8 @@ static void add_twiddles2(adda_gb300_ctx *c, Blob &b, int which, bool fx)
 				tx[o][at] = make_int4(h[0], h[1], h[2], h[3]);
 			}
 		const int slot = o ? 3 : which;
-		b.add(&c->tw2f[slot], tf[o]);
 		if (fx) b.add(&c->tw2x[slot], tx[o]);
+		else b.add(&c->tw2f[slot], tf[o]);
 	}
 }
 
@@ -271,10 +274,15 @@ static int create_impl(const adda_gb300_problem *p, adda_gb300_ctx *c, const std
 		}
 		add_twiddles(c, tables, d, g3[d]);
 	}
-	for (int d = 0; d < 3; d++) c->p2[d] = make_plan2(g3[d]);
-	c->fx = !c->surface && c->p2[0].r1 && c->p2[1].r1 && c->p2[2].r1;
-	for (int d = 0; d < 3; d++)
-		if (c->p2[d].r1) add_twiddles2(c, tables, d, c->fx);
+	for (int d = 0; d < 3; d++) {
+		c->p2[d] = make_plan2(g3[d], false);
+		c->p2x[d] = make_plan2(g3[d], true);
+	}
+	c->fx = !c->surface && c->p2x[0].r1 && c->p2x[1].r1 && c->p2x[2].r1;
+	for (int d = 0; d < 3; d++) {
+		if (c->p2[d].r1) add_twiddles2(c, tables, d, false);
+		if (c->fx) add_twiddles2(c, tables, d, true);
+	}
 	int rc = tables.upload(&c->tables);
 	if (rc) return rc;
 	// lattices: check order (z, y, x ascending), build per-line dipole ranges. Particle q of a group occupies slot q

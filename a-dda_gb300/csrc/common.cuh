@@ -360,11 +360,20 @@ struct FftPlan {
 	int r[ADDA_FFT_MAXPASS];
 };
 
-// n = r1*r2 of the two-pass line transforms (fft_lines2.cuh; make_plan2 in api.cu); r1 = 0: no such factors
-constexpr int RADIX_MAX = 16;
+// n = r1*r2 of the two-pass line transforms (fft_lines2.cuh; make_plan2 in api.cu); r1 = 0: no such factors. big: a radix
+// above RADIX_MAX (kernels of their own, with more registers)
+constexpr int RADIX_MAX = 16, RADIX_BIG = 32;
 struct Plan2 {
 	int n, r1, r2;
+	bool big;
 };
+// the radices above RADIX_MAX that are built: all products of small primes up to 32 in FP32, fewer in fixed point
+constexpr bool radix_built(int r, bool fx)
+{
+	if (r <= RADIX_MAX) return r >= 1;
+	if (r == 18 || r == 20 || r == 24 || r == 25 || r == 32) return true;
+	return !fx && (r == 21 || r == 22 || r == 26 || r == 27 || r == 28 || r == 30);
+}
 
 // multiply by exp(s*i*theta) given c=cos(theta), s_=s*sin(theta)
 template <typename C> __device__ __forceinline__ C crot(C v, double c, double s_)

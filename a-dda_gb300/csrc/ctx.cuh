@@ -131,7 +131,7 @@ struct adda_gb300_ctx {
 	double2 *tw64[3] = {nullptr, nullptr, nullptr};
 	float2 *tw32[3] = {nullptr, nullptr, nullptr};
 	// two-pass transforms (fft_lines2.cuh): radices and twiddles per axis (x, y, z; [3] the y axis's inverse order)
-	adda::Plan2 p2[3] = {};
+	adda::Plan2 p2[3] = {}, p2x[3] = {}; // FP32, fixed point
 	float2 *tw2f[4] = {nullptr, nullptr, nullptr, nullptr};
 	int4 *tw2x[4] = {nullptr, nullptr, nullptr, nullptr};
 	// FP64 matvec in 64-bit fixed point: all three axes have two-pass plans and there is no substrate
@@ -187,7 +187,7 @@ namespace adda {
 
 // plan.cpp-equivalent helpers (api.cu)
 FftPlan make_plan(int n, int max_radix);
-Plan2 make_plan2(int n);
+Plan2 make_plan2(int n, bool fx);
 
 // dmatrix.cu
 int dmatrix_build(adda_gb300_ctx *c);

@@ -1,7 +1,7 @@
 // fft_lines2.cuh - two-pass transforms of lines whose length is a product of two register radices.
 //
-// A line of n = r1*r2 elements (r1, r2 <= RADIX_MAX, every 7-smooth factor times at most one 11 or 13, so nearly all
-// sizes fftFit gives) is transformed as: element i = j + r2*t; thread j < r2 does DFT_r1 over t in registers, multiplies
+// A line of n = r1*r2 elements (radices up to 32 of the prime factors 2, 3, 5, 7, 11, 13, so nearly all sizes up to 512
+// that fftFit gives) is transformed as: element i = j + r2*t; thread j < r2 does DFT_r1 over t in registers, multiplies
 // by W_n^(j*q) and leaves Y[q][j] in shared memory; thread q < r1 does DFT_r2 over j and holds X[q + r1*p]. One
 // exchange, whatever the radices; they are run-time numbers (block-uniform switches), so one kernel serves all sizes.
 //
@@ -63,6 +63,7 @@ __device__ __forceinline__ long long fx_mulc(long long v, double c)
 // v * (c + i s), compile-time constants; |c| == |s| (odd multiples of pi/4) takes two real products
 __device__ __forceinline__ fx2 crot(fx2 v, double c, double s)
 {
+	if (c == 0) return s > 0 ? fx2{-v.y, v.x} : fx2{v.y, -v.x}; // a quarter turn: 1 is no constant of the products
 	if (c == s) return fx2{fx_mulc(v.x - v.y, c), fx_mulc(v.x + v.y, c)};
 	if (c == -s) return fx2{fx_mulc(v.x + v.y, c), fx_mulc(v.y - v.x, c)};
 	const long long kc = (long long)(c * 9223372036854775808.0), ks = (long long)(s * 9223372036854775808.0);
@@ -289,15 +290,30 @@ template <typename C, int R> __device__ __forceinline__ void dftr(C *v, bool inv
 	else if constexpr (R == 12) dft_coprime<C, 4, 3>(v, inv);
 	else if constexpr (R == 14) dft_coprime<C, 2, 7>(v, inv);
 	else if constexpr (R == 15) dft_coprime<C, 3, 5>(v, inv);
+	else if constexpr (R == 18) dft_coprime<C, 2, 9>(v, inv);
+	else if constexpr (R == 20) dft_coprime<C, 4, 5>(v, inv);
+	else if constexpr (R == 21) dft_coprime<C, 3, 7>(v, inv);
+	else if constexpr (R == 22) dft_coprime<C, 2, 11>(v, inv);
+	else if constexpr (R == 24) dft_coprime<C, 8, 3>(v, inv);
+	else if constexpr (R == 25) dft_twiddled<C, 5, 5>(v, inv);
+	else if constexpr (R == 26) dft_coprime<C, 2, 13>(v, inv);
+	else if constexpr (R == 27) dft_twiddled<C, 9, 3>(v, inv);
+	else if constexpr (R == 28) dft_coprime<C, 4, 7>(v, inv);
+	else if constexpr (R == 30) dft_coprime<C, 2, 15>(v, inv);
 	else static_assert(R < 0, "radix not built");
 }
 
-// the radices of the run-time switches (1 to RADIX_MAX); CALL sees the radix as the constant RR
+// the radices of the run-time switches, by class: RC_SMALL 1 to RADIX_MAX, RC_BIG 9 to RADIX_BIG (a plan is big when one
+// of its radices is above RADIX_MAX; the other is then at least 9). CALL sees the radix as the constant RR
+enum RadixClass { RC_SMALL = 0, RC_BIG = 1 };
+constexpr bool radix_in_class(int r, int rc, bool fx) { return radix_built(r, fx) && (rc == RC_BIG ? r >= 9 : r <= RADIX_MAX); }
 #define ADDA_RADIX_CASE(r, ...)                                                                                     \
-	case r: {                                                                                                       \
-		constexpr int RR = r;                                                                                       \
-		__VA_ARGS__;                                                                                                \
-	} break;
+	case r:                                                                                                         \
+		if constexpr (radix_in_class(r, RC, A::FX)) {                                                               \
+			constexpr int RR = r;                                                                                   \
+			__VA_ARGS__;                                                                                            \
+		}                                                                                                           \
+		break;
 #define ADDA_RADIX_SWITCH(rv, ...)                                                                                  \
 	switch (rv) {                                                                                                   \
 		ADDA_RADIX_CASE(1, __VA_ARGS__) ADDA_RADIX_CASE(2, __VA_ARGS__) ADDA_RADIX_CASE(3, __VA_ARGS__)             \
@@ -305,9 +321,13 @@ template <typename C, int R> __device__ __forceinline__ void dftr(C *v, bool inv
 		ADDA_RADIX_CASE(7, __VA_ARGS__) ADDA_RADIX_CASE(8, __VA_ARGS__) ADDA_RADIX_CASE(9, __VA_ARGS__)             \
 		ADDA_RADIX_CASE(10, __VA_ARGS__) ADDA_RADIX_CASE(11, __VA_ARGS__) ADDA_RADIX_CASE(12, __VA_ARGS__)          \
 		ADDA_RADIX_CASE(13, __VA_ARGS__) ADDA_RADIX_CASE(14, __VA_ARGS__) ADDA_RADIX_CASE(15, __VA_ARGS__)          \
-		ADDA_RADIX_CASE(16, __VA_ARGS__)                                                                            \
+		ADDA_RADIX_CASE(16, __VA_ARGS__) ADDA_RADIX_CASE(18, __VA_ARGS__) ADDA_RADIX_CASE(20, __VA_ARGS__)          \
+		ADDA_RADIX_CASE(21, __VA_ARGS__) ADDA_RADIX_CASE(22, __VA_ARGS__) ADDA_RADIX_CASE(24, __VA_ARGS__)          \
+		ADDA_RADIX_CASE(25, __VA_ARGS__) ADDA_RADIX_CASE(26, __VA_ARGS__) ADDA_RADIX_CASE(27, __VA_ARGS__)          \
+		ADDA_RADIX_CASE(28, __VA_ARGS__) ADDA_RADIX_CASE(30, __VA_ARGS__) ADDA_RADIX_CASE(32, __VA_ARGS__)          \
 		default: break;                                                                                             \
 	}
+constexpr int radix_max(int rc) { return rc == RC_BIG ? RADIX_BIG : RADIX_MAX; }
 
 // ---------------------------------------------------------------------------------------------------------------
 // the two passes
@@ -345,7 +365,7 @@ __device__ __forceinline__ void pass_first(LD ld, typename A::C *xb, int ks, int
 	C v[R];
 #pragma unroll
 	for (int t = 0; t < L; t++) v[t] = ld(t, j + r2 * t);
-	if constexpr (HALF && !A::FX && (R == 8 || R == 16)) dft_half_in<C, R>(v, INV);
+	if constexpr (HALF && !A::FX && (R == 8 || R == 16 || R == 32)) dft_half_in<C, R>(v, INV);
 	else {
 #pragma unroll
 		for (int t = L; t < R; t++) v[t] = cx<C>(0, 0);

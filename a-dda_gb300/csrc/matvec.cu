@@ -5,10 +5,6 @@
 namespace adda {
 
 int matvec_setup_f32(adda_gb300_ctx *c); // matvec_f32.cu
-namespace mv {
-int l2_setup_yz(); // matvec_lines2.cu
-int l2_setup_x();  // matvec_lines2_x.cu
-} // namespace mv
 
 namespace {
 
@@ -27,7 +23,10 @@ __global__ void reduce_partials_k(const double *partial, size_t nblk, double *ou
 size_t matvec_partial_blocks(const adda_gb300_ctx *c, bool dbl)
 {
 	// K3 grid: ceil(bY/w1) x bZ blocks per RHS
-	const int w = dbl && mv::use_fx(c) ? mv::FX_W1 : c->shape[dbl ? 0 : 1].w1;
+	const MvShape &s = c->shape[dbl ? 0 : 1];
+	int w = s.w1;
+	if (dbl && mv::use_fx(c)) w = mv::FX_W1;
+	else if (!dbl && mv::use_l2_x(c, s) && c->p2[0].big) w = mv::L2_BIG_W1;
 	return (size_t)((c->bY + w - 1) / w) * c->bZ;
 }
 
@@ -52,9 +51,7 @@ int matvec_setup(adda_gb300_ctx *c)
 		return ADDA_GB300_EINVAL;
 	}
 	int rc = mv::set_attrs_tv<double, double2>();
-	if (rc || (rc = mv::setup_yz<double>()) || (rc = mv::setup_yz<float>()) || (rc = mv::l2_setup_yz()) ||
-		(rc = mv::l2_setup_x()))
-		return rc;
+	if (rc || (rc = mv::setup_yz<double>()) || (rc = mv::setup_yz<float>())) return rc;
 	return matvec_setup_f32(c);
 }
 

@@ -869,14 +869,25 @@ inline bool use_l2_f32(const adda_gb300_ctx *c, int axis, int n) { return static
 inline bool use_l2_x(const adda_gb300_ctx *c, const MvShape &s) { return use_l2_f32(c, 0, c->gX) && s.w1 >= 4; }
 inline bool use_l2_z(const adda_gb300_ctx *c, const MvShape &s) { return use_l2_f32(c, 2, c->gZ) && s.w2 >= 8; }
 inline bool use_l2_y(const adda_gb300_ctx *c) { return use_l2_f32(c, 1, c->gY) && !c->surface; }
-int l2_fftz_run(adda_gb300_ctx *c, const MvGeom<float> &p, int mode, int w2, dim3 g, cudaStream_t st);
+// y-lines per K1/K3 block of an x axis with a radix above 16 (one width, whatever the shape says)
+constexpr int L2_BIG_W1 = 4;
+int l2_fftz_run(adda_gb300_ctx *c, const MvGeom<float> &p, int mode, int w2, int ck, cudaStream_t st);
 int l2_ffty_run(adda_gb300_ctx *c, const MvGeom<float> &p, int ck, int pairs, cudaStream_t st);
-template <typename V> int l2_scatter_run(adda_gb300_ctx *c, const MvP<float, V> &p, int w1, dim3 g, cudaStream_t st);
+template <typename V> int l2_scatter_run(adda_gb300_ctx *c, const MvP<float, V> &p, int w1, cudaStream_t st);
 template <typename V>
-int l2_gather_run(adda_gb300_ctx *c, const MvP<float, V> &p, int w1, dim3 g, const MvEpi &e, cudaStream_t st);
+int l2_gather_run(adda_gb300_ctx *c, const MvP<float, V> &p, int w1, const MvEpi &e, cudaStream_t st);
 int fx_scatter_run(adda_gb300_ctx *c, const MvP<double, double2> &p, cudaStream_t st);
 int fx_gather_run(adda_gb300_ctx *c, const MvP<double, double2> &p, const MvEpi &e, cudaStream_t st);
 int fx_yz_run(adda_gb300_ctx *c, const MvGeom<double> &p, int ck, cudaStream_t st);
+// the same for plans with a radix above 16 (matvec_lines2_big.cu, matvec_lines2_bigfx.cu)
+int l2_fftz_big(adda_gb300_ctx *c, const MvGeom<float> &p, int mode, int ck, cudaStream_t st);
+int l2_ffty_big(adda_gb300_ctx *c, const MvGeom<float> &p, int ck, int pairs, cudaStream_t st);
+template <typename V> int l2_scatter_big(adda_gb300_ctx *c, const MvP<float, V> &p, cudaStream_t st);
+template <typename V> int l2_gather_big(adda_gb300_ctx *c, const MvP<float, V> &p, const MvEpi &e, cudaStream_t st);
+int fx_fftz_big(adda_gb300_ctx *c, const MvGeom<double> &p, int mode, int ck, cudaStream_t st);
+int fx_ffty_big(adda_gb300_ctx *c, const MvGeom<double> &p, int ck, cudaStream_t st);
+int fx_scatter_big(adda_gb300_ctx *c, const MvP<double, double2> &p, cudaStream_t st);
+int fx_gather_big(adda_gb300_ctx *c, const MvP<double, double2> &p, const MvEpi &e, cudaStream_t st);
 
 // the y/z stage of one chunk of x-slabs (K2a, [K2a surface], K2b, K2c) with the context's tile shape, on stream st
 template <typename T> int launch_yz(adda_gb300_ctx *c, MvGeom<T> p, int ck, const MvShape &sh, cudaStream_t st)
@@ -896,7 +907,7 @@ template <typename T> int launch_yz(adda_gb300_ctx *c, MvGeom<T> p, int ck, cons
 	auto fftz = [&](auto mode) {
 		constexpr int MODE = decltype(mode)::value;
 		if constexpr (sizeof(T) == 4)
-			if (l2z) return l2_fftz_run(c, p, MODE, sh.w2, g2, st);
+			if (l2z) return l2_fftz_run(c, p, MODE, sh.w2, ck, st);
 		ADDA_NS_SWITCH(c->gZ, ADDA_W_SWITCH(has_w2, sh.w2, (launch_next((mv_fftz<T, W, MODE, NS>), g2, col_threads<T, NS, W>(),
 			tile_smem<T>(c->gZ, W), st, p))));
 		ADDA_LAUNCHED();
@@ -1003,7 +1014,7 @@ int launch_matvec(adda_gb300_ctx *c, int R, const V *arg, V *res, int her, const
 	}
 	else {
 		l2 = use_l2_x(c, sh);
-		if (l2 && (rc = l2_scatter_run<V>(c, p, sh.w1, g1, st))) return rc;
+		if (l2 && (rc = l2_scatter_run<V>(c, p, sh.w1, st))) return rc;
 	}
 	if (!l2) {
 		ADDA_NS_SWITCH(c->gX, ADDA_W_SWITCH(has_w1, sh.w1, (launch_next((mv_scatter_fftx<T, V, W, NS>), g1,
@@ -1033,7 +1044,7 @@ int launch_matvec(adda_gb300_ctx *c, int R, const V *arg, V *res, int her, const
 	}
 	if (l2) {
 		if constexpr (dbl) return fx_gather_run(c, p, epi, st);
-		else return l2_gather_run<V>(c, p, sh.w1, g1, epi, st);
+		else return l2_gather_run<V>(c, p, sh.w1, epi, st);
 	}
 	ADDA_NS_SWITCH(c->gX, ADDA_W_SWITCH(has_w1, sh.w1, (launch_next((mv_fftx_gather<T, V, W, NS>), g1, col_threads<T, NS, 3 * W>(),
 		tile_smem<T>(c->gX, 3 * W), st, p, epi))));

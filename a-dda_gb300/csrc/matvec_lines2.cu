@@ -49,59 +49,28 @@ __global__ void __launch_bounds__(128) fx_drow(const double2 *D, int4 *Dfx, int 
 	if (threadIdx.x == 0) eD[blockIdx.x] = h >= 0x7ff00000 ? FX_BAD : emax - 1075 - (up + FX_TOP - 53);
 }
 
-int l2_fftz_run(adda_gb300_ctx *c, const MvGeom<float> &p, int mode, int w2, dim3 g, cudaStream_t st)
+int l2_fftz_run(adda_gb300_ctx *c, const MvGeom<float> &p, int mode, int w2, int ck, cudaStream_t st)
 {
-	const Lines2<Ar32> q = make_lines2<Ar32>(c);
-	const int nt = l2_threads(w2, c->p2[2]);
-	const size_t sm = l2_z_smem<Ar32>(c->p2[2], w2);
+	if (c->p2[2].big) return l2_fftz_big(c, p, mode, ck, st);
 #define ADDA_L2Z(W, MODE)                                                                                            \
-	if (w2 == W && mode == MODE) launch_next((l2_fftz<Ar32, W, MODE, 8>), g, nt, sm, st, p, q);
+	if (w2 == W && mode == MODE) return l2_z<Ar32, W, MODE, 8, RC_SMALL>(c, p, ck, st);
 	ADDA_L2Z(8, 0) ADDA_L2Z(8, 1) ADDA_L2Z(8, 2) ADDA_L2Z(16, 0) ADDA_L2Z(16, 1) ADDA_L2Z(16, 2)
 	ADDA_L2Z(32, 0) ADDA_L2Z(32, 1) ADDA_L2Z(32, 2)
 #undef ADDA_L2Z
-	ADDA_LAUNCHED();
-	return ADDA_GB300_OK;
+	return ADDA_GB300_EINVAL;
 }
 
 int l2_ffty_run(adda_gb300_ctx *c, const MvGeom<float> &p, int ck, int pairs, cudaStream_t st)
 {
-	const Lines2<Ar32> q = make_lines2<Ar32>(c);
-	const int P = std::max(c->p2[1].r1, c->p2[1].r2), G = pairs;
-	const dim3 g((c->gZ * p.R + G - 1) / G, ck);
-	launch_next((l2_fft_y<Ar32, 16>), g, (3 * G * P + 31) / 32 * 32, l2_y_smem<Ar32>(c->p2[1], G), st, p, q, G, P);
-	ADDA_LAUNCHED();
-	return ADDA_GB300_OK;
+	return c->p2[1].big ? l2_ffty_big(c, p, ck, pairs, st) : l2_y<Ar32, 16, RC_SMALL>(c, p, ck, pairs, st);
 }
 
 int fx_yz_run(adda_gb300_ctx *c, const MvGeom<double> &p, int ck, cudaStream_t st)
 {
-	constexpr int W1 = FX_W1, W2 = FX_W2;
-	const Lines2<ArFx> q = make_lines2<ArFx>(c);
-	const dim3 g2((c->bY + W2 - 1) / W2, 3 * ck, p.R);
-	const int ntz = l2_threads(W2, c->p2[2]);
-	const size_t smz = l2_z_smem<ArFx>(c->p2[2], W2);
-	launch_next((l2_fftz<ArFx, W2, 0, W1>), g2, ntz, smz, st, p, q);
-	ADDA_LAUNCHED();
-	const int P = std::max(c->p2[1].r1, c->p2[1].r2), G = std::min(8, 128 / (3 * P));
-	const dim3 g((c->gZ * p.R + G - 1) / G, ck);
-	launch_next((l2_fft_y<ArFx, W2>), g, (3 * G * P + 31) / 32 * 32, l2_y_smem<ArFx>(c->p2[1], G), st, p, q, G, P);
-	ADDA_LAUNCHED();
-	launch_next((l2_fftz<ArFx, W2, 1, W1>), g2, ntz, smz, st, p, q);
-	ADDA_LAUNCHED();
-	return ADDA_GB300_OK;
-}
-
-int l2_setup_yz()
-{
-	constexpr int W1 = FX_W1, W2 = FX_W2;
-	ADDA_L2_SMEM((l2_fftz<ArFx, W2, 0, W1>));
-	ADDA_L2_SMEM((l2_fftz<ArFx, W2, 1, W1>));
-	ADDA_L2_SMEM((l2_fft_y<ArFx, W2>));
-	ADDA_L2_SMEM((l2_fft_y<Ar32, 16>));
-	ADDA_L2_SMEM((l2_fftz<Ar32, 32, 0, 8>));
-	ADDA_L2_SMEM((l2_fftz<Ar32, 32, 1, 8>));
-	ADDA_L2_SMEM((l2_fftz<Ar32, 32, 2, 8>));
-	return ADDA_GB300_OK;
+	int rc = c->p2x[2].big ? fx_fftz_big(c, p, 0, ck, st) : l2_z<ArFx, FX_W2, 0, FX_W1, RC_SMALL>(c, p, ck, st);
+	if (!rc) rc = c->p2x[1].big ? fx_ffty_big(c, p, ck, st) : l2_y<ArFx, FX_W2, RC_SMALL>(c, p, ck, 0, st);
+	if (!rc) rc = c->p2x[2].big ? fx_fftz_big(c, p, 1, ck, st) : l2_z<ArFx, FX_W2, 1, FX_W1, RC_SMALL>(c, p, ck, st);
+	return rc;
 }
 
 } // namespace mv

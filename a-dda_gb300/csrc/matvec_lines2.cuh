@@ -80,8 +80,8 @@ __device__ __forceinline__ void st_cs(fx2 *p, fx2 v) { __stcs(reinterpret_cast<l
 template <class A> using TileC = typename CxT<typename A::T>::type;
 
 // K1: S.x of W x-lines (one z) into a tile, then the x transform of its 3W lines
-template <class A, typename V, int W, int W2>
-__global__ void __launch_bounds__(32 * ((3 * W * RADIX_MAX + 31) / 32), A::FX ? 512 / (3 * W * RADIX_MAX) : 1)
+template <class A, typename V, int W, int W2, int RC>
+__global__ void __launch_bounds__(32 * ((3 * W * radix_max(RC) + 31) / 32), A::FX && RC == RC_SMALL ? 512 / (3 * W * RADIX_MAX) : 1)
 	l2_scatter_x(MvP<typename A::T, V> p, Lines2<A> q)
 {
 	chain_entry<!A::FX>();
@@ -178,8 +178,8 @@ __global__ void __launch_bounds__(32 * ((3 * W * RADIX_MAX + 31) / 32), A::FX ? 
 
 // K2a (MODE 0), K2c (MODE 1) and K2a of the reflected transform (MODE 2, FP32: the inverse sign into TzR): the z
 // transform of W y-lines of one (RHS, kx, component)
-template <class A, int W, int MODE, int W1>
-__global__ void __launch_bounds__(W * RADIX_MAX, A::FX ? 512 / (W * RADIX_MAX) : 1) l2_fftz(MvGeom<typename A::T> p, Lines2<A> q)
+template <class A, int W, int MODE, int W1, int RC>
+__global__ void __launch_bounds__(W * radix_max(RC), A::FX && RC == RC_SMALL ? 512 / (W * RADIX_MAX) : 1) l2_fftz(MvGeom<typename A::T> p, Lines2<A> q)
 {
 	chain_entry<!A::FX>();
 	typedef typename A::C C;
@@ -308,8 +308,8 @@ __device__ __forceinline__ fx2 fx_dot3(int4 a, int4 b, int4 c, const FxV &u, con
 // shared slot. Pass 1 leaves Y[q][j] in row q; from there thread q works in its own row (second pass, first inverse
 // pass), and the second inverse pass reads columns. The D product takes the three components of row q's elements
 // c, c+3, ... (c the thread's component). Rows are r2|1 long: every phase is free of bank conflicts.
-template <class A, int W2>
-__global__ void __launch_bounds__(A::FX ? 128 : 384, A::FX ? 4 : 2)
+template <class A, int W2, int RC>
+__global__ void __launch_bounds__(A::FX ? 128 : 384, RC == RC_BIG ? (A::FX ? 2 : 1) : (A::FX ? 4 : 2))
 	l2_fft_y(MvGeom<typename A::T> p, Lines2<A> q, int G, int P)
 {
 	chain_entry<!A::FX>();
@@ -470,8 +470,8 @@ __global__ void __launch_bounds__(A::FX ? 128 : 384, A::FX ? 4 : 2)
 }
 
 // K3: inverse x transform of W y-lines (one z), then y = x + S.X for their dipoles with the epilogue reductions
-template <class A, typename V, int W, int W2>
-__global__ void __launch_bounds__(32 * ((3 * W * RADIX_MAX + 31) / 32), A::FX ? 512 / (3 * W * RADIX_MAX) : 1)
+template <class A, typename V, int W, int W2, int RC>
+__global__ void __launch_bounds__(32 * ((3 * W * radix_max(RC) + 31) / 32), A::FX && RC == RC_SMALL ? 512 / (3 * W * RADIX_MAX) : 1)
 	l2_gather_x(MvP<typename A::T, V> p, Lines2<A> q, MvEpi e)
 {
 	chain_entry<!A::FX>();
@@ -579,9 +579,10 @@ inline FxExp fx_tables(const adda_gb300_ctx *c, size_t *ints = nullptr)
 template <class A> inline Lines2<A> make_lines2(const adda_gb300_ctx *c)
 {
 	Lines2<A> q;
-	q.px = c->p2[0];
-	q.py = c->p2[1];
-	q.pz = c->p2[2];
+	const Plan2 *p = A::FX ? c->p2x : c->p2;
+	q.px = p[0];
+	q.py = p[1];
+	q.pz = p[2];
 	if constexpr (A::FX) {
 		q.tx = c->tw2x[0];
 		q.ty = c->tw2x[1];
@@ -600,9 +601,59 @@ template <class A> inline Lines2<A> make_lines2(const adda_gb300_ctx *c)
 	}
 	return q;
 }
-// opt-in of a kernel to the shared memory of large blocks, once per kernel and device
-#define ADDA_L2_SMEM(kern) ADDA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_CAP))
+// launch of a kernel; shared memory near the default limit (48 KB with the static part) and above is opted in to, once
+// per kernel and device
+template <auto KERN, typename... Ar>
+inline int l2_launch(const adda_gb300_ctx *c, dim3 g, int nt, size_t sm, cudaStream_t st, const Ar &...args)
+{
+	static std::atomic<unsigned long long> opted{0};
+	const unsigned long long bit = 1ull << (c->device & 63);
+	if (sm > 32 * 1024 && !(opted.load(std::memory_order_acquire) & bit)) {
+		ADDA_CUDA(cudaFuncSetAttribute(KERN, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_CAP));
+		opted.fetch_or(bit, std::memory_order_release);
+	}
+	launch_next(KERN, g, dim3(nt), sm, st, args...);
+	ADDA_LAUNCHED();
+	return ADDA_GB300_OK;
+}
 inline int l2_threads(int lines, const Plan2 &p) { return (lines * std::max(p.r1, p.r2) + 31) / 32 * 32; }
+
+// columns per block of the y kernel: as asked for in FP32, 128 threads in fixed point
+template <class A> inline int l2_columns(const Plan2 &p, int pairs)
+{
+	const int t = 3 * std::max(p.r1, p.r2);
+	return std::max(1, std::min(A::FX ? 8 : pairs, (A::FX ? 128 : 384) / t));
+}
+
+template <class A, int W, int MODE, int W1, int RC>
+inline int l2_z(adda_gb300_ctx *c, const MvGeom<typename A::T> &p, int ck, cudaStream_t st)
+{
+	const Lines2<A> q = make_lines2<A>(c);
+	const dim3 g((c->bY + W - 1) / W, 3 * ck, p.R);
+	return l2_launch<l2_fftz<A, W, MODE, W1, RC>>(c, g, l2_threads(W, q.pz), l2_z_smem<A>(q.pz, W), st, p, q);
+}
+template <class A, int W2, int RC>
+inline int l2_y(adda_gb300_ctx *c, const MvGeom<typename A::T> &p, int ck, int pairs, cudaStream_t st)
+{
+	const Lines2<A> q = make_lines2<A>(c);
+	const int P = std::max(q.py.r1, q.py.r2), G = l2_columns<A>(q.py, pairs);
+	const dim3 g((c->gZ * p.R + G - 1) / G, ck);
+	return l2_launch<l2_fft_y<A, W2, RC>>(c, g, (3 * G * P + 31) / 32 * 32, l2_y_smem<A>(q.py, G), st, p, q, G, P);
+}
+template <class A, typename V, int W, int W2, int RC>
+inline int l2_k1(adda_gb300_ctx *c, const MvP<typename A::T, V> &p, cudaStream_t st)
+{
+	const Lines2<A> q = make_lines2<A>(c);
+	const dim3 g((c->bY + W - 1) / W, c->bZ, p.R);
+	return l2_launch<l2_scatter_x<A, V, W, W2, RC>>(c, g, l2_threads(3 * W, q.px), l2_xtile_smem<A>(c->bX, q.px, W), st, p, q);
+}
+template <class A, typename V, int W, int W2, int RC>
+inline int l2_k3(adda_gb300_ctx *c, const MvP<typename A::T, V> &p, const MvEpi &e, cudaStream_t st)
+{
+	const Lines2<A> q = make_lines2<A>(c);
+	const dim3 g((c->bY + W - 1) / W, c->bZ, p.R);
+	return l2_launch<l2_gather_x<A, V, W, W2, RC>>(c, g, l2_threads(3 * W, q.px), l2_xtile_smem<A>(c->bX, q.px, W), st, p, q, e);
+}
 
 } // namespace mv
 } // namespace adda

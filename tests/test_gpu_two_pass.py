@@ -1,5 +1,4 @@
-"""The matvec on two-pass transforms (axis lengths n = r1*r2 with radices up to 16): every FP64 matvec, in 64-bit fixed
-point, and the FP32 matvec of lengths without compile-time kernels.
+"""The matvec on two-pass transforms (axis lengths n = r1*r2 with radices up to 32): the FP64 matvec, in 64-bit fixed point, and the FP32 matvec of lengths without compile-time kernels.
 
 FP64 tolerance: a transform adds noise of about 2^-54 of its block's largest value, six transforms and the D product
 follow one another, and the largest value of these random data is below 16 times their rms: 7 * 16 * 2^-54 = 6e-15.
@@ -13,9 +12,12 @@ from test_gpu_parity import context, cube_setup, random_vec
 pytestmark = pytest.mark.gpu
 TOL64, TOL32 = 6e-15, 5e-6
 
-# lengths whose plans hold every radix from 1 to 16 in the first and in the second pass
+# lengths whose plans hold every radix in the first or the second pass
 LENGTHS = [2, 4, 6, 10, 14, 18, 22, 26, 32, 36, 44, 52, 70, 78, 80, 90, 96, 98, 110, 130, 132, 154, 156, 168, 180, 182,
            196, 208, 210, 224, 240, 256]
+# radices above 16 (FP32: 18 to 32; fixed point: 18, 20, 24, 25, 32, the other lengths fall back to FP64 instructions)
+LENGTHS += [162, 198, 200, 216, 220, 234, 250, 252, 264, 288, 294, 300, 308, 324, 336, 350, 352, 360, 364, 378, 390, 396,
+            400, 416, 432, 448, 450, 480, 486, 500, 512]
 
 
 def check(s, x, her=False, precs=("fp64", "fp32")):
