@@ -278,7 +278,7 @@ static int create_impl(const adda_gb300_problem *p, adda_gb300_ctx *c, const std
 		c->p2[d] = make_plan2(g3[d], false);
 		c->p2x[d] = make_plan2(g3[d], true);
 	}
-	c->fx = !c->surface && c->p2x[0].r1 && c->p2x[1].r1 && c->p2x[2].r1;
+	c->fx = c->p2x[0].r1 && c->p2x[1].r1 && c->p2x[2].r1;
 	for (int d = 0; d < 3; d++) {
 		if (c->p2[d].r1) add_twiddles2(c, tables, d, false);
 		if (c->fx) add_twiddles2(c, tables, d, true);
@@ -349,7 +349,7 @@ static int create_impl(const adda_gb300_problem *p, adda_gb300_ctx *c, const std
 		ADDA_CUDA(cudaMalloc(&c->Dfx, sizeof(int4) * dlen));
 		// every top below every exponent (each byte 0x80: far below FX_LOW), as each matvec leaves them
 		const size_t ne = fx_exps_ints(c);
-		ADDA_CUDA(cudaMalloc(&c->fx_exps, sizeof(int) * (ne + (size_t)c->gX * c->DsZ)));
+		ADDA_CUDA(cudaMalloc(&c->fx_exps, sizeof(int) * (ne + (size_t)c->gX * (c->DsZ + (c->surface ? c->gZ : 0)))));
 		ADDA_CUDA(cudaMemset(c->fx_exps, 0x80, sizeof(int) * ne));
 		c->fx_eD = c->fx_exps + ne;
 	}
@@ -357,6 +357,7 @@ static int create_impl(const adda_gb300_problem *p, adda_gb300_ctx *c, const std
 		const size_t rlen = (size_t)c->gX * c->gZ * (c->gY / 2 + 1) * 6;
 		ADDA_CUDA(cudaMalloc(&c->R64, sizeof(double2) * rlen));
 		ADDA_CUDA(cudaMalloc(&c->R32, sizeof(float2) * rlen));
+		if (c->fx) ADDA_CUDA(cudaMalloc(&c->Rfx, sizeof(int4) * rlen));
 	}
 	// matvec work: Xf for Rmax RHS in FP64; the z-chunk buffer is sized to ~48 MB so that it stays in L2
 	const size_t R = c->Rmax;
@@ -413,7 +414,7 @@ int adda_gb300_destroy(adda_gb300_ctx *c)
 	solver_free(c);
 	void *bufs[] = {c->d_line_start, c->d_xy, c->d_mat, c->d_pos, c->D64, c->D32, c->cc64, c->ccs64, c->ccs32,
 		c->Xf, c->Tz, c->TzR, c->Tz2, c->TzR2, c->R64, c->R32, c->partial, c->d_red, c->vin, c->vout, c->pvec64,
-		c->tables, c->Dfx, c->fx_exps, c->fld};
+		c->tables, c->Dfx, c->Rfx, c->fx_exps, c->fld};
 	if (c->stream2) cudaStreamSynchronize(c->stream2);
 	for (void *b : bufs)
 		if (b) cudaFree(b);

@@ -134,11 +134,12 @@ struct adda_gb300_ctx {
 	adda::Plan2 p2[3] = {}, p2x[3] = {}; // FP32, fixed point
 	float2 *tw2f[4] = {nullptr, nullptr, nullptr, nullptr};
 	int4 *tw2x[4] = {nullptr, nullptr, nullptr, nullptr};
-	// FP64 matvec in 64-bit fixed point: all three axes have two-pass plans and there is no substrate
+	// FP64 matvec in 64-bit fixed point: all three axes have two-pass plans
 	bool fx = false;
 	void *Dfx = nullptr;    // D in fixed point, [gX][DsZ][DsY][6]
+	void *Rfx = nullptr;    // R in fixed point, [gX][gZ][gY/2+1][6]
 	int *fx_exps = nullptr; // exponents of the data between the kernels (matvec_lines2.cuh: FxExp)
-	int *fx_eD = nullptr;   // exponents of Dfx's rows [gX][DsZ] (behind them)
+	int *fx_eD = nullptr;   // exponents of Dfx's rows [gX][DsZ], then of Rfx's [gX][gZ] (behind them)
 	void *tables = nullptr; // the allocation behind the twiddle tables
 	// interaction matrix, reduced layout [gX][DsZ][DsY][6]
 	double2 *D64 = nullptr;
@@ -194,7 +195,7 @@ int dmatrix_build(adda_gb300_ctx *c);
 
 // matvec_lines2.cu
 size_t fx_exps_ints(const adda_gb300_ctx *c); // ints of fx_exps
-int fx_dmatrix(adda_gb300_ctx *c);            // D64 -> Dfx, fx_eD
+int fx_dmatrix(adda_gb300_ctx *c);            // D64, R64 -> Dfx, Rfx, fx_eD
 
 // matvec.cu
 int matvec_setup(adda_gb300_ctx *c); // tile shapes, kernel attributes

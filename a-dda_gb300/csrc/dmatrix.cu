@@ -659,8 +659,8 @@ int dmatrix_build(adda_gb300_ctx *c)
 	cudaFree(S);
 	cudaFree(d_tabs);
 	cudaFree(d_index);
-	if (!rc && c->fx) rc = fx_dmatrix(c);
 	if (!rc && c->surface) rc = rmatrix_build(c);
+	if (!rc && c->fx) rc = fx_dmatrix(c);
 	if (!rc) c->dready = true;
 	return rc;
 }

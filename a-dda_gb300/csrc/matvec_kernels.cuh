@@ -767,6 +767,7 @@ template <typename T, int NS, int W> constexpr bool has_w2()
 }
 template <typename T, int NS, int P> constexpr bool has_pairs()
 {
+	if (sizeof(T) == 4 && NS != 0) return false; // the register K2b has these lengths
 	return P == Tiles<T>::PAIRS || (sizeof(T) == 4 && (P == 2 || P == 4)) || (NS == 0 && P == 1);
 }
 inline bool shape_instantiated(bool f32, int n1, int n2, int ny, const MvShape &s)
@@ -855,8 +856,7 @@ template <typename T> int setup_yz()
 }
 
 // the stages on two-pass transforms (matvec_lines2.cuh, compiled in matvec_lines2*.cu; measured there against the
-// kernels above, which stay for what they do not cover: axes without a two-pass plan, substrates in FP64, the narrow
-// widths of long axes).
+// kernels above, which stay for what they do not cover: axes without a two-pass plan, the narrow widths of long axes).
 // FP64: all stages in fixed point when the context has the plans and the default tile widths, in place of which the
 // fixed-point kernels have their own: FX_W1 y-lines per K1/K3 block, FX_W2 per K2a/K2c block.
 constexpr int FX_W1 = 2, FX_W2 = 8;
@@ -868,7 +868,7 @@ inline bool use_fx(const adda_gb300_ctx *c)
 inline bool use_l2_f32(const adda_gb300_ctx *c, int axis, int n) { return static_len(n) == 0 && c->p2[axis].r1 > 0; }
 inline bool use_l2_x(const adda_gb300_ctx *c, const MvShape &s) { return use_l2_f32(c, 0, c->gX) && s.w1 >= 4; }
 inline bool use_l2_z(const adda_gb300_ctx *c, const MvShape &s) { return use_l2_f32(c, 2, c->gZ) && s.w2 >= 8; }
-inline bool use_l2_y(const adda_gb300_ctx *c) { return use_l2_f32(c, 1, c->gY) && !c->surface; }
+inline bool use_l2_y(const adda_gb300_ctx *c) { return use_l2_f32(c, 1, c->gY); }
 // y-lines per K1/K3 block of an x axis with a radix above 16 (one width, whatever the shape says)
 constexpr int L2_BIG_W1 = 4;
 int l2_fftz_run(adda_gb300_ctx *c, const MvGeom<float> &p, int mode, int w2, int ck, cudaStream_t st);

@@ -68,6 +68,8 @@ int l2_ffty_run(adda_gb300_ctx *c, const MvGeom<float> &p, int ck, int pairs, cu
 int fx_yz_run(adda_gb300_ctx *c, const MvGeom<double> &p, int ck, cudaStream_t st)
 {
 	int rc = c->p2x[2].big ? fx_fftz_big(c, p, 0, ck, st) : l2_z<ArFx, FX_W2, 0, FX_W1, RC_SMALL>(c, p, ck, st);
+	if (!rc && c->surface)
+		rc = c->p2x[2].big ? fx_fftz_big(c, p, 2, ck, st) : l2_z<ArFx, FX_W2, 2, FX_W1, RC_SMALL>(c, p, ck, st);
 	if (!rc) rc = c->p2x[1].big ? fx_ffty_big(c, p, ck, st) : l2_y<ArFx, FX_W2, RC_SMALL>(c, p, ck, 0, st);
 	if (!rc) rc = c->p2x[2].big ? fx_fftz_big(c, p, 1, ck, st) : l2_z<ArFx, FX_W2, 1, FX_W1, RC_SMALL>(c, p, ck, st);
 	return rc;
@@ -79,6 +81,11 @@ int fx_dmatrix(adda_gb300_ctx *c)
 {
 	mv::fx_drow<<<c->gX * c->DsZ, 128, 0, c->stream>>>(c->D64, (int4 *)c->Dfx, c->fx_eD, c->DsY * 6);
 	ADDA_LAUNCHED();
+	if (c->surface) {
+		mv::fx_drow<<<c->gX * c->gZ, 128, 0, c->stream>>>(c->R64, (int4 *)c->Rfx, c->fx_eD + (size_t)c->gX * c->DsZ,
+			(c->gY / 2 + 1) * 6);
+		ADDA_LAUNCHED();
+	}
 	ADDA_CUDA(cudaStreamSynchronize(c->stream));
 	return ADDA_GB300_OK;
 }

@@ -26,14 +26,17 @@ namespace mv {
 struct FxExp {
 	int *ex;    // after K1: [R][bZ][ny1] e of a K1 block (W1 y-lines, all kx and components)
 	int *ez;    // after K2a: [R][gX][3][ny2] e of a K2a block (W2 y-lines, all kz)
+	int *ezr;   // the same of the reflected transform (particle near a substrate)
 	int *ey;    // after K2b: [R][gX][gZ] e of a column (all y and components)
 	int *ex2;   // after K2c: [R][gX][3][ny2] e of a K2c block
 	int *topx;  // [R][ny2] top of all K1 blocks of W2 y-lines; K3 puts it back to FX_LOW for the next matvec
-	int *topz;  // [R][gX] top of all K2a blocks of a kx
+	int *topz;  // [R][gX] top of all K2a blocks of a kx (of both transforms)
 	int *topy;  // [R][gX] top of all columns of a kx
 	int *topx2; // [R] top of all K2c blocks
 	const fx2 *D;  // interaction matrix, components scaled to 2^60 per row, as split halves (see fx_split)
 	const int *eD; // [gX][DsZ] exponents of its rows
+	const fx2 *Rm; // reflected interaction, likewise
+	const int *eR; // [gX][gZ]
 	int ny1, ny2;
 };
 
@@ -176,7 +179,7 @@ __global__ void __launch_bounds__(32 * ((3 * W * radix_max(RC) + 31) / 32), A::F
 	}
 }
 
-// K2a (MODE 0), K2c (MODE 1) and K2a of the reflected transform (MODE 2, FP32: the inverse sign into TzR): the z
+// K2a (MODE 0), K2c (MODE 1) and K2a of the reflected transform (MODE 2: the inverse sign into TzR): the z
 // transform of W y-lines of one (RHS, kx, component)
 template <class A, int W, int MODE, int W1, int RC>
 __global__ void __launch_bounds__(W * radix_max(RC), A::FX && RC == RC_SMALL ? 512 / (W * RADIX_MAX) : 1) l2_fftz(MvGeom<typename A::T> p, Lines2<A> q)
@@ -184,7 +187,6 @@ __global__ void __launch_bounds__(W * radix_max(RC), A::FX && RC == RC_SMALL ? 5
 	chain_entry<!A::FX>();
 	typedef typename A::C C;
 	constexpr bool INV = MODE == 1, SGN = MODE != 0;
-	static_assert(MODE != 2 || !A::FX, "no fixed-point surface mode");
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	if (rhs_done(p, blockIdx.z)) return; // blockIdx.z = RHS
 	__shared__ unsigned sor;
@@ -253,7 +255,7 @@ __global__ void __launch_bounds__(W * radix_max(RC), A::FX && RC == RC_SMALL ? 5
 		if (threadIdx.x == 0) {
 			const int e = et + q.shz;
 			const int t = top >= FX_BAD / 2 ? FX_BAD : e + fx_bits(acc);
-			(INV ? q.f.ex2 : q.f.ez)[(((size_t)r * p.gX + kx) * 3 + comp) * q.f.ny2 + blockIdx.x] = e;
+			(INV ? q.f.ex2 : MODE == 2 ? q.f.ezr : q.f.ez)[(((size_t)r * p.gX + kx) * 3 + comp) * q.f.ny2 + blockIdx.x] = e;
 			atomicMax(INV ? q.f.topx2 + r : q.f.topz + (size_t)r * p.gX + kx, t);
 		}
 	}
@@ -308,7 +310,9 @@ __device__ __forceinline__ fx2 fx_dot3(int4 a, int4 b, int4 c, const FxV &u, con
 // shared slot. Pass 1 leaves Y[q][j] in row q; from there thread q works in its own row (second pass, first inverse
 // pass), and the second inverse pass reads columns. The D product takes the three components of row q's elements
 // c, c+3, ... (c the thread's component). Rows are r2|1 long: every phase is free of bank conflicts.
-template <class A, int W2, int RC>
+// SURF (particle near a substrate): three more slots hold the lines of TzR; the product adds R~ times their spectra
+// (M21 = M12, M31 = -M13, M32 = -M23, cReflMatrVec cmplx.h:391-401; R reduced in y only).
+template <class A, int W2, int RC, bool SURF>
 __global__ void __launch_bounds__(A::FX ? 128 : 384, RC == RC_BIG ? (A::FX ? 2 : 1) : (A::FX ? 4 : 2))
 	l2_fft_y(MvGeom<typename A::T> p, Lines2<A> q, int G, int P)
 {
@@ -323,30 +327,37 @@ __global__ void __launch_bounds__(A::FX ? 128 : 384, RC == RC_BIG ? (A::FX ? 2 :
 	const int r = unit % p.R, kz = unit / p.R;
 	const bool live = g < G && kz < p.gZ && !rhs_done(p, r);
 	const int kxl = blockIdx.y, kx = p.kx0 + kxl, bY = p.bY, gY = p.gY;
-	C *buf = reinterpret_cast<C *>(smem_raw) + (size_t)g * 3 * slot; // the column's slots
+	constexpr int NS = SURF ? 2 : 1; // sets of three slots
+	C *buf = reinterpret_cast<C *>(smem_raw) + (size_t)g * 3 * NS * slot; // the column's slots
 	C *line = buf + c * slot;                                        // the thread's own line
-	C *col = reinterpret_cast<C *>(p.Tz) + ((((size_t)r * p.CK + kxl) * 3 + c) * p.gZ + kz) * (size_t)bY;
+	const size_t at = ((((size_t)r * p.CK + kxl) * 3 + c) * p.gZ + kz) * (size_t)bY;
+	C *col = reinterpret_cast<C *>(p.Tz) + at;
 	int et = 0, top = 0;
-	const int *ez = nullptr;
+	size_t eat = 0;
 	if constexpr (A::FX) {
 		if (threadIdx.x < 24) sor[threadIdx.x / 8][threadIdx.x % 8] = 0;
 		if (live) {
 			top = q.f.topz[(size_t)r * p.gX + kx];
-			ez = q.f.ez + (((size_t)r * p.gX + kx) * 3 + c) * q.f.ny2;
+			eat = (((size_t)r * p.gX + kx) * 3 + c) * q.f.ny2;
 		}
 		et = top - FX_TOP;
 	}
 	if (live && j < r2) {
-		auto ld = [&](int, int y) {
-			if (y >= bY) return cx<C>(0, 0);
-			C v = ld_cg(col + y);
-			if constexpr (A::FX) {
-				const int d = ez[y / W2] - et;
-				v = fx2{fx_shift_by(v.x, d), fx_shift_by(v.y, d)};
-			}
-			return v;
-		};
-		ADDA_RADIX_SWITCH(r1, (pass_first<A, RR, false, true>(ld, line, pitch, j, j, r2, q.ty, q.shy)))
+#pragma unroll 1
+		for (int h = 0; h < NS; h++) {
+			const C *src = h ? reinterpret_cast<const C *>(p.TzR) + at : col;
+			const int *ez = (h ? q.f.ezr : q.f.ez) + eat;
+			auto ld = [&](int, int y) {
+				if (y >= bY) return cx<C>(0, 0);
+				C v = ld_cg(src + y);
+				if constexpr (A::FX) {
+					const int d = ez[y / W2] - et;
+					v = fx2{fx_shift_by(v.x, d), fx_shift_by(v.y, d)};
+				}
+				return v;
+			};
+			ADDA_RADIX_SWITCH(r1, (pass_first<A, RR, false, true>(ld, line + 3 * h * slot, pitch, j, j, r2, q.ty, q.shy)))
+		}
 	}
 	__syncthreads();
 	const bool rz = kz >= p.DsZ;
@@ -355,26 +366,37 @@ __global__ void __launch_bounds__(A::FX ? 128 : 384, RC == RC_BIG ? (A::FX ? 2 :
 	unsigned acc = 0;
 	C *own = line + j * pitch;
 	if (act) {
-		auto ld = [&](int t) { return own[t]; };
-		auto st = [&](int t, int, C v) {
-			own[t] = v;
-			if constexpr (A::FX) {
-				fx_or(acc, v.x);
-				fx_or(acc, v.y);
-			}
-		};
-		ADDA_RADIX_SWITCH(r2, (pass_second<A, RR, false, false>(ld, st, j, r1)))
+#pragma unroll 1
+		for (int h = 0; h < NS; h++) {
+			C *o = own + 3 * h * slot;
+			auto ld = [&](int t) { return o[t]; };
+			auto st = [&](int t, int, C v) {
+				o[t] = v;
+				if constexpr (A::FX) {
+					fx_or(acc, v.x);
+					fx_or(acc, v.y);
+				}
+			};
+			ADDA_RADIX_SWITCH(r2, (pass_second<A, RR, false, false>(ld, st, j, r1)))
+		}
 	}
 	if constexpr (A::FX)
 		if (act) atomicOr(&sor[0][g], acc);
 	__syncthreads();
 	constexpr int k = 3;
-	int eo = 0, ed = 0, shv = 0;
+	int eo = 0, ed = 0, shv = 0, dD = 0, dR = 0;
 	if constexpr (A::FX) {
 		// the components of v are brought just below 2^60: the products leave out the lowest partial product, 2^-60 of
 		// the largest v and D; |sum of three| < 3 * 2^60.5 * 2^60.5, so 3 more bits than the upper 64 fit
 		shv = fx_bits(sor[0][g & 7]) - 60;
 		if (live) ed = q.f.eD[(size_t)kx * p.DsZ + zz];
+		if constexpr (SURF)
+			if (live) { // the row's two products at the larger of the two exponents
+				const int er = q.f.eR[(size_t)kx * p.gZ + kz];
+				dD = max(0, er - ed);
+				dR = max(0, ed - er);
+				ed = max(ed, er);
+			}
 		eo = et + q.shy + shv + ed + 64 - k;
 		acc = 0;
 	}
@@ -398,8 +420,30 @@ __global__ void __launch_bounds__(A::FX ? 128 : 384, RC == RC_BIG ? (A::FX ? 2 :
 				w1 = fx2{fx_shift_by(w1.x, -shv), fx_shift_by(w1.y, -shv)};
 				w2 = fx2{fx_shift_by(w2.x, -shv), fx_shift_by(w2.y, -shv)};
 				const FxV v0 = fx_vsplit(w0), v1 = fx_vsplit(w1), v2 = fx_vsplit(w2);
-				const fx2 o0 = fx_dot3(m0, m1, m2, v0, v1, v2, k), o1 = fx_dot3(m1, m3, m4, v0, v1, v2, k),
+				fx2 o0 = fx_dot3(m0, m1, m2, v0, v1, v2, k), o1 = fx_dot3(m1, m3, m4, v0, v1, v2, k),
 					o2 = fx_dot3(m2, m4, m5, v0, v1, v2, k);
+				if constexpr (SURF) {
+					const bool qy = ky > gY / 2;
+					const int4 *fr = reinterpret_cast<const int4 *>(q.f.Rm) + (((size_t)kx * p.gZ + kz) * p.RsY + (qy ? gY - ky : ky)) * 6;
+					m0 = __ldg(fr), m1 = __ldg(fr + 1), m2 = __ldg(fr + 2), m3 = __ldg(fr + 3), m4 = __ldg(fr + 4), m5 = __ldg(fr + 5);
+					if (qy) {
+						m1 = fx_neg4(m1);
+						m4 = fx_neg4(m4);
+					}
+					const C *ur = row + 3 * slot;
+					FxV u[3];
+#pragma unroll
+					for (int i = 0; i < 3; i++) {
+						const fx2 w = ur[i * slot + t];
+						u[i] = fx_vsplit(fx2{fx_shift_by(w.x, -shv), fx_shift_by(w.y, -shv)});
+					}
+					const auto add = [&](fx2 a, fx2 b) {
+						return fx2{fx_shift_by(a.x, -dD) + fx_shift_by(b.x, -dR), fx_shift_by(a.y, -dD) + fx_shift_by(b.y, -dR)};
+					};
+					o0 = add(o0, fx_dot3(m0, m1, m2, u[0], u[1], u[2], k));
+					o1 = add(o1, fx_dot3(m1, m3, m4, u[0], u[1], u[2], k));
+					o2 = add(o2, fx_dot3(fx_neg4(m2), fx_neg4(m4), m5, u[0], u[1], u[2], k));
+				}
 				fx_or(acc, o0.x);
 				fx_or(acc, o0.y);
 				fx_or(acc, o1.x);
@@ -419,9 +463,27 @@ __global__ void __launch_bounds__(A::FX ? 128 : 384, RC == RC_BIG ? (A::FX ? 2 :
 				if (ry != rz) m4 = cneg(m4);
 				if (rz) m2 = cneg(m2);
 				const C v0 = row[t], v1 = row[slot + t], v2 = row[2 * slot + t];
-				row[t] = cfma(m0, v0, cfma(m1, v1, cmul(m2, v2)));
-				row[slot + t] = cfma(m1, v0, cfma(m3, v1, cmul(m4, v2)));
-				row[2 * slot + t] = cfma(m2, v0, cfma(m4, v1, cmul(m5, v2)));
+				C o0 = cfma(m0, v0, cfma(m1, v1, cmul(m2, v2))), o1 = cfma(m1, v0, cfma(m3, v1, cmul(m4, v2))),
+				  o2 = cfma(m2, v0, cfma(m4, v1, cmul(m5, v2)));
+				if constexpr (SURF) {
+					const bool qy = ky > gY / 2;
+					const float4 *fr = reinterpret_cast<const float4 *>(p.Rm) + (((size_t)kx * p.gZ + kz) * p.RsY + (qy ? gY - ky : ky)) * 3;
+					const float4 e0 = __ldg(fr), e1 = __ldg(fr + 1), e2 = __ldg(fr + 2);
+					m0 = make_float2(e0.x, e0.y), m1 = make_float2(e0.z, e0.w), m2 = make_float2(e1.x, e1.y);
+					m3 = make_float2(e1.z, e1.w), m4 = make_float2(e2.x, e2.y), m5 = make_float2(e2.z, e2.w);
+					if (qy) {
+						m1 = cneg(m1);
+						m4 = cneg(m4);
+					}
+					const C *ur = row + 3 * slot;
+					const C u0 = ur[t], u1 = ur[slot + t], u2 = ur[2 * slot + t];
+					o0 = cfma(m0, u0, cfma(m1, u1, cfma(m2, u2, o0)));
+					o1 = cfma(m1, u0, cfma(m3, u1, cfma(m4, u2, o1)));
+					o2 = cfma(cneg(m2), u0, cfma(cneg(m4), u1, cfma(m5, u2, o2)));
+				}
+				row[t] = o0;
+				row[slot + t] = o1;
+				row[2 * slot + t] = o2;
 			}
 		}
 	}
@@ -543,9 +605,9 @@ template <class A> inline size_t l2_z_smem(const Plan2 &p, int w)
 {
 	return sizeof(typename A::C) * (size_t)p.r1 * xch_ks(w, p.r2);
 }
-template <class A> inline size_t l2_y_smem(const Plan2 &p, int g)
+template <class A> inline size_t l2_y_smem(const Plan2 &p, int g, bool surf)
 {
-	return sizeof(typename A::C) * (size_t)g * 3 * p.r1 * (p.r2 | 1);
+	return sizeof(typename A::C) * (size_t)g * (surf ? 6 : 3) * p.r1 * (p.r2 | 1);
 }
 // the exponent tables inside fx_exps
 inline FxExp fx_tables(const adda_gb300_ctx *c, size_t *ints = nullptr)
@@ -559,6 +621,8 @@ inline FxExp fx_tables(const adda_gb300_ctx *c, size_t *ints = nullptr)
 	at += R * c->bZ * f.ny1;
 	f.ez = at;
 	at += R * gX * 3 * f.ny2;
+	f.ezr = at;
+	if (c->surface) at += R * gX * 3 * f.ny2;
 	f.ey = at;
 	at += R * gX * c->gZ;
 	f.ex2 = at;
@@ -574,6 +638,8 @@ inline FxExp fx_tables(const adda_gb300_ctx *c, size_t *ints = nullptr)
 	if (ints) *ints = (size_t)(at - c->fx_exps);
 	f.D = (const fx2 *)c->Dfx;
 	f.eD = c->fx_eD;
+	f.Rm = (const fx2 *)c->Rfx;
+	f.eR = c->fx_eD + (size_t)c->gX * c->DsZ;
 	return f;
 }
 template <class A> inline Lines2<A> make_lines2(const adda_gb300_ctx *c)
@@ -636,9 +702,12 @@ template <class A, int W2, int RC>
 inline int l2_y(adda_gb300_ctx *c, const MvGeom<typename A::T> &p, int ck, int pairs, cudaStream_t st)
 {
 	const Lines2<A> q = make_lines2<A>(c);
-	const int P = std::max(q.py.r1, q.py.r2), G = l2_columns<A>(q.py, pairs);
+	// a column near a substrate has twice the lines: half the columns
+	const int P = std::max(q.py.r1, q.py.r2), G = l2_columns<A>(q.py, c->surface ? std::max(1, pairs / 2) : pairs);
 	const dim3 g((c->gZ * p.R + G - 1) / G, ck);
-	return l2_launch<l2_fft_y<A, W2, RC>>(c, g, (3 * G * P + 31) / 32 * 32, l2_y_smem<A>(q.py, G), st, p, q, G, P);
+	const int nt = (3 * G * P + 31) / 32 * 32;
+	if (c->surface) return l2_launch<l2_fft_y<A, W2, RC, true>>(c, g, nt, l2_y_smem<A>(q.py, G, true), st, p, q, G, P);
+	return l2_launch<l2_fft_y<A, W2, RC, false>>(c, g, nt, l2_y_smem<A>(q.py, G, false), st, p, q, G, P);
 }
 template <class A, typename V, int W, int W2, int RC>
 inline int l2_k1(adda_gb300_ctx *c, const MvP<typename A::T, V> &p, cudaStream_t st)

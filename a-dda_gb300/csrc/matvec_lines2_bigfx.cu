@@ -7,6 +7,7 @@ namespace mv {
 
 int fx_fftz_big(adda_gb300_ctx *c, const MvGeom<double> &p, int mode, int ck, cudaStream_t st)
 {
+	if (mode == 2) return l2_z<ArFx, FX_W2, 2, FX_W1, RC_BIG>(c, p, ck, st);
 	return mode ? l2_z<ArFx, FX_W2, 1, FX_W1, RC_BIG>(c, p, ck, st) : l2_z<ArFx, FX_W2, 0, FX_W1, RC_BIG>(c, p, ck, st);
 }
 int fx_ffty_big(adda_gb300_ctx *c, const MvGeom<double> &p, int ck, cudaStream_t st)

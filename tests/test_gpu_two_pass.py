@@ -121,3 +121,25 @@ def test_scalar_steps_in_the_last_block(method, grid):
         assert rel(res["p"][r] / scale[r], want) < 1e-9
     o.close()
     c.close()
+
+
+@pytest.mark.parametrize("box", [(6, 5, 4), (11, 9, 13), (32, 32, 32), (25, 10, 45), (7, 100, 6), (6, 5, 110)])
+def test_particle_near_a_substrate(box):
+    """the reflected transform and product: small and large radices, odd boxes, a power-of-two grid"""
+    import adda_gb300 as A
+    s = cube_setup(box, tuple(A.fft_fit(2 * v, 2) for v in box))
+    s.surface = dict(zsum_shift=1.25, msub=1.5 + 0.1j, relation="img")
+    o = oracle_for(s)
+    c = A.Context(s.box, s.pos, s.mat, s.gridspace, s.wavenum, s.grid, nrhs_max=2, surface=s.surface)
+    c.init_dmatrix()
+    x = random_vec(s.n, 2, sum(box))
+    for r in range(2):
+        c.set_cc(r, s.cc[r].reshape(1, 3))
+    for her in (False, True):
+        y, yf = c.matvec(x, "fp64", her)[0], c.matvec(x, "fp32", her)[0]
+        for r in range(2):
+            o.set_cc(s.cc[r].reshape(1, 3))
+            yr = o.matvec(x[r], her)[0]
+            assert rel(y[r], yr) < TOL64 and rel(yf[r], yr) < TOL32
+    o.close()
+    c.close()
