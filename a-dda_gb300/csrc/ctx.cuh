@@ -38,20 +38,18 @@ inline void count_launch(unsigned long long k = 1) { g_launches.fetch_add(k, std
 // run, and wait in chain_entry() until it has completed. Every kernel launched with launch_next() calls chain_entry()
 // before anything else, on every path: a kernel that returned without waiting would let its successor start before its
 // predecessor has completed. Measured: one FP32 matvec (five kernels) at 32^3 30.1 -> 20.6 us, at 96^3 89 -> 80, at 256^3
-// 676 -> 658. Inside a graph the kernels follow one another quickly by themselves, and the same launches made the adjoint
-// solve of a 32^3 cube slower (23.8 -> 26.5 ms): captured launches stay plain.
-// EARLY: the successor's blocks are set up from now on; otherwise when this kernel's blocks end (the fixed-point kernels of
-// large grids lose 2 % to waiting blocks that hold shared memory).
-template <bool EARLY = true> __device__ __forceinline__ void chain_entry()
+// 676 -> 658.
+// early: the successor's blocks are set up from now on; otherwise when this kernel's blocks end, which is better inside
+// graphs (adjoint solve of a 32^3 cube: 22.6 ms against 25.7 early and 23.2 with plain launches) and for the fixed-point
+// kernels (early, 256^3 takes 2 % longer: the waiting blocks hold shared memory).
+__device__ __forceinline__ void chain_entry(bool early = false)
 {
 	asm volatile("griddepcontrol.wait;" ::: "memory");
-	if constexpr (EARLY) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+	if (early) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 template <typename... K, typename... A>
 inline void launch_next(void (*kern)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const A &...args)
 {
-	cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-	cudaStreamIsCapturing(st, &cap);
 	cudaLaunchAttribute at;
 	at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
 	at.val.programmaticStreamSerializationAllowed = 1;
@@ -61,7 +59,7 @@ inline void launch_next(void (*kern)(K...), dim3 grid, dim3 block, size_t smem, 
 	cfg.dynamicSmemBytes = smem;
 	cfg.stream = st;
 	cfg.attrs = &at;
-	cfg.numAttrs = cap == cudaStreamCaptureStatusNone ? 1 : 0;
+	cfg.numAttrs = 1;
 	cudaLaunchKernelEx(&cfg, kern, K(args)...); // errors are read by ADDA_LAUNCHED
 }
 

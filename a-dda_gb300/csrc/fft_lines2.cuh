@@ -100,10 +100,14 @@ __device__ __forceinline__ fx2 fx_cmul(fx2 v, int4 w, bool conj)
 }
 // v / 2^s rounded
 __device__ __forceinline__ long long fx_rshift(long long v, int s) { return (v + (1ll << (s - 1))) >> s; }
-// v * 2^d rounded, d of either sign (the caller's range makes a left shift safe)
-__device__ __forceinline__ long long fx_shift_by(long long v, int d)
+// v * 2^d rounded, d of either sign (the caller's range makes a left shift safe); d is mostly the same for a whole warp,
+// so the two directions are separate paths
+__device__ __forceinline__ fx2 fx_shift(fx2 v, int d)
 {
-	return d >= 0 ? v << d : fx_rshift(v, min(-d, 63));
+	if (d >= 0) return fx2{v.x << d, v.y << d};
+	const int s = min(-d, 62);
+	const long long half = 1ll << (s - 1);
+	return fx2{(v.x + half) >> s, (v.y + half) >> s};
 }
 // bits that v and the values OR-ed into the same accumulator need: their common magnitude is below
 // 2^(64 - clz(acc)) (the accumulator holds high words of |v| or |v|-1)

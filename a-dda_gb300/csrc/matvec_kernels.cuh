@@ -67,6 +67,7 @@ template <typename T> struct MvGeom {
 	int RsY;
 	int rpp;           // RHS per particle: RHS r uses lattice slot r / rpp (a group context, adda_gb300_create_group)
 	size_t lat_stride; // dipoles per lattice slot
+	bool early;        // chain_entry
 };
 
 template <typename T, typename V> struct MvP : MvGeom<T> {
@@ -111,7 +112,7 @@ template <typename T, typename V, int W, int NS>
 __global__ void __launch_bounds__(col_threads<T, NS, 3 * W>(), (col_minblocks<T, NS, 3 * W>()))
 	mv_scatter_fftx(MvP<T, V> p)
 {
-	chain_entry();
+	chain_entry(p.early);
 	typedef typename CxT<T>::type C;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	if (rhs_done(p, blockIdx.z)) return; // blockIdx.z = RHS
@@ -189,7 +190,7 @@ __global__ void __launch_bounds__(col_threads<T, NS, 3 * W>(), (col_minblocks<T,
 template <typename T, int W, int MODE, int NS>
 __global__ void __launch_bounds__(col_threads<T, NS, W>(), (col_minblocks<T, NS, W>())) mv_fftz(MvGeom<T> p)
 {
-	chain_entry();
+	chain_entry(p.early);
 	constexpr bool INV = MODE == 1, SGN = MODE != 0;
 	typedef typename CxT<T>::type C;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -278,7 +279,7 @@ __global__ void __launch_bounds__(col_threads<T, NS, W>(), (col_minblocks<T, NS,
 // with its 32 lanes along y (coalesced rows of Tz, odd tile stride: conflict-free).
 template <typename T, int NS, int P> __global__ void __launch_bounds__(256) mv_fft_y_dmul(MvGeom<T> p)
 {
-	chain_entry();
+	chain_entry(p.early);
 	typedef typename CxT<T>::type C;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	if (all_done(p)) return;
@@ -355,7 +356,7 @@ template <typename T, int NS, int P> __global__ void __launch_bounds__(256) mv_f
 // transform into Tz. Line l = pair*6 + c6, c6 < 3 from Tz, c6 >= 3 from TzR.
 template <typename T, int NS, int P> __global__ void __launch_bounds__(256) mv_fft_y_surf(MvGeom<T> p)
 {
-	chain_entry();
+	chain_entry(p.early);
 	typedef typename CxT<T>::type C;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	if (all_done(p)) return;
@@ -450,7 +451,7 @@ template <int NS, int NT, bool SURF = false>
 __global__ void __launch_bounds__(NT, NS >= 512 ? (NT >= 256 ? 1 : 256 / NT) : (SURF ? 3 : 4) * 128 / NT)
 	mv_fft_y_reg(MvGeom<float> p)
 {
-	chain_entry();
+	chain_entry(p.early);
 	typedef float2 C;
 	constexpr int T = RegShape<NS>::T, E = RegShape<NS>::E, BUF = RegShape<NS>::BUF, G = NT / T;
 	constexpr int NSLOT = SURF ? 4 : 3;
@@ -669,7 +670,7 @@ template <typename T, typename V, int W, int NS>
 __global__ void __launch_bounds__(col_threads<T, NS, 3 * W>(), (col_minblocks<T, NS, 3 * W>()))
 	mv_fftx_gather(MvP<T, V> p, MvEpi e)
 {
-	chain_entry();
+	chain_entry(p.early);
 	typedef typename CxT<T>::type C;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	if (rhs_done(p, blockIdx.z)) return; // blockIdx.z = RHS
@@ -1005,6 +1006,9 @@ int launch_matvec(adda_gb300_ctx *c, int R, const V *arg, V *res, int her, const
 	p.rpp = c->rpp;
 	p.lat_stride = c->lat_stride;
 	cudaStream_t st = c->stream;
+	cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+	ADDA_CUDA(cudaStreamIsCapturing(st, &cap));
+	p.early = !dbl && cap == cudaStreamCaptureStatusNone;
 	const dim3 g1((c->bY + sh.w1 - 1) / sh.w1, c->bZ, R);
 	int rc;
 	bool l2 = false; // K1 and K3 on two-pass transforms

@@ -87,7 +87,7 @@ template <class A, typename V, int W, int W2, int RC>
 __global__ void __launch_bounds__(32 * ((3 * W * radix_max(RC) + 31) / 32), A::FX && RC == RC_SMALL ? 512 / (3 * W * RADIX_MAX) : 1)
 	l2_scatter_x(MvP<typename A::T, V> p, Lines2<A> q)
 {
-	chain_entry<!A::FX>();
+	chain_entry(p.early);
 	typedef typename A::C C;
 	typedef TileC<A> TC;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(32 * ((3 * W * radix_max(RC) + 31) / 32), A::F
 template <class A, int W, int MODE, int W1, int RC>
 __global__ void __launch_bounds__(W * radix_max(RC), A::FX && RC == RC_SMALL ? 512 / (W * RADIX_MAX) : 1) l2_fftz(MvGeom<typename A::T> p, Lines2<A> q)
 {
-	chain_entry<!A::FX>();
+	chain_entry(p.early);
 	typedef typename A::C C;
 	constexpr bool INV = MODE == 1, SGN = MODE != 0;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(W * radix_max(RC), A::FX && RC == RC_SMALL ? 5
 				C v = ld_cg(tz + (size_t)z * p.bY + l);
 				if constexpr (A::FX) {
 					const int d = ey[z] - et;
-					v = fx2{fx_shift_by(v.x, d), fx_shift_by(v.y, d)};
+					v = fx_shift(v, d);
 				}
 				return v;
 			}
@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(W * radix_max(RC), A::FX && RC == RC_SMALL ? 5
 				C v = ld_cs(xf + (size_t)z * p.bY + l);
 				if constexpr (A::FX) {
 					const int d = ex[(size_t)z * q.f.ny1] - et;
-					v = fx2{fx_shift_by(v.x, d), fx_shift_by(v.y, d)};
+					v = fx_shift(v, d);
 				}
 				return v;
 			}
@@ -316,7 +316,7 @@ template <class A, int W2, int RC, bool SURF>
 __global__ void __launch_bounds__(A::FX ? 128 : 384, RC == RC_BIG ? (A::FX ? 2 : 1) : (A::FX ? 4 : 2))
 	l2_fft_y(MvGeom<typename A::T> p, Lines2<A> q, int G, int P)
 {
-	chain_entry<!A::FX>();
+	chain_entry(p.early);
 	typedef typename A::C C;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	__shared__ unsigned sor[3][8];
@@ -352,7 +352,7 @@ __global__ void __launch_bounds__(A::FX ? 128 : 384, RC == RC_BIG ? (A::FX ? 2 :
 				C v = ld_cg(src + y);
 				if constexpr (A::FX) {
 					const int d = ez[y / W2] - et;
-					v = fx2{fx_shift_by(v.x, d), fx_shift_by(v.y, d)};
+					v = fx_shift(v, d);
 				}
 				return v;
 			};
@@ -416,9 +416,16 @@ __global__ void __launch_bounds__(A::FX ? 128 : 384, RC == RC_BIG ? (A::FX ? 2 :
 				if (ry != rz) m4 = fx_neg4(m4);
 				if (rz) m2 = fx_neg4(m2);
 				fx2 w0 = row[t], w1 = row[slot + t], w2 = row[2 * slot + t];
-				w0 = fx2{fx_shift_by(w0.x, -shv), fx_shift_by(w0.y, -shv)};
-				w1 = fx2{fx_shift_by(w1.x, -shv), fx_shift_by(w1.y, -shv)};
-				w2 = fx2{fx_shift_by(w2.x, -shv), fx_shift_by(w2.y, -shv)};
+				if (shv <= 0) {
+					w0 = fx2{w0.x << -shv, w0.y << -shv};
+					w1 = fx2{w1.x << -shv, w1.y << -shv};
+					w2 = fx2{w2.x << -shv, w2.y << -shv};
+				}
+				else {
+					w0 = fx_shift(w0, -shv);
+					w1 = fx_shift(w1, -shv);
+					w2 = fx_shift(w2, -shv);
+				}
 				const FxV v0 = fx_vsplit(w0), v1 = fx_vsplit(w1), v2 = fx_vsplit(w2);
 				fx2 o0 = fx_dot3(m0, m1, m2, v0, v1, v2, k), o1 = fx_dot3(m1, m3, m4, v0, v1, v2, k),
 					o2 = fx_dot3(m2, m4, m5, v0, v1, v2, k);
@@ -435,10 +442,10 @@ __global__ void __launch_bounds__(A::FX ? 128 : 384, RC == RC_BIG ? (A::FX ? 2 :
 #pragma unroll
 					for (int i = 0; i < 3; i++) {
 						const fx2 w = ur[i * slot + t];
-						u[i] = fx_vsplit(fx2{fx_shift_by(w.x, -shv), fx_shift_by(w.y, -shv)});
+						u[i] = fx_vsplit(fx_shift(w, -shv));
 					}
 					const auto add = [&](fx2 a, fx2 b) {
-						return fx2{fx_shift_by(a.x, -dD) + fx_shift_by(b.x, -dR), fx_shift_by(a.y, -dD) + fx_shift_by(b.y, -dR)};
+						return cadd(fx_shift(a, -dD), fx_shift(b, -dR));
 					};
 					o0 = add(o0, fx_dot3(m0, m1, m2, u[0], u[1], u[2], k));
 					o1 = add(o1, fx_dot3(m1, m3, m4, u[0], u[1], u[2], k));
@@ -536,7 +543,7 @@ template <class A, typename V, int W, int W2, int RC>
 __global__ void __launch_bounds__(32 * ((3 * W * radix_max(RC) + 31) / 32), A::FX && RC == RC_SMALL ? 512 / (3 * W * RADIX_MAX) : 1)
 	l2_gather_x(MvP<typename A::T, V> p, Lines2<A> q, MvEpi e)
 {
-	chain_entry<!A::FX>();
+	chain_entry(p.early);
 	typedef typename A::C C;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	if (rhs_done(p, blockIdx.z)) return; // blockIdx.z = RHS
@@ -565,7 +572,7 @@ __global__ void __launch_bounds__(32 * ((3 * W * radix_max(RC) + 31) / 32), A::F
 			C v = ld_cs(src + (size_t)kx * 3 * plane);
 			if constexpr (A::FX) {
 				const int d = ex[(size_t)kx * 3 * q.f.ny2] - et;
-				v = fx2{fx_shift_by(v.x, d), fx_shift_by(v.y, d)};
+				v = fx_shift(v, d);
 			}
 			return v;
 		};
