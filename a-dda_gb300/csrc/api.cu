@@ -344,7 +344,7 @@ static int create_impl(const adda_gb300_problem *p, adda_gb300_ctx *c, const std
 	// interaction matrix
 	const size_t dlen = (size_t)c->gX * c->DsZ * c->DsY * 6;
 	ADDA_CUDA(cudaMalloc(&c->D64, sizeof(double2) * dlen));
-	ADDA_CUDA(cudaMalloc(&c->D32, sizeof(float2) * dlen));
+	ADDA_CUDA(cudaMalloc(&c->D32, sizeof(float2) * rows_len((size_t)c->gX * c->DsZ, c->gY, c->DsY)));
 	if (c->fx) {
 		ADDA_CUDA(cudaMalloc(&c->Dfx, sizeof(int4) * dlen));
 		// every top below every exponent (each byte 0x80: far below FX_LOW), as each matvec leaves them
@@ -356,7 +356,7 @@ static int create_impl(const adda_gb300_problem *p, adda_gb300_ctx *c, const std
 	if (c->surface) {
 		const size_t rlen = (size_t)c->gX * c->gZ * (c->gY / 2 + 1) * 6;
 		ADDA_CUDA(cudaMalloc(&c->R64, sizeof(double2) * rlen));
-		ADDA_CUDA(cudaMalloc(&c->R32, sizeof(float2) * rlen));
+		ADDA_CUDA(cudaMalloc(&c->R32, sizeof(float2) * rows_len((size_t)c->gX * c->gZ, c->gY, c->gY / 2 + 1)));
 		if (c->fx) ADDA_CUDA(cudaMalloc(&c->Rfx, sizeof(int4) * rlen));
 	}
 	// matvec work: Xf for Rmax RHS in FP64; the z-chunk buffer is sized to ~48 MB so that it stays in L2

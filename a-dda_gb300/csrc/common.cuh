@@ -375,6 +375,17 @@ constexpr bool radix_built(int r, bool fx)
 	return !fx && (r == 21 || r == 22 || r == 26 || r == 27 || r == 28 || r == 30);
 }
 
+// The FP32 interaction matrices D32 and R32 hold a row (one kx, kz; ny entries in y of 6 components) as [ky][6], or, for
+// the y lengths of the register form of K2b (mv_fft_y_reg), as six planes of row_pitch(ny) entries, each from a 32-byte
+// sector on: its lanes hold consecutive ky, so that a load of one component touches 1-2 lines instead of 6-13. One matvec,
+// [ky][6] -> planes: 64^3 on a substrate 209 -> 180 us, a 128^3 sphere 657 -> 647 us, 256^3 7.13 -> 6.97 ms (planes on
+// 128-byte lines: the same). The two-pass K2b (l2_fft_y) keeps [ky][6], where each lane's 48 bytes are its own sectors
+// (planes: 48^3 80 -> 83 us, 96^3 with 8 RHS 822 -> 844 us, 128^3 FP64 4.95 -> 5.05 ms).
+__host__ __device__ constexpr bool planar_rows(int gY) { return gY == 64 || gY == 128 || gY == 256 || gY == 512; }
+__host__ __device__ constexpr int row_pitch(int ny) { return (ny + 3) / 4 * 4; }
+// entries of `rows` rows
+inline size_t rows_len(size_t rows, int gY, int ny) { return rows * 6 * (planar_rows(gY) ? row_pitch(ny) : ny); }
+
 // multiply by exp(s*i*theta) given c=cos(theta), s_=s*sin(theta)
 template <typename C> __device__ __forceinline__ C crot(C v, double c, double s_)
 {

@@ -492,10 +492,20 @@ __global__ void r_extract(double2 *Rm, const double2 *S, int a, int gX, int gY, 
 	}
 }
 
-__global__ void to_f32(float2 *dst, const double2 *src, size_t n)
+// FP32 copy of a matrix [rows][ny][6], in planes per component where K2b reads those (planar_rows)
+__global__ void to_f32(float2 *dst, const double2 *src, size_t rows, int ny, bool planar)
 {
-	for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x)
-		dst[t] = make_float2((float)src[t].x, (float)src[t].y);
+	const int pitch = row_pitch(ny);
+	const size_t n = rows * 6 * ny;
+	for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x) {
+		const double2 v = src[t];
+		size_t at = t;
+		if (planar) {
+			const size_t e = t / 6, row = e / ny;
+			at = (row * 6 + (t - 6 * e)) * pitch + (e - row * ny);
+		}
+		dst[at] = make_float2((float)v.x, (float)v.y);
+	}
 }
 
 int grid_for(size_t n)
@@ -567,7 +577,7 @@ int rmatrix_build(adda_gb300_ctx *c)
 			if (cudaGetLastError() != cudaSuccess) { rc = ADDA_GB300_ECUDA; break; }
 		}
 		if (rc) break;
-		to_f32<<<grid_for(rlen), 256, 0, c->stream>>>(c->R32, c->R64, rlen);
+		to_f32<<<grid_for(rlen), 256, 0, c->stream>>>(c->R32, c->R64, (size_t)gX * gZ, RsY, planar_rows(gY));
 		count_launch();
 		if (cudaGetLastError() != cudaSuccess) { rc = ADDA_GB300_ECUDA; break; }
 		if (cudaStreamSynchronize(c->stream) != cudaSuccess) { rc = ADDA_GB300_ECUDA; break; }
@@ -649,7 +659,7 @@ int dmatrix_build(adda_gb300_ctx *c)
 			if (cudaGetLastError() != cudaSuccess) { rc = ADDA_GB300_ECUDA; break; }
 		}
 		if (rc) break;
-		to_f32<<<grid_for(dlen), 256, 0, c->stream>>>(c->D32, c->D64, dlen);
+		to_f32<<<grid_for(dlen), 256, 0, c->stream>>>(c->D32, c->D64, (size_t)gX * c->DsZ, c->DsY, planar_rows(c->gY));
 		count_launch();
 		if (cudaGetLastError() != cudaSuccess) { rc = ADDA_GB300_ECUDA; break; }
 		if (cudaStreamSynchronize(c->stream) != cudaSuccess) { rc = ADDA_GB300_ECUDA; break; }

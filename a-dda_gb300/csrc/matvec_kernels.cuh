@@ -468,11 +468,12 @@ __global__ void __launch_bounds__(NT, NS >= 512 ? (NT >= 256 ? 1 : 256 / NT) : (
 	const size_t lz = (size_t)p.gZ * p.bY;
 	C *col = p.Tz + (((size_t)r * p.CK + kxl) * 3) * lz + (size_t)kz * p.bY;
 	// the column's D row (and R row) start moving into L2 now, so that the product after the forward transforms
-	// finds them there; one lane of the first RHS's group asks (rows of 6 complex per ky: multiples of 48 bytes)
+	// finds them there; one lane of the first RHS's group asks (rows of six planes: multiples of 192 bytes)
 	if (j1 == 0 && r == 0) {
-		prefetch_l2_bulk(p.D + ((size_t)kx * p.DsZ + (kz >= p.DsZ ? p.gZ - kz : kz)) * DY * 6,
-			(unsigned)(DY * 6 * sizeof(C)));
-		if constexpr (SURF) prefetch_l2_bulk(p.Rm + ((size_t)kx * p.gZ + kz) * DY * 6, (unsigned)(DY * 6 * sizeof(C)));
+		constexpr unsigned RB = 6 * row_pitch(DY) * sizeof(C);
+		prefetch_l2_bulk(reinterpret_cast<const unsigned char *>(p.D) +
+			((size_t)kx * p.DsZ + (kz >= p.DsZ ? p.gZ - kz : kz)) * RB, RB);
+		if constexpr (SURF) prefetch_l2_bulk(reinterpret_cast<const unsigned char *>(p.Rm) + ((size_t)kx * p.gZ + kz) * RB, RB);
 	}
 	// the three component lines go to their slots asynchronously (lane j1 writes and later reads only its own
 	// elements, at j*T + j1), one commit group each, so components 1 and 2 arrive during component 0's transform;
@@ -517,16 +518,15 @@ __global__ void __launch_bounds__(NT, NS >= 512 ? (NT >= 256 ? 1 : 256 / NT) : (
 	}
 	const bool rz = kz >= p.DsZ;
 	const int zz = rz ? p.gZ - kz : kz;
-	const float4 *drow = reinterpret_cast<const float4 *>(p.D + ((size_t)kx * p.DsZ + zz) * DY * 6);
+	const C *drow = p.D + ((size_t)kx * p.DsZ + zz) * (6 * row_pitch(DY));
 #pragma unroll
 	for (int j = 0; j < E; j++) {
 		const int ky = j1 + T * j;
 		const bool ry = ky >= DY;
 		const int yy = ry ? NS - ky : ky;
-		const float4 *f = drow + (size_t)yy * 3;
-		const float4 d0 = __ldg(f), d1 = __ldg(f + 1), d2 = __ldg(f + 2);
-		C m0 = make_float2(d0.x, d0.y), m1 = make_float2(d0.z, d0.w), m2 = make_float2(d1.x, d1.y);
-		C m3 = make_float2(d1.z, d1.w), m4 = make_float2(d2.x, d2.y), m5 = make_float2(d2.z, d2.w);
+		constexpr int RP = row_pitch(DY);
+		const C *f = drow + yy;
+		C m0 = __ldg(f), m1 = __ldg(f + RP), m2 = __ldg(f + 2 * RP), m3 = __ldg(f + 3 * RP), m4 = __ldg(f + 4 * RP), m5 = __ldg(f + 5 * RP);
 		if (ry) m1 = cneg(m1);
 		if (ry != rz) m4 = cneg(m4);
 		if (rz) m2 = cneg(m2);
@@ -536,7 +536,7 @@ __global__ void __launch_bounds__(NT, NS >= 512 ? (NT >= 256 ? 1 : 256 / NT) : (
 		v[j] = cfma(m2, v0, cfma(m4, v1, cmul(m5, v2)));
 	}
 	if constexpr (SURF) {
-		const float4 *rrow = reinterpret_cast<const float4 *>(p.Rm + ((size_t)kx * p.gZ + kz) * DY * 6);
+		const C *rrow = p.Rm + ((size_t)kx * p.gZ + kz) * (6 * row_pitch(DY));
 #pragma unroll 1
 		for (int c = 0; c < 3; c++) {
 			C *ub = slot + (c == 1 ? 2 : 3) * BUF; // u_0 and u_2 in slot 3, u_1 in slot 2 (free after component 2)
@@ -565,29 +565,18 @@ __global__ void __launch_bounds__(NT, NS >= 512 ? (NT >= 256 ? 1 : 256 / NT) : (
 			for (int j = 0; j < E; j++) {
 				const int ky = j1 + T * j;
 				const bool qy = ky >= DY;
-				const float4 *f = rrow + (size_t)(qy ? NS - ky : ky) * 3;
-				const float4 d0 = __ldg(f), d1 = __ldg(f + 1), d2 = __ldg(f + 2);
-				C a0, a1, a2; // column c of R~ with the reduced-y signs of xy and yz
-				if (c == 0) {
-					a0 = make_float2(d0.x, d0.y);
-					a1 = make_float2(d0.z, d0.w);
-					a2 = make_float2(-d1.x, -d1.y);
-					if (qy) a1 = cneg(a1);
-				}
-				else if (c == 1) {
-					a0 = make_float2(d0.z, d0.w);
-					a1 = make_float2(d1.z, d1.w);
-					a2 = make_float2(-d2.x, -d2.y);
-					if (qy) {
+				// column c of R~ with the reduced-y signs of xy and yz: (xx, xy, -xz), (xy, yy, -yz), (xz, yz, zz)
+				constexpr int RP = row_pitch(DY);
+				const C *f = rrow + (qy ? NS - ky : ky);
+				C a0 = __ldg(f + (c == 0 ? 0 : c == 1 ? RP : 2 * RP)), a1 = __ldg(f + (c == 0 ? RP : c == 1 ? 3 * RP : 4 * RP)),
+				  a2 = __ldg(f + (c == 0 ? 2 * RP : c == 1 ? 4 * RP : 5 * RP));
+				if (c < 2) a2 = cneg(a2);
+				if (qy) {
+					if (c == 1) {
 						a0 = cneg(a0);
 						a2 = cneg(a2);
 					}
-				}
-				else {
-					a0 = make_float2(d1.x, d1.y);
-					a1 = make_float2(d2.x, d2.y);
-					a2 = make_float2(d2.z, d2.w);
-					if (qy) a1 = cneg(a1);
+					else a1 = cneg(a1);
 				}
 				slot[j * T + j1] = cfma(a0, u[j], slot[j * T + j1]);
 				slot[BUF + j * T + j1] = cfma(a1, u[j], slot[BUF + j * T + j1]);
@@ -731,7 +720,7 @@ inline int static_len(int n)
 // component at 512, compiled for fewer resident blocks)
 template <typename T> inline bool use_k2b_reg(int gY)
 {
-	return sizeof(T) == 4 && (gY == 64 || gY == 128 || gY == 256 || gY == 512);
+	return sizeof(T) == 4 && planar_rows(gY);
 }
 
 // shared memory of a tile kernel for nl lines of length n: one tile in the column form (FP32, compile-time length),
