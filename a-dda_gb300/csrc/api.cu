@@ -379,6 +379,7 @@ static int create_impl(const adda_gb300_problem *p, adda_gb300_ctx *c, const std
 	c->CK32max = c->chunk_fixed ? c->CK32
 		: (int)std::max<size_t>(1, std::min<size_t>(c->gX, ((size_t)CHUNK_TUNE_MAX_MB << 20) / (slab * sizeof(float2))));
 	const size_t tz = std::max(c->CK64 * sizeof(double2), c->CK32max * sizeof(float2)) * slab;
+	c->Tz_bytes = tz;
 	ADDA_CUDA(cudaMalloc(&c->Tz, tz));
 	ADDA_CUDA(cudaMalloc(&c->Tz2, tz));
 	if (c->surface) {

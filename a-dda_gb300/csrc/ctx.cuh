@@ -151,6 +151,7 @@ struct adda_gb300_ctx {
 	// matvec work
 	void *Xf = nullptr;               // [R][gX][3][bZ][bY] after the X transform
 	void *Tz = nullptr;               // [R][CK][3][gZ][bY] chunk of x-slabs after the Z transform
+	size_t Tz_bytes = 0;
 	void *TzR = nullptr;              // surface: the same chunk transformed along z with the inverse sign
 	// the odd chunks' buffers and stream: two chunks of the y/z stage run at once (one's K2a/K2b/K2c filling the
 	// other's tail), joined before K3 by events (also inside a stream capture)

@@ -20,6 +20,7 @@
 #include "ctx.cuh"
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 
 namespace adda {
@@ -29,7 +30,7 @@ namespace {
 constexpr int FLD_RUN = 128;        // dipoles whose limb products fit 64-bit sums: 2^55 each
 constexpr int FLD_SPAN = 512;       // dipoles whose sums stay below 2^62 in fixed point
 constexpr int FLD_RESIDENT = 20;    // resident warps (blocks) an SM of the sum
-constexpr int FLD_FIN = 8;          // threads that add up a direction's partial sums
+constexpr int FLD_FIN_D = 8;        // directions per block of the last sum
 constexpr size_t FLD_TABLE = 64u << 20; // bytes of phase tables per launch (bounds the directions of one)
 
 // largest high word of |P|'s components per RHS (hmax zeroed before)
@@ -175,40 +176,50 @@ __device__ __forceinline__ double2 cmuld(double2 a, double2 b)
 {
 	return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
-// 32 directions of one RHS per block: fixed-order sum of the partials (FLD_FIN threads a direction), (I - nn), and the
+// FLD_FIN_D directions of one RHS per block: fixed-order sum of the partials (32 threads a direction), (I - nn), and the
 // factor (-i k^3) exp(-i k r0.n) with r0 the centre offset of the box's first dipole (make_particle.c:2305-2308).
 // out [R][ndir][3], directions d0...
-__global__ void __launch_bounds__(32 * FLD_FIN) fld_finish(const double *part, int slices, int nd, int ld, int R,
+__global__ void __launch_bounds__(32 * FLD_FIN_D) fld_finish(const double *part, int slices, int nd, int ld, int R,
 	const double *dirs, double k, double gs, int bX, int bY, int bZ, double2 *out, int ndir, int d0)
 {
-	__shared__ double sh[FLD_FIN][6][32];
-	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, r = blockIdx.y, d = blockIdx.x * 32 + lane;
+	__shared__ double sh[32][6][FLD_FIN_D], amp[2][FLD_FIN_D];
+	const int l = threadIdx.x % FLD_FIN_D, w = threadIdx.x / FLD_FIN_D, r = blockIdx.y, d = blockIdx.x * FLD_FIN_D + l;
 	double s[6] = {0, 0, 0, 0, 0, 0};
 	if (d < nd)
-		for (int b = w; b < slices; b += FLD_FIN)
+		for (int b = w; b < slices; b += 32)
 #pragma unroll
 			for (int c = 0; c < 6; c++) s[c] += part[(((size_t)b * R + r) * 6 + c) * ld + d];
 #pragma unroll
-	for (int c = 0; c < 6; c++) sh[w][c][lane] = s[c];
+	for (int c = 0; c < 6; c++) sh[w][c][l] = s[c];
+	double n[3] = {0, 0, 0};
+	if (d < nd)
+		for (int c = 0; c < 3; c++) n[c] = dirs[3 * d + c];
+	if (w == 31) { // the last warp, while the first ones add up
+		const double r0[3] = {-gs * (bX - 1) / 2.0, -gs * (bY - 1) / 2.0, -gs * (bZ - 1) / 2.0};
+		double sn, cs;
+		sincos(-k * (r0[0] * n[0] + r0[1] * n[1] + r0[2] * n[2]), &sn, &cs);
+		const double k3 = k * k * k;
+		amp[0][l] = sn * k3; // -i k^3 (cs + i sn)
+		amp[1][l] = -cs * k3;
+	}
+	__syncthreads();
+	if (w < 6) {
+		double t = sh[0][w][l];
+		for (int b = 1; b < 32; b++) t += sh[b][w][l];
+		sh[0][w][l] = t; // this thread's own
+	}
 	__syncthreads();
 	if (w || d >= nd) return;
 #pragma unroll
-	for (int c = 0; c < 6; c++)
-		for (int b = 1; b < FLD_FIN; b++) s[c] += sh[b][c][lane];
-	const double n[3] = {dirs[3 * d], dirs[3 * d + 1], dirs[3 * d + 2]};
+	for (int c = 0; c < 6; c++) s[c] = sh[0][c][l];
 	double2 dpr = make_double2(0, 0);
 	for (int c = 0; c < 3; c++) {
 		dpr.x += s[2 * c] * n[c];
 		dpr.y += s[2 * c + 1] * n[c];
 	}
-	const double r0[3] = {-gs * (bX - 1) / 2.0, -gs * (bY - 1) / 2.0, -gs * (bZ - 1) / 2.0};
-	double sn, cs;
-	sincos(-k * (r0[0] * n[0] + r0[1] * n[1] + r0[2] * n[2]), &sn, &cs);
-	const double k3 = k * k * k;
-	const double2 amp = make_double2(sn * k3, -cs * k3); // -i k^3 (cs + i sn)
 	for (int c = 0; c < 3; c++)
-		out[((size_t)r * ndir + d0 + d) * 3 + c] = cmuld(amp, make_double2(s[2 * c] - dpr.x * n[c],
-			s[2 * c + 1] - dpr.y * n[c]));
+		out[((size_t)r * ndir + d0 + d) * 3 + c] = cmuld(make_double2(amp[0][l], amp[1][l]),
+			make_double2(s[2 * c] - dpr.x * n[c], s[2 * c + 1] - dpr.y * n[c]));
 }
 
 } // namespace
@@ -221,22 +232,29 @@ int scattered_fields(adda_gb300_ctx *c, int R, int ndir, const double *dirs, dou
 	// directions per launch: the tables' budget, a multiple of 32 within the grid's limit
 	const int per = (int)std::max<size_t>(32, std::min<size_t>(32768, FLD_TABLE / (rows * sizeof(int4)) / 32 * 32));
 	const int ld = std::min(per, (ndir + 31) / 32 * 32), groups = ld / 32;
-	// ranges of dipoles: three waves of resident warps (lines of different length even out), at least 256 dipoles each
+	// ranges of dipoles: three waves of resident warps (lines of different length even out); where few directions leave the
+	// chip emptier than that, sqrt(N / 16) dipoles each, at least 16: a dipole costs a lone warp 0.44 us (latency), a range
+	// 0.025 us in fld_finish. Measured with 33 to 80 directions (sum and finish, ranges of 256 -> this): 16x8x8 box 119 ->
+	// 20 us, 36x27x22 ellipsoid 127 -> 36, 42^3 sphere 142 -> 62
 	const size_t warps = (size_t)152 * FLD_RESIDENT * 3, per_slice = (size_t)groups * R;
-	const size_t slices = std::max<size_t>(1, std::min<size_t>((N + 255) / 256, warps / per_slice));
+	const size_t least = std::max<size_t>(16, (size_t)std::sqrt((double)N / 16));
+	const size_t slices = std::max<size_t>(1, std::min<size_t>((N + least - 1) / least, warps / per_slice));
 	const size_t span = std::max<size_t>(1, (N + slices - 1) / slices);
 	const auto up = [](size_t v) { return (v + 255) / 256 * 256; };
 	const size_t b_dirs = up(sizeof(double) * 3 * ndir), b_out = up(sizeof(double2) * 3 * (size_t)ndir * R),
 				 b_max = up(sizeof(int) * R), b_tab = up(sizeof(int4) * rows * ld), b_part = up(sizeof(double) * slices * R * 6 * ld);
 	const size_t need = b_dirs + b_out + b_max + b_tab + b_part;
-	if (need > c->fld_bytes) {
+	// the work space is the matvec's chunk buffer, free between two matvecs of the context's stream, where that is large
+	// enough: allocating 2 MB costs a context's first call 100 us
+	const bool own = need > c->Tz_bytes;
+	if (own && need > c->fld_bytes) {
 		if (c->fld) cudaFree(c->fld);
 		c->fld = nullptr;
 		c->fld_bytes = 0;
 		ADDA_CUDA(cudaMalloc(&c->fld, need));
 		c->fld_bytes = need;
 	}
-	unsigned char *at = (unsigned char *)c->fld;
+	unsigned char *at = (unsigned char *)(own ? c->fld : c->Tz);
 	const auto take = [&](size_t n) {
 		unsigned char *q = at;
 		at += n;
@@ -263,7 +281,7 @@ int scattered_fields(adda_gb300_ctx *c, int R, int ndir, const double *dirs, dou
 		fld_sum<<<dim3(groups, (unsigned)slices, R), 32, 0, s>>>(d_p, c->d_pos, c->d_xy, c->d_line_start, N, d_tab, d_max, nd,
 			ld, c->bX, c->bY, c->bZ, span, d_part, c->rpp, c->lat_stride);
 		ADDA_LAUNCHED();
-		fld_finish<<<dim3(groups, R), 32 * FLD_FIN, 0, s>>>(d_part, (int)slices, nd, ld, R, d_dirs + 3 * (size_t)d0, c->k,
+		fld_finish<<<dim3((nd + FLD_FIN_D - 1) / FLD_FIN_D, R), 32 * FLD_FIN_D, 0, s>>>(d_part, (int)slices, nd, ld, R, d_dirs + 3 * (size_t)d0, c->k,
 			c->gridspace, c->bX, c->bY, c->bZ, d_out, ndir, d0);
 		ADDA_LAUNCHED();
 	}

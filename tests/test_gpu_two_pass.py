@@ -1,4 +1,5 @@
-"""The matvec on two-pass transforms (axis lengths n = r1*r2 with radices up to 32): the FP64 matvec, in 64-bit fixed point, and the FP32 matvec of lengths without compile-time kernels.
+"""The matvec on two-pass transforms (axis lengths n = r1*r2 with radices up to 32): the FP64 matvec, in 64-bit fixed
+point, and the FP32 matvec of lengths without compile-time kernels.
 
 FP64 tolerance: a transform adds noise of about 2^-54 of its block's largest value, six transforms and the D product
 follow one another, and the largest value of these random data is below 16 times their rms: 7 * 16 * 2^-54 = 6e-15.
