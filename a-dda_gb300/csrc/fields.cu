@@ -76,17 +76,21 @@ __global__ void __launch_bounds__(256) fld_tables(const double *dirs, int nd, in
 	if (d >= nd) return;
 	const int axis = t < bX ? 0 : t < bX + bY ? 1 : 2;
 	const int i = t - (axis ? bX : 0) - (axis == 2 ? bY : 0);
+	// the phase ph + lo to twice the precision: a table's error is the same for every dipole of a plane, so it averages
+	// out less than the rounding of a phase per dipole
+	const double n = dirs[3 * d + axis], t0 = n * i, ph = -kd * t0, lo = __fma_rn(-kd, t0, -ph) - kd * __fma_rn(n, i, -t0);
 	double sn, cs;
-	sincos(-kd * (dirs[3 * d + axis] * i), &sn, &cs);
+	sincos(ph, &sn, &cs);
+	const long long c = __double2ll_rn(cs * 4611686018427387904.0) + __double2ll_rn(-lo * sn * 4611686018427387904.0);
+	const long long q = __double2ll_rn(sn * 4611686018427387904.0) + __double2ll_rn(lo * cs * 4611686018427387904.0);
 	int4 o;
 	if (axis == 0) {
-		fld_limbs(__double2ll_rn(cs * 18014398509481984.0), o.x, o.y);
-		fld_limbs(__double2ll_rn(sn * 18014398509481984.0), o.z, o.w);
+		fld_limbs(fx_rshift(c, 8), o.x, o.y);
+		fld_limbs(fx_rshift(q, 8), o.z, o.w);
 	}
 	else {
-		const long long c = __double2ll_rn(cs * 4611686018427387904.0), s = __double2ll_rn(sn * 4611686018427387904.0);
 		fx_split(c, o.x, o.y);
-		fx_split(s, o.z, o.w);
+		fx_split(q, o.z, o.w);
 		o.y = max(o.y, -0x7fffffff); // negated in fx_cmul
 		o.w = max(o.w, -0x7fffffff);
 	}
@@ -204,9 +208,15 @@ __global__ void __launch_bounds__(32 * FLD_FIN_D) fld_finish(const double *part,
 	}
 	__syncthreads();
 	if (w < 6) {
-		double t = sh[0][w][l];
-		for (int b = 1; b < 32; b++) t += sh[b][w][l];
-		sh[0][w][l] = t; // this thread's own
+		// pairwise: a serial sum of 32 rounds twice as much as the dipoles' sums
+		double t[32];
+#pragma unroll
+		for (int b = 0; b < 32; b++) t[b] = sh[b][w][l];
+#pragma unroll
+		for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+			for (int b = 0; b < o; b++) t[b] += t[b + o];
+		sh[0][w][l] = t[0]; // this thread's own
 	}
 	__syncthreads();
 	if (w || d >= nd) return;
