@@ -10,8 +10,10 @@
 //   - P (relative to the largest |component| of the RHS) and X are 54-bit fixed point in two signed limbs of 27 bits.
 //     A complex product is 12 32x32+64-bit multiply-adds (2 cycles each); the limb products of up to FLD_RUN dipoles
 //     accumulate in 64 bits without carries.
-// One unit is 2^-54 of the largest P component (FP64 rounding of a typical term) and the tables are accurate to 2^-53;
-// the rounding of the phase's argument dominates both this and a direct FP64 sum (2e-15 at 64^3).
+// One unit is 2^-54 of the largest P component (FP64 rounding of a typical term); the phases of the tables and of the
+// box centre are taken to twice the precision before the sine. Error of the fields against extended precision (direct
+// FP64 sum with a sincos per dipole -> this): 12^3 to 16^3 boxes 3.1-4.5e-16 -> 4.2-5.1e-16, 20^3 4.8e-16 -> 2.6e-16,
+// 36x27x22 8.0e-16 -> 5.9e-16.
 // Measured: 64^3 sphere (137 k dipoles), 2 RHS, 2080 directions, with the host copies and the cross sections: 57.1 ms
 // with an FP64 sincos per dipole and direction -> 3.27 ms, of which fld_sum 3.1 ms (66 instructions a dipole and warp;
 // the multiply-add pipe's bound is 1.3 ms, the rest are the loads' latency at 20 warps an SM). One warp per block: with
@@ -199,9 +201,21 @@ __global__ void __launch_bounds__(32 * FLD_FIN_D) fld_finish(const double *part,
 	if (d < nd)
 		for (int c = 0; c < 3; c++) n[c] = dirs[3 * d + c];
 	if (w == 31) { // the last warp, while the first ones add up
-		const double r0[3] = {-gs * (bX - 1) / 2.0, -gs * (bY - 1) / 2.0, -gs * (bZ - 1) / 2.0};
+		// phase -k r0.n = k gs n.(box - 1)/2, to twice the precision like the tables'
+		const double m[3] = {(bX - 1) / 2.0, (bY - 1) / 2.0, (bZ - 1) / 2.0};
+		double h = 0, lo = 0;
+		for (int c = 0; c < 3; c++) {
+			const double t = n[c] * m[c], g = h + t, z = g - h;
+			lo += __fma_rn(n[c], m[c], -t) + ((h - (g - z)) + (t - z));
+			h = g;
+		}
+		const double kg = k * gs, ph = kg * h;
+		lo = __fma_rn(kg, h, -ph) + __fma_rn(k, gs, -kg) * h + kg * lo;
 		double sn, cs;
-		sincos(-k * (r0[0] * n[0] + r0[1] * n[1] + r0[2] * n[2]), &sn, &cs);
+		sincos(ph, &sn, &cs);
+		const double c0 = cs;
+		cs = __fma_rn(-lo, sn, cs);
+		sn = __fma_rn(lo, c0, sn);
 		const double k3 = k * k * k;
 		amp[0][l] = sn * k3; // -i k^3 (cs + i sn)
 		amp[1][l] = -cs * k3;
