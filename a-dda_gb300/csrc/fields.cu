@@ -69,9 +69,11 @@ __global__ void __launch_bounds__(256) fld_split(const double2 *P, size_t n3, co
 	}
 }
 
-// phase tables of nd directions (row length ld): x factors as limbs of 2^54, y and z factors as 2^62 split for fx_cmul
+// phase tables of nd directions (row length ld): x factors as limbs of 2^54, y and z factors as 2^62 split for fx_cmul.
+// kd + kl: the wave number times the spacing, k gs, to twice the precision, as in fld_finish: a rounding of it that only
+// one of the two had would grow with the distance from the box's corner (1.4e-14 at the far end of a 300 long box)
 __global__ void __launch_bounds__(256) fld_tables(const double *dirs, int nd, int ld, int bX, int bY, int bZ, double kd,
-	int4 *tab)
+	double kl, int4 *tab)
 {
 	const int d = blockIdx.x * blockDim.x + threadIdx.x;
 	int t = blockIdx.y; // table row: x, then y, then z
@@ -80,7 +82,8 @@ __global__ void __launch_bounds__(256) fld_tables(const double *dirs, int nd, in
 	const int i = t - (axis ? bX : 0) - (axis == 2 ? bY : 0);
 	// the phase ph + lo to twice the precision: a table's error is the same for every dipole of a plane, so it averages
 	// out less than the rounding of a phase per dipole
-	const double n = dirs[3 * d + axis], t0 = n * i, ph = -kd * t0, lo = __fma_rn(-kd, t0, -ph) - kd * __fma_rn(n, i, -t0);
+	const double n = dirs[3 * d + axis], t0 = n * i, ph = -kd * t0,
+				 lo = __fma_rn(-kd, t0, -ph) - kd * __fma_rn(n, i, -t0) - kl * t0;
 	double sn, cs;
 	sincos(ph, &sn, &cs);
 	const long long c = __double2ll_rn(cs * 4611686018427387904.0) + __double2ll_rn(-lo * sn * 4611686018427387904.0);
@@ -297,10 +300,11 @@ int scattered_fields(adda_gb300_ctx *c, int R, int ndir, const double *dirs, dou
 	ADDA_LAUNCHED();
 	fld_split<<<gp, 256, 0, s>>>(c->pvec64, n3, d_max, d_p);
 	ADDA_LAUNCHED();
+	const double kd = c->k * c->gridspace, kl = std::fma(c->k, c->gridspace, -kd);
 	for (int d0 = 0; d0 < ndir; d0 += ld) {
 		const int nd = std::min(ld, ndir - d0);
 		fld_tables<<<dim3((nd + 255) / 256, (unsigned)rows), 256, 0, s>>>(d_dirs + 3 * (size_t)d0, nd, ld, c->bX, c->bY, c->bZ,
-			c->k * c->gridspace, d_tab);
+			kd, kl, d_tab);
 		ADDA_LAUNCHED();
 		fld_sum<<<dim3(groups, (unsigned)slices, R), 32, 0, s>>>(d_p, c->d_pos, c->d_xy, c->d_line_start, N, d_tab, d_max, nd,
 			ld, c->bX, c->bY, c->bZ, span, d_part, c->rpp, c->lat_stride);

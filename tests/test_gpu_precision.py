@@ -52,3 +52,69 @@ def test_uncoupled_components_of_a_flat_box(box):
             err = np.sqrt(float((np.abs(y[r, :, a] - want[:, a]) ** 2).sum() / (np.abs(want[:, a]) ** 2).sum()))
             assert err < TOL, (r, a, err)
     c.close()
+
+
+# ---------------------------------------------------------------------------------------------------------------------
+# Scattered fields. Tolerance: three phase factors of a term and the box centre's have 1.5 * 2^-53 each (a sine's 1 ulp
+# and its rounding to the table), the polarisations 2^-54 of their largest, about 5 times their rms, and the last sums, the
+# projection and the products a handful of 2^-53; all random: sqrt(4 * 1.5^2 + 2.5^2 + 6) * 2^-53 = 5e-16 of the rms field,
+# with a factor of 4 for the fields of single directions.
+FIELD_TOL = 2e-15
+
+
+def full_box(box, k, dpl=15.0):
+    s = cube_setup(box, tuple(2 * b for b in box))
+    s.kd, s.wavenum = 2 * math.pi / dpl, k
+    s.gridspace = s.kd / k
+    s.cc = [np.array([(0.3 + 0.02j) * s.gridspace ** 3] * 3)] * 2
+    return s
+
+
+def fields_of(s, x, dirs):
+    """the context's fields for x handed over as the solution (no iterations), and the polarisations they are of"""
+    import torch
+    R = len(x)
+    c = context(s, R=R)
+    d_x = torch.from_numpy(np.ascontiguousarray(x.reshape(R, -1), dtype=np.complex128).view(np.float64)).cuda()
+    d_p = torch.empty_like(d_x)
+    torch.cuda.synchronize()
+    c.solve_device(d_x.data_ptr(), R, d_x.data_ptr(), d_p.data_ptr(), prec="fp64", maxiter=0, init="x0")
+    torch.cuda.synchronize()
+    e = c.scattered_fields(dirs, R)
+    c.close()
+    return e, d_p.cpu().numpy().view(np.complex128).reshape(R, s.n, 3)
+
+
+def fields_direct(s, P, dirs):
+    """-i k^3 (I - nn) sum P exp(-i k n.r), r from the box centre, in extended precision"""
+    r = LD(s.gridspace) * (s.pos.astype(LD) - (np.array(s.box, dtype=LD) - 1) / 2)
+    out = np.empty((len(P), len(dirs), 3), CLD)
+    for i, d in enumerate(dirs.astype(LD)):
+        w = np.exp(-1j * (LD(s.wavenum) * (r @ d)).astype(CLD))
+        for q in range(len(P)):
+            f = w @ P[q].astype(CLD)
+            out[q, i] = -1j * LD(s.wavenum) ** 3 * (f - d * (f @ d))
+    return out
+
+
+def field_errors(got, want):
+    """per RHS and direction, relative to that direction's field"""
+    n = lambda v: np.sqrt((np.abs(v) ** 2).sum(-1).astype(np.float64))
+    return n(got - want) / n(want)
+
+
+def some_dirs(n, seed):
+    d = np.random.default_rng(seed).standard_normal((n, 3))
+    return d / np.linalg.norm(d, axis=1, keepdims=True)
+
+
+@pytest.mark.parametrize("k", [2 * math.pi, 2 * math.pi / 0.6328, 0.7, 9.3e6])
+@pytest.mark.parametrize("box", [(300, 2, 3), (3, 300, 2), (2, 3, 300)])
+def test_fields_with_any_wave_number(box, k):
+    """k times the spacing is not a double: every factor of the phase, and the box centre's, takes the same value of it"""
+    s = full_box(box, k)
+    x = random_vec(s.n, 2, 7)
+    dirs = np.concatenate([some_dirs(40, 3), [[0.8, 0.6, 0], [0.6, 0, 0.8]]])
+    e, P = fields_of(s, x, dirs)
+    err = field_errors(e, fields_direct(s, P, dirs))
+    assert np.sqrt((err ** 2).mean()) < FIELD_TOL
