@@ -54,6 +54,32 @@ __device__ __forceinline__ void fld_limbs(long long v, int &h, int &l)
 	l = (int)((unsigned)v << 5) >> 5;
 	h = (int)((v - l) >> 27);
 }
+// d in units of 2^(emax - 1076), |result| < 2^54, rounded once and away from zero in the middle: as many values up as down
+// (a second rounding, or one towards +infinity, adds up over the dipoles: 3e-14 of the field of 40000)
+__device__ __forceinline__ long long fld_fixed(double d, int emax)
+{
+	const int hi = __double2hiint(d), ex = (hi >> 20) & 0x7ff, sh = emax - max(ex, 1);
+	long long m = ((long long)((hi & 0xfffff) | (ex ? 0x100000 : 0)) << 33) | (long long)(unsigned)__double2loint(d) << 1;
+	m = sh > 60 ? 0 : sh ? fx_rshift(m, sh) : m;
+	return hi < 0 ? -m : m;
+}
+// acc += v * w without a rounding: the low words collect in lo (carried over into acc), the rest as fx_cmul
+__device__ __forceinline__ void fld_madd(fx2 v, int4 w, long long &ax, long long &ay, unsigned &lx, unsigned &ly)
+{
+	int xh, xl, yh, yl;
+	fx_split(v.x, xh, xl);
+	fx_split(v.y, yh, yl);
+	long long t = (long long)xh * w.y + (long long)xl * w.x;
+	t = (long long)yh * -w.w + t;
+	t = (long long)yl * -w.z + t;
+	long long u = (long long)xh * w.w + (long long)xl * w.z;
+	u = (long long)yh * w.y + u;
+	u = (long long)yl * w.x + u;
+	lx += (unsigned)t;
+	ly += (unsigned)u;
+	ax += (long long)xh * w.x + ((long long)yh * -w.z + ((t >> 32) + (lx < (unsigned)t)));
+	ay += (long long)xh * w.z + ((long long)yh * w.x + ((u >> 32) + (ly < (unsigned)u)));
+}
 // P in limbs: component i of RHS r at [r*n3 + i], (re high, re low, im high, im low)
 __global__ void __launch_bounds__(256) fld_split(const double2 *P, size_t n3, const int *hmax, int4 *out)
 {
@@ -62,9 +88,8 @@ __global__ void __launch_bounds__(256) fld_split(const double2 *P, size_t n3, co
 	for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n3; i += (size_t)gridDim.x * blockDim.x) {
 		const double2 v = P[r * n3 + i];
 		int4 o;
-		// fx_from_double gives |v| < 2^FX_TOP: down to 54 bits, value = v * 2^(emax - 1076)
-		fld_limbs(fx_rshift(fx_from_double(v.x, emax), FX_TOP - 54), o.x, o.y);
-		fld_limbs(fx_rshift(fx_from_double(v.y, emax), FX_TOP - 54), o.z, o.w);
+		fld_limbs(fld_fixed(v.x, emax), o.x, o.y);
+		fld_limbs(fld_fixed(v.y, emax), o.z, o.w);
 		out[r * n3 + i] = o;
 	}
 }
@@ -124,6 +149,7 @@ __global__ void __launch_bounds__(32, FLD_RESIDENT) fld_sum(const int4 *P, const
 	while (i < i1) {
 		const size_t iend = min(i1, i + FLD_SPAN);
 		long long S[6] = {0, 0, 0, 0, 0, 0};
+		unsigned low[6] = {0, 0, 0, 0, 0, 0};
 		while (i < iend) {
 			// one run: dipoles of one x-line, at most FLD_RUN of them
 			const int y = pos[3 * i + 1], z = pos[3 * i + 2];
@@ -161,18 +187,20 @@ __global__ void __launch_bounds__(32, FLD_RESIDENT) fld_sum(const int4 *P, const
 			int4 yz;
 			fx_split(q.x << 2, yz.x, yz.y);
 			fx_split(q.y << 2, yz.z, yz.w);
-			yz.y = max(yz.y, -0x7fffffff); // negated in fx_cmul
-			yz.w = max(yz.w, -0x7fffffff);
+			yz.w = max(yz.w, -0x7fffffff); // negated in fld_madd
 #pragma unroll
 			for (int c = 0; c < 3; c++) {
 				// (U * 2^54 + T * 2^27) / 2^54
-				const fx2 s = fx_cmul(fx2{U[2 * c] + (T[2 * c] >> 27), U[2 * c + 1] + (T[2 * c + 1] >> 27)}, yz, false);
-				S[2 * c] += s.x;
-				S[2 * c + 1] += s.y;
+				fld_madd(fx2{U[2 * c] + (T[2 * c] >> 27), U[2 * c + 1] + (T[2 * c + 1] >> 27)}, yz, S[2 * c], S[2 * c + 1],
+					low[2 * c], low[2 * c + 1]);
 			}
 		}
 #pragma unroll
-		for (int c = 0; c < 6; c++) tot[c] += fx_to_double(S[c], e);
+		for (int c = 0; c < 6; c++) {
+			// the upper 62 bits of S and low
+			const int sh = max(0, min(__clzll(S[c] ^ (S[c] >> 63)) - 2, 31));
+			tot[c] += fx_to_double((S[c] << sh) + (long long)(sh ? low[c] >> (32 - sh) : 0), e - sh);
+		}
 	}
 	if (d < nd) {
 		double *o = part + ((size_t)blockIdx.y * R + r) * 6 * ld + d;

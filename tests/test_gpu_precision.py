@@ -118,3 +118,19 @@ def test_fields_with_any_wave_number(box, k):
     e, P = fields_of(s, x, dirs)
     err = field_errors(e, fields_direct(s, P, dirs))
     assert np.sqrt((err ** 2).mean()) < FIELD_TOL
+
+
+@pytest.mark.parametrize("size", [1.0, 0.25, 0.0625])
+@pytest.mark.parametrize("d", [(1, 0, 0), (-1, 0, 0), (0, 0.6, 0.8)])
+def test_field_roundings_do_not_lean(size, d):
+    """a plate's polarisations of random sign whose last bit falls in the middle of the fixed-point unit (one larger dipole
+    sets the unit): if the middle always goes up, 40000 of them add 1e-16 each to a field of 200"""
+    s = full_box((1, 200, 200), 1.0)
+    s.cc = [np.ones(3)] * 2
+    g = np.random.default_rng(5)
+    v = size * (1 + 2.0 ** -52)
+    x = v * (g.choice([-1, 1], (2, s.n, 3)) + 1j * g.choice([-1, 1], (2, s.n, 3)))
+    x[:, 0] = 1
+    e, P = fields_of(s, x, np.array([d], dtype=float))
+    assert np.array_equal(P, x)
+    assert field_errors(e, fields_direct(s, P, np.array([d], dtype=float))).max() < FIELD_TOL
