@@ -7,15 +7,17 @@
 //     tables of (boxX + boxY + boxZ) values per direction instead of one sincos per dipole and direction;
 //   - along an x-line only X[x] changes: the dipoles of a line are summed with it, and the line's sum is multiplied by
 //     Y[y] Z[z];
-//   - P (relative to the largest |component| of the RHS) and X are 54-bit fixed point in two signed limbs of 27 bits.
+//   - P (relative to the RHS's largest value of the same component: a field along a dominant component is made of the
+//     other two only) and X are 54-bit fixed point in two signed limbs of 27 bits.
 //     A complex product is 12 32x32+64-bit multiply-adds (2 cycles each); the limb products of up to FLD_RUN dipoles
 //     accumulate in 64 bits without carries.
 // One unit is 2^-54 of the largest P component (FP64 rounding of a typical term); the phases of the tables and of the
-// box centre are taken to twice the precision before the sine. Error of the fields against extended precision (direct
-// FP64 sum with a sincos per dipole -> this): 12^3 to 16^3 boxes 3.1-4.5e-16 -> 4.2-5.1e-16, 20^3 4.8e-16 -> 2.6e-16,
-// 36x27x22 8.0e-16 -> 5.9e-16.
+// box centre are taken to twice the precision before the sine, from the same k gs, and no rounding leans to one side.
+// Error of the fields against 80-bit sums (direct FP64 sum with a sincos per dipole -> this): 12^3 box 3.0e-16 -> 2.1e-16,
+// 20^3 5.7e-16 -> 2.4e-16, 36x28x22 9.4e-16 -> 2.7e-16, 64^3 1.4e-15 -> 2.9e-16. (A plain FP64 sum in numpy or torch is
+// itself 5e-15 off at 64^3.)
 // Measured: 64^3 sphere (137 k dipoles), 2 RHS, 2080 directions, with the host copies and the cross sections: 57.1 ms
-// with an FP64 sincos per dipole and direction -> 3.27 ms, of which fld_sum 3.1 ms (66 instructions a dipole and warp;
+// with an FP64 sincos per dipole and direction -> 3.36 ms, of which fld_sum 3.2 ms (66 instructions a dipole and warp;
 // the multiply-add pipe's bound is 1.3 ms, the rest are the loads' latency at 20 warps an SM). One warp per block: with
 // blocks of four warps the last wave was half empty (5.4 ms, with a data-dependent loop over the dipoles).
 #include "fft_lines2.cuh"
@@ -29,23 +31,30 @@ namespace adda {
 
 namespace {
 
+constexpr int FLD_NT = 192;         // threads per block of the passes over P
 constexpr int FLD_RUN = 128;        // dipoles whose limb products fit 64-bit sums: 2^55 each
 constexpr int FLD_SPAN = 512;       // dipoles whose sums stay below 2^62 in fixed point
 constexpr int FLD_RESIDENT = 20;    // resident warps (blocks) an SM of the sum
 constexpr int FLD_FIN_D = 8;        // directions per block of the last sum
 constexpr size_t FLD_TABLE = 64u << 20; // bytes of phase tables per launch (bounds the directions of one)
 
-// largest high word of |P|'s components per RHS (hmax zeroed before)
-__global__ void __launch_bounds__(256) fld_max(const double2 *P, size_t n3, int *hmax)
+// largest high word of |P| per RHS and component (hmax [R][3] zeroed before). The stride is a multiple of 3, so a thread
+// stays with one component
+__global__ void __launch_bounds__(FLD_NT) fld_max(const double2 *P, size_t n3, int *hmax)
 {
-	const int r = blockIdx.y;
+	static_assert(FLD_NT % 3 == 0, "a thread's component");
+	__shared__ int s[3];
+	const int r = blockIdx.y, c = threadIdx.x % 3;
+	if (threadIdx.x < 3) s[threadIdx.x] = 0;
+	__syncthreads();
 	int h = 0;
-	for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n3; i += (size_t)gridDim.x * blockDim.x) {
+	for (size_t i = blockIdx.x * (size_t)FLD_NT + threadIdx.x; i < n3; i += (size_t)gridDim.x * FLD_NT) {
 		const double2 v = P[r * n3 + i];
 		h = max(h, max(__double2hiint(v.x) & 0x7fffffff, __double2hiint(v.y) & 0x7fffffff));
 	}
-	h = __reduce_max_sync(0xffffffffu, h);
-	if ((threadIdx.x & 31) == 0) atomicMax(hmax + r, h);
+	atomicMax(s + c, h);
+	__syncthreads();
+	if (threadIdx.x < 3) atomicMax(hmax + 3 * r + threadIdx.x, s[threadIdx.x]);
 }
 
 // two signed limbs of 27 bits of |v| < 2^54
@@ -80,12 +89,12 @@ __device__ __forceinline__ void fld_madd(fx2 v, int4 w, long long &ax, long long
 	ax += (long long)xh * w.x + ((long long)yh * -w.z + ((t >> 32) + (lx < (unsigned)t)));
 	ay += (long long)xh * w.z + ((long long)yh * w.x + ((u >> 32) + (ly < (unsigned)u)));
 }
-// P in limbs: component i of RHS r at [r*n3 + i], (re high, re low, im high, im low)
-__global__ void __launch_bounds__(256) fld_split(const double2 *P, size_t n3, const int *hmax, int4 *out)
+// P in limbs: element i of RHS r at [r*n3 + i], (re high, re low, im high, im low)
+__global__ void __launch_bounds__(FLD_NT) fld_split(const double2 *P, size_t n3, const int *hmax, int4 *out)
 {
 	const int r = blockIdx.y;
-	const int emax = max(1, hmax[r] >> 20);
-	for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n3; i += (size_t)gridDim.x * blockDim.x) {
+	const int emax = max(1, hmax[3 * r + threadIdx.x % 3] >> 20);
+	for (size_t i = blockIdx.x * (size_t)FLD_NT + threadIdx.x; i < n3; i += (size_t)gridDim.x * FLD_NT) {
 		const double2 v = P[r * n3 + i];
 		int4 o;
 		fld_limbs(fld_fixed(v.x, emax), o.x, o.y);
@@ -143,7 +152,7 @@ __global__ void __launch_bounds__(32, FLD_RESIDENT) fld_sum(const int4 *P, const
 	// the particle's own dipoles (a smaller particle of a group is padded to N)
 	const size_t i0 = (size_t)blockIdx.y * span, i1 = min((size_t)lstart[(size_t)bZ * bY], i0 + span);
 	const int4 *tx = tab + d, *ty = tx + (size_t)bX * ld, *tz = ty + (size_t)bY * ld;
-	const int e = max(1, hmax[r] >> 20) - 1074; // of S: a quarter of P's integers (fx_cmul)
+	const int hm[3] = {hmax[3 * r], hmax[3 * r + 1], hmax[3 * r + 2]};
 	double tot[6] = {0, 0, 0, 0, 0, 0};
 	size_t i = i0;
 	while (i < i1) {
@@ -197,15 +206,15 @@ __global__ void __launch_bounds__(32, FLD_RESIDENT) fld_sum(const int4 *P, const
 		}
 #pragma unroll
 		for (int c = 0; c < 6; c++) {
-			// the upper 62 bits of S and low
-			const int sh = max(0, min(__clzll(S[c] ^ (S[c] >> 63)) - 2, 31));
+			// the upper 62 bits of S and low; a unit of S is four of P's
+			const int sh = max(0, min(__clzll(S[c] ^ (S[c] >> 63)) - 2, 31)), e = max(1, hm[c / 2] >> 20) - 1074;
 			tot[c] += fx_to_double((S[c] << sh) + (long long)(sh ? low[c] >> (32 - sh) : 0), e - sh);
 		}
 	}
 	if (d < nd) {
 		double *o = part + ((size_t)blockIdx.y * R + r) * 6 * ld + d;
 #pragma unroll
-		for (int c = 0; c < 6; c++) o[(size_t)c * ld] = hmax[r] >= 0x7ff00000 ? __hiloint2double(0x7ff80000, 0) : tot[c];
+		for (int c = 0; c < 6; c++) o[(size_t)c * ld] = hm[c / 2] >= 0x7ff00000 ? __hiloint2double(0x7ff80000, 0) : tot[c];
 	}
 }
 
@@ -297,7 +306,7 @@ int scattered_fields(adda_gb300_ctx *c, int R, int ndir, const double *dirs, dou
 	const size_t span = std::max<size_t>(1, (N + slices - 1) / slices);
 	const auto up = [](size_t v) { return (v + 255) / 256 * 256; };
 	const size_t b_dirs = up(sizeof(double) * 3 * ndir), b_out = up(sizeof(double2) * 3 * (size_t)ndir * R),
-				 b_max = up(sizeof(int) * R), b_tab = up(sizeof(int4) * rows * ld), b_part = up(sizeof(double) * slices * R * 6 * ld);
+				 b_max = up(sizeof(int) * 3 * R), b_tab = up(sizeof(int4) * rows * ld), b_part = up(sizeof(double) * slices * R * 6 * ld);
 	const size_t need = b_dirs + b_out + b_max + b_tab + b_part;
 	// the work space is the matvec's chunk buffer, free between two matvecs of the context's stream, where that is large
 	// enough: allocating 2 MB costs a context's first call 100 us
@@ -322,11 +331,11 @@ int scattered_fields(adda_gb300_ctx *c, int R, int ndir, const double *dirs, dou
 	int4 *d_p = (int4 *)c->vin; // the staging buffer of the host-pointer matvec: R*3N complex doubles
 	double *d_part = (double *)take(b_part);
 	ADDA_CUDA(cudaMemcpyAsync(d_dirs, dirs, sizeof(double) * 3 * ndir, cudaMemcpyHostToDevice, s));
-	ADDA_CUDA(cudaMemsetAsync(d_max, 0, sizeof(int) * R, s));
-	const dim3 gp((unsigned)std::max<size_t>(1, std::min<size_t>((n3 + 255) / 256, 152 * 8)), R);
-	fld_max<<<gp, 256, 0, s>>>(c->pvec64, n3, d_max);
+	ADDA_CUDA(cudaMemsetAsync(d_max, 0, sizeof(int) * 3 * R, s));
+	const dim3 gp((unsigned)std::max<size_t>(1, std::min<size_t>((n3 + FLD_NT - 1) / FLD_NT, 152 * 10)), R);
+	fld_max<<<gp, FLD_NT, 0, s>>>(c->pvec64, n3, d_max);
 	ADDA_LAUNCHED();
-	fld_split<<<gp, 256, 0, s>>>(c->pvec64, n3, d_max, d_p);
+	fld_split<<<gp, FLD_NT, 0, s>>>(c->pvec64, n3, d_max, d_p);
 	ADDA_LAUNCHED();
 	const double kd = c->k * c->gridspace, kl = std::fma(c->k, c->gridspace, -kd);
 	for (int d0 = 0; d0 < ndir; d0 += ld) {

@@ -134,3 +134,15 @@ def test_field_roundings_do_not_lean(size, d):
     e, P = fields_of(s, x, np.array([d], dtype=float))
     assert np.array_equal(P, x)
     assert field_errors(e, fields_direct(s, P, np.array([d], dtype=float))).max() < FIELD_TOL
+
+
+@pytest.mark.parametrize("scale", [(1, 1e-3, 1e-6), (1e-6, 1, 1e-9), (1e-12, 1e-7, 1), (1, 1e-200, 1e-300)])
+def test_fields_along_a_dominant_component(scale):
+    """the field in the direction of a component is made of the other two alone, however small they are"""
+    s = full_box((24, 18, 14), 1.0)
+    x = random_vec(s.n, 6, 11).reshape(6, s.n, 3) * np.array(scale)
+    dirs = np.concatenate([np.eye(3), -np.eye(3), some_dirs(10, 5)])
+    e, P = fields_of(s, x, dirs)
+    want = fields_direct(s, P, dirs)
+    n = lambda v: np.sqrt((np.abs(v).astype(LD) ** 2).sum((0, 2)))  # per direction, over the right-hand sides
+    assert (n(e - want) / n(want)).max() < FIELD_TOL
