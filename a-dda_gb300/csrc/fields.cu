@@ -1,7 +1,8 @@
 // fields.cu - scattering amplitudes of the last solve in a set of directions (CalcFieldFree, crosssec.c:506-596):
 // E_r(n) = (-i k^3) exp(-i k r0.n) (I - nn) sum_j P_rj exp(-i kd n.pos_j).
 //
-// The sum is FP64-exact work on a chip whose FP64 pipe issues one instruction per 76 cycles and scheduler, so it runs on
+// One or two directions, or few dipoles: a sincos per dipole and direction (fld_few; the rule is in scattered_fields). Else
+// the sum is FP64-exact work on a chip whose FP64 pipe issues one instruction per 76 cycles and scheduler, so it runs on
 // the integer pipes:
 //   - the lattice makes the phase a product of three factors, one per axis: exp(-i kd n.pos) = X[x] Y[y] Z[z], taken from
 //     tables of (boxX + boxY + boxZ) values per direction instead of one sincos per dipole and direction;
@@ -22,6 +23,7 @@
 // blocks of four warps the last wave was half empty (5.4 ms, with a data-dependent loop over the dipoles).
 #include "fft_lines2.cuh"
 #include "ctx.cuh"
+#include "krylov.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -32,6 +34,7 @@ namespace adda {
 namespace {
 
 constexpr int FLD_NT = 192;         // threads per block of the passes over P
+constexpr int FEW_NT = 256;         // threads per block of the direct sum
 constexpr int FLD_RUN = 128;        // dipoles whose limb products fit 64-bit sums: 2^55 each
 constexpr int FLD_SPAN = 512;       // dipoles whose sums stay below 2^62 in fixed point
 constexpr int FLD_RESIDENT = 20;    // resident warps (blocks) an SM of the sum
@@ -218,6 +221,54 @@ __global__ void __launch_bounds__(32, FLD_RESIDENT) fld_sum(const int4 *P, const
 	}
 }
 
+// Few directions: partial sums in FP64 with a sincos per dipole and direction, grid (ranges, directions, RHS), positions from
+// the box centre; part as fld_sum's. The phase is a.(2 r) to twice the precision: a's high parts (few_phase) make exact
+// products and sums
+__global__ void __launch_bounds__(FEW_NT) fld_few(const double2 *P, const uint16_t *pos, const uint32_t *lstart, size_t N,
+	const double *phase, int ld, int bX, int bY, int bZ, double *part, int rpp, size_t lst)
+{
+	const int d = blockIdx.y, r = blockIdx.z, R = gridDim.z;
+	const size_t lq = (size_t)(r / rpp), lines = (size_t)bZ * bY; // RHS r's particle (group contexts)
+	pos += lq * lst * 3;
+	const size_t n1 = lstart[lq * (lines + 1) + lines];
+	double a[6];
+#pragma unroll
+	for (int c = 0; c < 6; c++) a[c] = phase[6 * d + c];
+	double s[6] = {0, 0, 0, 0, 0, 0};
+	for (size_t j = blockIdx.x * (size_t)FEW_NT + threadIdx.x; j < n1; j += (size_t)gridDim.x * FEW_NT) {
+		// twice the position from the centre: whole numbers
+		const double x = 2 * pos[3 * j] - (bX - 1), y = 2 * pos[3 * j + 1] - (bY - 1), z = 2 * pos[3 * j + 2] - (bZ - 1);
+		const double lo = __fma_rn(a[3], x, __fma_rn(a[4], y, a[5] * z));
+		double sn, cs;
+		sincos(__fma_rn(a[0], x, __fma_rn(a[1], y, a[2] * z)), &sn, &cs);
+		const double wr = __fma_rn(-lo, sn, cs), wi = __fma_rn(lo, cs, sn);
+#pragma unroll
+		for (int c = 0; c < 3; c++) {
+			const double2 p = P[((size_t)r * N + j) * 3 + c];
+			s[2 * c] += p.x * wr - p.y * wi;
+			s[2 * c + 1] += p.x * wi + p.y * wr;
+		}
+	}
+	double tot[6];
+	block_totals<6>(s, tot);
+	if (threadIdx.x == 0)
+#pragma unroll
+		for (int c = 0; c < 6; c++) part[(((size_t)blockIdx.x * R + r) * 6 + c) * ld + d] = tot[c];
+}
+// -k gs n / 2 as high parts, whole multiples of a power of two that leaves all phases of the box below 2^51 of it, and the
+// rest; kd + kl = k gs
+void few_phase(const double n[3], const int box[3], double kd, double kl, double a[6])
+{
+	double most = 0;
+	for (int c = 0; c < 3; c++) most += std::fabs(kd * n[c]) * box[c];
+	const double unit = most > 0 && most < 1e300 ? std::ldexp(1.0, std::max(std::ilogb(most) - 51, -1000)) : 1.0;
+	for (int c = 0; c < 3; c++) {
+		const double v = -0.5 * kd * n[c], lo = -0.5 * (std::fma(kd, n[c], 2 * v) + kl * n[c]);
+		a[c] = most < 1e300 ? std::nearbyint(v / unit) * unit : v;
+		a[3 + c] = (v - a[c]) + lo;
+	}
+}
+
 __device__ __forceinline__ double2 cmuld(double2 a, double2 b)
 {
 	return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
@@ -226,7 +277,7 @@ __device__ __forceinline__ double2 cmuld(double2 a, double2 b)
 // factor (-i k^3) exp(-i k r0.n) with r0 the centre offset of the box's first dipole (make_particle.c:2305-2308).
 // out [R][ndir][3], directions d0...
 __global__ void __launch_bounds__(32 * FLD_FIN_D) fld_finish(const double *part, int slices, int nd, int ld, int R,
-	const double *dirs, double k, double gs, int bX, int bY, int bZ, double2 *out, int ndir, int d0)
+	const double *dirs, double k, double kd, double kl, int bX, int bY, int bZ, double2 *out, int ndir, int d0)
 {
 	__shared__ double sh[32][6][FLD_FIN_D], amp[2][FLD_FIN_D];
 	const int l = threadIdx.x % FLD_FIN_D, w = threadIdx.x / FLD_FIN_D, r = blockIdx.y, d = blockIdx.x * FLD_FIN_D + l;
@@ -241,7 +292,7 @@ __global__ void __launch_bounds__(32 * FLD_FIN_D) fld_finish(const double *part,
 	if (d < nd)
 		for (int c = 0; c < 3; c++) n[c] = dirs[3 * d + c];
 	if (w == 31) { // the last warp, while the first ones add up
-		// phase -k r0.n = k gs n.(box - 1)/2, to twice the precision like the tables'
+		// phase -k r0.n = k gs n.(box - 1)/2, to twice the precision like the tables' (box 1: no phase, fld_few)
 		const double m[3] = {(bX - 1) / 2.0, (bY - 1) / 2.0, (bZ - 1) / 2.0};
 		double h = 0, lo = 0;
 		for (int c = 0; c < 3; c++) {
@@ -249,8 +300,8 @@ __global__ void __launch_bounds__(32 * FLD_FIN_D) fld_finish(const double *part,
 			lo += __fma_rn(n[c], m[c], -t) + ((h - (g - z)) + (t - z));
 			h = g;
 		}
-		const double kg = k * gs, ph = kg * h;
-		lo = __fma_rn(kg, h, -ph) + __fma_rn(k, gs, -kg) * h + kg * lo;
+		const double ph = kd * h;
+		lo = __fma_rn(kd, h, -ph) + kl * h + kd * lo;
 		double sn, cs;
 		sincos(ph, &sn, &cs);
 		const double c0 = cs;
@@ -292,6 +343,14 @@ int scattered_fields(adda_gb300_ctx *c, int R, int ndir, const double *dirs, dou
 {
 	const size_t N = c->N, n3 = 3 * N;
 	cudaStream_t s = c->stream;
+	const double kd = c->k * c->gridspace, kl = std::fma(c->k, c->gridspace, -kd);
+	// few directions for the dipoles and RHS at hand: a sincos each (0.13 ns of the FP64 pipes per dipole, RHS and direction)
+	// against two passes over P, the tables and 32 directions whether asked for or not (20 us and 0.3 to 0.5 ns per dipole
+	// and RHS). Measured direct / tables, us: 1, 2, 3, 4 directions of a 64^3 sphere with 1 RHS 51, 69, 82, 93 / 126, with
+	// 2 RHS 68, 94, 120, 155 / 149, of a 128^3 sphere with 2 RHS 280, 513, 748, 870 / 700; 16 directions of a 32^3 sphere
+	// with 1 RHS 60 / 65, 2 RHS 87 / 68; 60 directions of 8^3 34 / 52, 16^3 with 1 and 2 RHS 46, 58 / 52
+	const size_t work = N * (size_t)R;
+	const bool few = ndir <= 2 || work * (ndir - 2) < 250000;
 	const size_t rows = (size_t)c->bX + c->bY + c->bZ;
 	// directions per launch: the tables' budget, a multiple of 32 within the grid's limit
 	const int per = (int)std::max<size_t>(32, std::min<size_t>(32768, FLD_TABLE / (rows * sizeof(int4)) / 32 * 32));
@@ -302,12 +361,15 @@ int scattered_fields(adda_gb300_ctx *c, int R, int ndir, const double *dirs, dou
 	// 20 us, 36x27x22 ellipsoid 127 -> 36, 42^3 sphere 142 -> 62
 	const size_t warps = (size_t)152 * FLD_RESIDENT * 3, per_slice = (size_t)groups * R;
 	const size_t least = std::max<size_t>(16, (size_t)std::sqrt((double)N / 16));
-	const size_t slices = std::max<size_t>(1, std::min<size_t>((N + least - 1) / least, warps / per_slice));
+	// the direct sum: one to eight dipoles a thread, so that the FP64 pipes of all SMs have work, at most 128 ranges
+	const size_t each = FEW_NT * std::min<size_t>(8, std::max<size_t>(1, work * ndir / ((size_t)152 * 4 * FEW_NT)));
+	const size_t slices = std::max<size_t>(1, few ? std::min<size_t>((N + each - 1) / each, 128)
+		: std::min<size_t>((N + least - 1) / least, warps / per_slice));
 	const size_t span = std::max<size_t>(1, (N + slices - 1) / slices);
 	const auto up = [](size_t v) { return (v + 255) / 256 * 256; };
 	const size_t b_dirs = up(sizeof(double) * 3 * ndir), b_out = up(sizeof(double2) * 3 * (size_t)ndir * R),
-				 b_max = up(sizeof(int) * 3 * R), b_tab = up(sizeof(int4) * rows * ld), b_part = up(sizeof(double) * slices * R * 6 * ld);
-	const size_t need = b_dirs + b_out + b_max + b_tab + b_part;
+				 b_max = up(sizeof(int) * 3 * R), b_tab = few ? 0 : up(sizeof(int4) * rows * ld), b_part = up(sizeof(double) * slices * R * 6 * ld);
+	const size_t b_phase = few ? up(sizeof(double) * 6 * ndir) : 0, need = b_dirs + b_phase + b_out + b_max + b_tab + b_part;
 	// the work space is the matvec's chunk buffer, free between two matvecs of the context's stream, where that is large
 	// enough: allocating 2 MB costs a context's first call 100 us
 	const bool own = need > c->Tz_bytes;
@@ -324,30 +386,44 @@ int scattered_fields(adda_gb300_ctx *c, int R, int ndir, const double *dirs, dou
 		at += n;
 		return q;
 	};
-	double *d_dirs = (double *)take(b_dirs);
+	double *d_dirs = (double *)take(b_dirs), *d_phase = (double *)take(b_phase);
 	double2 *d_out = (double2 *)take(b_out);
 	int *d_max = (int *)take(b_max);
 	int4 *d_tab = (int4 *)take(b_tab);
 	int4 *d_p = (int4 *)c->vin; // the staging buffer of the host-pointer matvec: R*3N complex doubles
 	double *d_part = (double *)take(b_part);
 	ADDA_CUDA(cudaMemcpyAsync(d_dirs, dirs, sizeof(double) * 3 * ndir, cudaMemcpyHostToDevice, s));
-	ADDA_CUDA(cudaMemsetAsync(d_max, 0, sizeof(int) * 3 * R, s));
-	const dim3 gp((unsigned)std::max<size_t>(1, std::min<size_t>((n3 + FLD_NT - 1) / FLD_NT, 152 * 10)), R);
-	fld_max<<<gp, FLD_NT, 0, s>>>(c->pvec64, n3, d_max);
-	ADDA_LAUNCHED();
-	fld_split<<<gp, FLD_NT, 0, s>>>(c->pvec64, n3, d_max, d_p);
-	ADDA_LAUNCHED();
-	const double kd = c->k * c->gridspace, kl = std::fma(c->k, c->gridspace, -kd);
+	if (few) {
+		const int box[3] = {c->bX, c->bY, c->bZ};
+		std::vector<double> a(6 * (size_t)ndir);
+		for (int d = 0; d < ndir; d++) few_phase(dirs + 3 * (size_t)d, box, kd, kl, &a[6 * (size_t)d]);
+		ADDA_CUDA(cudaMemcpyAsync(d_phase, a.data(), sizeof(double) * a.size(), cudaMemcpyHostToDevice, s));
+	}
+	else {
+		ADDA_CUDA(cudaMemsetAsync(d_max, 0, sizeof(int) * 3 * R, s));
+		const dim3 gp((unsigned)std::max<size_t>(1, std::min<size_t>((n3 + FLD_NT - 1) / FLD_NT, 152 * 10)), R);
+		fld_max<<<gp, FLD_NT, 0, s>>>(c->pvec64, n3, d_max);
+		ADDA_LAUNCHED();
+		fld_split<<<gp, FLD_NT, 0, s>>>(c->pvec64, n3, d_max, d_p);
+		ADDA_LAUNCHED();
+	}
 	for (int d0 = 0; d0 < ndir; d0 += ld) {
 		const int nd = std::min(ld, ndir - d0);
-		fld_tables<<<dim3((nd + 255) / 256, (unsigned)rows), 256, 0, s>>>(d_dirs + 3 * (size_t)d0, nd, ld, c->bX, c->bY, c->bZ,
-			kd, kl, d_tab);
-		ADDA_LAUNCHED();
-		fld_sum<<<dim3(groups, (unsigned)slices, R), 32, 0, s>>>(d_p, c->d_pos, c->d_xy, c->d_line_start, N, d_tab, d_max, nd,
-			ld, c->bX, c->bY, c->bZ, span, d_part, c->rpp, c->lat_stride);
-		ADDA_LAUNCHED();
-		fld_finish<<<dim3((nd + FLD_FIN_D - 1) / FLD_FIN_D, R), 32 * FLD_FIN_D, 0, s>>>(d_part, (int)slices, nd, ld, R, d_dirs + 3 * (size_t)d0, c->k,
-			c->gridspace, c->bX, c->bY, c->bZ, d_out, ndir, d0);
+		const double *dd = d_dirs + 3 * (size_t)d0;
+		if (few) {
+			fld_few<<<dim3((unsigned)slices, nd, R), FEW_NT, 0, s>>>(c->pvec64, c->d_pos, c->d_line_start, N,
+				d_phase + 6 * (size_t)d0, ld, c->bX, c->bY, c->bZ, d_part, c->rpp, c->lat_stride);
+			ADDA_LAUNCHED();
+		}
+		else {
+			fld_tables<<<dim3((nd + 255) / 256, (unsigned)rows), 256, 0, s>>>(dd, nd, ld, c->bX, c->bY, c->bZ, kd, kl, d_tab);
+			ADDA_LAUNCHED();
+			fld_sum<<<dim3(groups, (unsigned)slices, R), 32, 0, s>>>(d_p, c->d_pos, c->d_xy, c->d_line_start, N, d_tab, d_max, nd,
+				ld, c->bX, c->bY, c->bZ, span, d_part, c->rpp, c->lat_stride);
+			ADDA_LAUNCHED();
+		}
+		fld_finish<<<dim3((nd + FLD_FIN_D - 1) / FLD_FIN_D, R), 32 * FLD_FIN_D, 0, s>>>(d_part, (int)slices, nd, ld, R, dd, c->k, kd,
+			kl, few ? 1 : c->bX, few ? 1 : c->bY, few ? 1 : c->bZ, d_out, ndir, d0);
 		ADDA_LAUNCHED();
 	}
 	ADDA_CUDA(cudaMemcpyAsync(ebuff, d_out, sizeof(double2) * 3 * (size_t)ndir * R, cudaMemcpyDeviceToHost, s));

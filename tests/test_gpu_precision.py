@@ -70,17 +70,19 @@ def full_box(box, k, dpl=15.0):
     return s
 
 
-def fields_of(s, x, dirs):
-    """the context's fields for x handed over as the solution (no iterations), and the polarisations they are of"""
+def fields_of(s, x, dirs, among=4000):
+    """the context's fields for x handed over as the solution (no iterations), among so many directions that they come
+    from the tables (0: these alone), and the polarisations they are of"""
     import torch
-    R = len(x)
+    R, nd = len(x), len(dirs)
+    dirs = np.concatenate([dirs, some_dirs(max(among - nd, 0), 99)])
     c = context(s, R=R)
     d_x = torch.from_numpy(np.ascontiguousarray(x.reshape(R, -1), dtype=np.complex128).view(np.float64)).cuda()
     d_p = torch.empty_like(d_x)
     torch.cuda.synchronize()
     c.solve_device(d_x.data_ptr(), R, d_x.data_ptr(), d_p.data_ptr(), prec="fp64", maxiter=0, init="x0")
     torch.cuda.synchronize()
-    e = c.scattered_fields(dirs, R)
+    e = c.scattered_fields(dirs, R)[:, :nd]
     c.close()
     return e, d_p.cpu().numpy().view(np.complex128).reshape(R, s.n, 3)
 
@@ -108,14 +110,15 @@ def some_dirs(n, seed):
     return d / np.linalg.norm(d, axis=1, keepdims=True)
 
 
+@pytest.mark.parametrize("among", [0, 4000])
 @pytest.mark.parametrize("k", [2 * math.pi, 2 * math.pi / 0.6328, 0.7, 9.3e6])
 @pytest.mark.parametrize("box", [(300, 2, 3), (3, 300, 2), (2, 3, 300)])
-def test_fields_with_any_wave_number(box, k):
+def test_fields_with_any_wave_number(box, k, among):
     """k times the spacing is not a double: every factor of the phase, and the box centre's, takes the same value of it"""
     s = full_box(box, k)
     x = random_vec(s.n, 2, 7)
     dirs = np.concatenate([some_dirs(40, 3), [[0.8, 0.6, 0], [0.6, 0, 0.8]]])
-    e, P = fields_of(s, x, dirs)
+    e, P = fields_of(s, x, dirs, among)
     err = field_errors(e, fields_direct(s, P, dirs))
     assert np.sqrt((err ** 2).mean()) < FIELD_TOL
 
@@ -146,3 +149,53 @@ def test_fields_along_a_dominant_component(scale):
     want = fields_direct(s, P, dirs)
     n = lambda v: np.sqrt((np.abs(v).astype(LD) ** 2).sum((0, 2)))  # per direction, over the right-hand sides
     assert (n(e - want) / n(want)).max() < FIELD_TOL
+
+
+@pytest.mark.parametrize("shape,R,dirs", [((10, 9, 8), 1, (1, 2, 31, 33, 340, 360)), ((40, 30, 25), 2, (1, 2, 5, 6, 7)),
+                                          ((1, 1, 1), 3, (1, 40))])
+def test_fields_of_few_directions(shape, R, dirs):
+    """both sides of the line between a sincos per dipole and the tables; one direction is two kernels"""
+    import adda_gb300 as A
+    s = full_box(shape, 2 * math.pi)
+    x = random_vec(s.n, R, 3)
+    d = some_dirs(max(dirs), 9)
+    pick = sorted({0, 1, 4, 5, 6, 30, 32, 39, 339, 359} & set(range(max(dirs))))
+    for n in dirs:
+        e, P = fields_of(s, x, d[:n], 0)
+        if n == dirs[0]:
+            want = fields_direct(s, P, d[pick])
+        q = [i for i, v in enumerate(pick) if v < n]
+        err = field_errors(e[:, [pick[i] for i in q]], want[:, q])
+        assert np.sqrt((err ** 2).mean()) < FIELD_TOL
+    # launches of the call alone
+    c = context(s, R=R)
+    import torch
+    d_x = torch.from_numpy(x.view(np.float64)).cuda()
+    torch.cuda.synchronize()
+    c.solve_device(d_x.data_ptr(), R, d_x.data_ptr(), prec="fp64", maxiter=0, init="x0")
+    before = A.kernel_launches()
+    c.scattered_fields(d[:1], R)
+    assert A.kernel_launches() - before == 2
+    c.close()
+
+
+def test_fields_of_few_directions_in_a_group():
+    """every particle of a group context sums its own dipoles"""
+    import torch
+
+    import adda_gb300 as A
+    ss = [A.Setup(grid=g, shape="ellipsoid", pars=(0.8, 0.6), m=1.4 + 0.05j, dpl=12) for g in (12, 8)]
+    c = A.Context.group(ss, rhs_per_particle=2)
+    x = np.zeros((4, 3 * c.n), complex)
+    for r in range(4):
+        c.set_cc(r, np.ones((1, 3)))
+        x[r] = c.group_pad(random_vec(ss[r // 2].n, 1, r)[0], r // 2).reshape(-1)
+    c.init_dmatrix()
+    d_x = torch.from_numpy(x.view(np.float64)).cuda()
+    torch.cuda.synchronize()
+    c.solve_device(d_x.data_ptr(), 4, d_x.data_ptr(), prec="fp64", maxiter=0, init="x0")
+    d = some_dirs(2, 4)
+    e = c.scattered_fields(d, 4)
+    many = c.scattered_fields(np.concatenate([d, some_dirs(2000, 5)]), 4)[:, :2]
+    assert field_errors(e, many.astype(CLD)).max() < 2 * FIELD_TOL
+    c.close()
