@@ -46,7 +46,8 @@ struct SolverWork {
 	double *hist = nullptr;
 	int hist_cap = 0;
 	double *vpart = nullptr; // vector-kernel partials [R][nbv][4]
-	int nbv = 0;
+	int nbv = 0;             // blocks per RHS of a solve's vector kernels
+	int nbc = 0;             // ... and of the cross sections, whatever was solved before
 	double *xpart = nullptr; // cross-section partials
 	int *h_done = nullptr;   // pinned
 	// iteration checkpoints: the state of the last FP64 solve (valid until the next solve) and loaded states
@@ -1328,7 +1329,10 @@ static int ensure_work(adda_gb300_ctx *c, int R, int hist_cap)
 		ADDA_CUDA(cudaMallocHost(&w->h_done, sizeof(int) * Rm));
 		w->nbv = (int)std::max<size_t>(1, std::min<size_t>(152 * 4, (n3 + NT - 1) / NT)); // the most of vector_blocks
 		ADDA_CUDA(cudaMalloc(&w->vpart, sizeof(double) * Rm * w->nbv * 4));
-		ADDA_CUDA(cudaMalloc(&w->xpart, sizeof(double) * Rm * w->nbv * 8));
+		// the cross sections' partial sums have blocks of their own (four elements a thread): the same polarisations give the
+		// same digits after a solve of any precision
+		w->nbc = (int)std::max<size_t>(1, std::min<size_t>(152 * 8, (n3 + 4 * NT - 1) / (4 * NT)));
+		ADDA_CUDA(cudaMalloc(&w->xpart, sizeof(double) * Rm * std::max(w->nbv, w->nbc) * 8));
 		if (!c->pvec64) ADDA_CUDA(cudaMalloc(&c->pvec64, vb));
 		if (c->P > 1) {
 			// group contexts: the vectors of a smaller particle are padded to the largest particle's length; the gather
@@ -2376,20 +2380,20 @@ int cross_sections(adda_gb300_ctx *c, int R, const double *prop, const double *i
 		d_prop = tmp;
 	}
 	ADDA_CUDA(cudaMemcpyAsync(d_prop, prop, sizeof(double) * 3 * R, cudaMemcpyHostToDevice, s));
-	const dim3 g(w->nbv, R);
+	const dim3 g(w->nbc, R);
 	const double kd = c->k * c->gridspace, k3 = c->k * c->k * c->k;
 	k_cross<<<g, NT, 0, s>>>(c->pvec64, c->d_pos, c->cc64, c->per_dip, c->nmat, c->d_mat, c->N, d_prop, kd, k3,
-		w->xpart, w->nbv, c->rpp, c->lat_stride);
+		w->xpart, w->nbc, c->rpp, c->lat_stride);
 	ADDA_LAUNCHED();
-	std::vector<double> part((size_t)R * w->nbv * 8);
+	std::vector<double> part((size_t)R * w->nbc * 8);
 	ADDA_CUDA(cudaMemcpyAsync(part.data(), w->xpart, sizeof(double) * part.size(), cudaMemcpyDeviceToHost, s));
 	ADDA_CUDA(cudaStreamSynchronize(s));
 	if (tmp) cudaFree(tmp);
 	const double PI = 3.14159265358979323846;
 	for (int r = 0; r < R; r++) {
 		double sm[7] = {0, 0, 0, 0, 0, 0, 0};
-		for (int b = 0; b < w->nbv; b++)
-			for (int j = 0; j < 7; j++) sm[j] += part[((size_t)r * w->nbv + b) * 8 + j];
+		for (int b = 0; b < w->nbc; b++)
+			for (int j = 0; j < 7; j++) sm[j] += part[((size_t)r * w->nbc + b) * 8 + j];
 		const double *n = prop + 3 * r, *e = incpol + 3 * r;
 		// tbuff = sum - n (n.sum); ebuff = -i k^3 exp(-i k r0.n) tbuff; Cext = 4pi/k^2 Re(ebuff.e)
 		double dre = 0, dim = 0;
@@ -2424,11 +2428,11 @@ int cross_sections_beam(adda_gb300_ctx *c, int R, const double *einc, double inc
 	const size_t n = (size_t)R * c->N * 3;
 	ADDA_CUDA(cudaMalloc(&d_e, sizeof(double2) * std::max<size_t>(n, 1)));
 	cudaError_t e = cudaMemcpyAsync(d_e, einc, sizeof(double2) * n, cudaMemcpyHostToDevice, s);
-	std::vector<double> part((size_t)R * w->nbv * 8);
+	std::vector<double> part((size_t)R * w->nbc * 8);
 	if (e == cudaSuccess) {
-		const dim3 g(w->nbv, R);
+		const dim3 g(w->nbc, R);
 		k_cross_beam<<<g, NT, 0, s>>>(c->pvec64, d_e, c->cc64, c->per_dip, c->nmat, c->d_mat, c->N,
-			c->k * c->k * c->k, w->xpart, w->nbv, c->rpp, c->lat_stride);
+			c->k * c->k * c->k, w->xpart, w->nbc, c->rpp, c->lat_stride);
 		count_launch();
 		e = cudaGetLastError();
 	}
@@ -2443,9 +2447,9 @@ int cross_sections_beam(adda_gb300_ctx *c, int R, const double *einc, double inc
 	const double PI = 3.14159265358979323846;
 	for (int r = 0; r < R; r++) {
 		double s0 = 0, s1 = 0;
-		for (int b = 0; b < w->nbv; b++) {
-			s0 += part[((size_t)r * w->nbv + b) * 8];
-			s1 += part[((size_t)r * w->nbv + b) * 8 + 1];
+		for (int b = 0; b < w->nbc; b++) {
+			s0 += part[((size_t)r * w->nbc + b) * 8];
+			s1 += part[((size_t)r * w->nbc + b) * 8 + 1];
 		}
 		if (cext) cext[r] = s0 * 4 * PI * c->k * inc_scale;
 		if (cabs) cabs[r] = 4 * PI * c->k * s1 * inc_scale;

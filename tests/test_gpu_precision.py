@@ -199,3 +199,25 @@ def test_fields_of_few_directions_in_a_group():
     many = c.scattered_fields(np.concatenate([d, some_dirs(2000, 5)]), 4)[:, :2]
     assert field_errors(e, many.astype(CLD)).max() < 2 * FIELD_TOL
     c.close()
+
+
+# ---------------------------------------------------------------------------------------------------------------------
+def test_cross_sections_do_not_depend_on_the_solve_before():
+    """the same polarisations give the same digits after an FP64 and after a mixed-precision solve"""
+    import torch
+
+    import adda_gb300 as A
+    s = A.Setup(grid=24, m=1.4 + 0.02j, dpl=12)
+    c = context(s, R=2)
+    prop, pol, e = np.stack([s.prop] * 2), np.stack(s.incpol), np.stack(s.einc)
+    for prec in ("mixed", "mixed_f32vec"):
+        res = c.solve(e, prec=prec, eps=1e-3)
+        got = [c.cross_sections(prop, pol), c.cross_sections_beam(e)]
+        d_x = torch.from_numpy(res["x"].view(np.float64)).cuda()
+        d_p = torch.empty_like(d_x)
+        torch.cuda.synchronize()
+        c.solve_device(d_x.data_ptr(), 2, d_x.data_ptr(), d_p.data_ptr(), prec="fp64", maxiter=0, init="x0")
+        torch.cuda.synchronize()
+        assert np.array_equal(d_p.cpu().numpy().view(np.complex128).reshape(2, -1), res["p"])
+        assert np.array_equal(np.array([c.cross_sections(prop, pol), c.cross_sections_beam(e)]), np.array(got))
+    c.close()
