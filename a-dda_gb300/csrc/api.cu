@@ -347,10 +347,9 @@ static int create_impl(const adda_gb300_problem *p, adda_gb300_ctx *c, const std
 	}
 	// interaction matrix
 	const size_t dlen = (size_t)c->gX * c->DsZ * c->DsY * 6;
-	ADDA_CUDA(cudaMalloc(&c->D64, sizeof(double2) * dlen));
+	ADDA_CUDA(cudaMalloc(c->fx ? &c->Dfx : &c->D64, sizeof(double2) * dlen));
 	ADDA_CUDA(cudaMalloc(&c->D32, sizeof(float2) * rows_len((size_t)c->gX * c->DsZ, c->gY, c->DsY)));
 	if (c->fx) {
-		ADDA_CUDA(cudaMalloc(&c->Dfx, sizeof(int4) * dlen));
 		// every top below every exponent (each byte 0x80: far below FX_LOW), as each matvec leaves them
 		const size_t ne = fx_exps_ints(c);
 		ADDA_CUDA(cudaMalloc(&c->fx_exps, sizeof(int) * (ne + (size_t)c->gX * (c->DsZ + (c->surface ? c->gZ : 0)))));
@@ -359,9 +358,8 @@ static int create_impl(const adda_gb300_problem *p, adda_gb300_ctx *c, const std
 	}
 	if (c->surface) {
 		const size_t rlen = (size_t)c->gX * c->gZ * (c->gY / 2 + 1) * 6;
-		ADDA_CUDA(cudaMalloc(&c->R64, sizeof(double2) * rlen));
+		ADDA_CUDA(cudaMalloc(c->fx ? &c->Rfx : &c->R64, sizeof(double2) * rlen));
 		ADDA_CUDA(cudaMalloc(&c->R32, sizeof(float2) * rows_len((size_t)c->gX * c->gZ, c->gY, c->gY / 2 + 1)));
-		if (c->fx) ADDA_CUDA(cudaMalloc(&c->Rfx, sizeof(int4) * rlen));
 	}
 	// matvec work: Xf for Rmax RHS in FP64; the z-chunk buffer is sized to ~48 MB so that it stays in L2
 	const size_t R = c->Rmax;
@@ -607,6 +605,7 @@ int adda_gb300_set_fft_shape(adda_gb300_ctx *c, int prec, const int shape[4])
 		set_error("set_fft_shape: invalid arguments");
 		return ADDA_GB300_EINVAL;
 	}
+	ADDA_CUDA(cudaSetDevice(c->device));
 	const bool f32 = prec == ADDA_PREC_FP32;
 	int rc = matvec_set_shape(c, f32, MvShape{shape[0], shape[1], shape[2], f32 ? shape[3] : 128});
 	if (!rc && f32) c->shape_fixed = true;
@@ -633,8 +632,7 @@ int adda_gb300_get_dmatrix(adda_gb300_ctx *c, double *out)
 		return ADDA_GB300_ESTATE;
 	}
 	ADDA_CUDA(cudaSetDevice(c->device));
-	ADDA_CUDA(cudaMemcpy(out, c->D64, sizeof(double2) * adda_gb300_dmatrix_len(c), cudaMemcpyDeviceToHost));
-	return ADDA_GB300_OK;
+	return dmatrix_get(c, false, out);
 }
 
 size_t adda_gb300_rmatrix_len(const adda_gb300_ctx *c)
@@ -650,8 +648,7 @@ int adda_gb300_get_rmatrix(adda_gb300_ctx *c, double *out)
 		return ADDA_GB300_ESTATE;
 	}
 	ADDA_CUDA(cudaSetDevice(c->device));
-	ADDA_CUDA(cudaMemcpy(out, c->R64, sizeof(double2) * adda_gb300_rmatrix_len(c), cudaMemcpyDeviceToHost));
-	return ADDA_GB300_OK;
+	return dmatrix_get(c, true, out);
 }
 
 __global__ void cc_sqrt_k(const double2 *cc, double2 *ccs64, float2 *ccs32, size_t n)

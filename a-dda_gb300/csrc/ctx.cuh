@@ -134,8 +134,9 @@ struct adda_gb300_ctx {
 	int4 *tw2x[4] = {nullptr, nullptr, nullptr, nullptr};
 	// FP64 matvec in 64-bit fixed point: all three axes have two-pass plans
 	bool fx = false;
-	void *Dfx = nullptr;    // D in fixed point, [gX][DsZ][DsY][6]
-	void *Rfx = nullptr;    // R in fixed point, [gX][gZ][gY/2+1][6]
+	// D [gX][DsZ][DsY][6] and R [gX][gZ][gY/2+1][6] in fixed point (int4 entries, as large as FP64 ones): in the place of
+	// D64 and R64, which are null unless a set tile shape has selected the FP64 transforms (dmatrix_build)
+	double2 *Dfx = nullptr, *Rfx = nullptr;
 	int *fx_exps = nullptr; // exponents of the data between the kernels (matvec_lines2.cuh: FxExp)
 	int *fx_eD = nullptr;   // exponents of Dfx's rows [gX][DsZ], then of Rfx's [gX][gZ] (behind them)
 	void *tables = nullptr; // the allocation behind the twiddle tables
@@ -191,12 +192,15 @@ Plan2 make_plan2(int n, bool fx);
 
 // dmatrix.cu
 int dmatrix_build(adda_gb300_ctx *c);
+int dmatrix_forms(adda_gb300_ctx *c);
+int dmatrix_get(adda_gb300_ctx *c, bool reflected, double *out);
 
 // matvec_lines2.cu
 size_t fx_exps_ints(const adda_gb300_ctx *c); // ints of fx_exps
-int fx_dmatrix(adda_gb300_ctx *c);            // D64, R64 -> Dfx, Rfx, fx_eD
+int fx_dmatrix(adda_gb300_ctx *c, const double2 *D, const double2 *R); // D, R (each if given) -> Dfx, Rfx, fx_eD
 
 // matvec.cu
+bool matvec_fixed(const adda_gb300_ctx *c); // FP64 matvecs run in fixed point
 int matvec_setup(adda_gb300_ctx *c); // tile shapes, kernel attributes
 int matvec_set_shape(adda_gb300_ctx *c, bool f32, const MvShape &s); // a tile shape the build holds and that fits
 bool matvec_shape_ok(const adda_gb300_ctx *c, bool f32, const MvShape &s);

@@ -530,7 +530,8 @@ int fft_lines_run(adda_gb300_ctx *c, double2 *data, const FftPlan &p, const doub
 	return ADDA_GB300_OK;
 }
 
-int rmatrix_build(adda_gb300_ctx *c)
+// D or R in FP64 into its buffer, and (narrow) its FP32 copy
+int rmatrix_build(adda_gb300_ctx *c, double2 *R64, bool narrow)
 {
 	const int bX = c->bX, bY = c->bY, bZ = c->bZ, gX = c->gX, gY = c->gY, gZ = c->gZ;
 	const int nk = 2 * bZ - 1, RsY = gY / 2 + 1;
@@ -572,13 +573,15 @@ int rmatrix_build(adda_gb300_ctx *c)
 			if (cudaGetLastError() != cudaSuccess) { rc = ADDA_GB300_ECUDA; break; }
 			if ((rc = fft_lines_run(c, S, c->pz[0], c->tw64[2], false, 1, gZ, gX * gY, 0, 1))) break;
 			if ((rc = fft_lines_run(c, S, c->py[0], c->tw64[1], false, gZ, 1, gZ, (size_t)gY * gZ, gX))) break;
-			r_extract<<<grid_for((size_t)gX * gZ * RsY), 256, 0, c->stream>>>(c->R64, S, a, gX, gY, gZ, RsY, invN);
+			r_extract<<<grid_for((size_t)gX * gZ * RsY), 256, 0, c->stream>>>(R64, S, a, gX, gY, gZ, RsY, invN);
 			count_launch();
 			if (cudaGetLastError() != cudaSuccess) { rc = ADDA_GB300_ECUDA; break; }
 		}
 		if (rc) break;
-		to_f32<<<grid_for(rlen), 256, 0, c->stream>>>(c->R32, c->R64, (size_t)gX * gZ, RsY, planar_rows(gY));
-		count_launch();
+		if (narrow) {
+			to_f32<<<grid_for(rlen), 256, 0, c->stream>>>(c->R32, R64, (size_t)gX * gZ, RsY, planar_rows(gY));
+			count_launch();
+		}
 		if (cudaGetLastError() != cudaSuccess) { rc = ADDA_GB300_ECUDA; break; }
 		if (cudaStreamSynchronize(c->stream) != cudaSuccess) { rc = ADDA_GB300_ECUDA; break; }
 	} while (0);
@@ -589,9 +592,7 @@ int rmatrix_build(adda_gb300_ctx *c)
 	return rc;
 }
 
-} // namespace
-
-int dmatrix_build(adda_gb300_ctx *c)
+int tensor_build(adda_gb300_ctx *c, double2 *D64, bool narrow)
 {
 	const int bX = c->bX, bY = c->bY, bZ = c->bZ, gX = c->gX, gY = c->gY, gZ = c->gZ;
 	const size_t lines = (size_t)bZ * bY;
@@ -653,14 +654,16 @@ int dmatrix_build(adda_gb300_ctx *c)
 			if ((rc = fft_lines_run(c, S, c->pz[0], c->tw64[2], false, 1, gZ, gX * gY, 0, 1))) break;
 			// y transform: element stride gZ, lines z adjacent, outer x
 			if ((rc = fft_lines_run(c, S, c->py[0], c->tw64[1], false, gZ, 1, gZ, (size_t)gY * gZ, gX))) break;
-			d_extract<<<grid_for((size_t)gX * c->DsZ * c->DsY), 256, 0, c->stream>>>(c->D64, S, a, gX, gY, gZ,
+			d_extract<<<grid_for((size_t)gX * c->DsZ * c->DsY), 256, 0, c->stream>>>(D64, S, a, gX, gY, gZ,
 				c->DsY, c->DsZ, invN);
 			count_launch();
 			if (cudaGetLastError() != cudaSuccess) { rc = ADDA_GB300_ECUDA; break; }
 		}
 		if (rc) break;
-		to_f32<<<grid_for(dlen), 256, 0, c->stream>>>(c->D32, c->D64, (size_t)gX * c->DsZ, c->DsY, planar_rows(c->gY));
-		count_launch();
+		if (narrow) {
+			to_f32<<<grid_for(dlen), 256, 0, c->stream>>>(c->D32, D64, (size_t)gX * c->DsZ, c->DsY, planar_rows(c->gY));
+			count_launch();
+		}
 		if (cudaGetLastError() != cudaSuccess) { rc = ADDA_GB300_ECUDA; break; }
 		if (cudaStreamSynchronize(c->stream) != cudaSuccess) { rc = ADDA_GB300_ECUDA; break; }
 	} while (0);
@@ -669,10 +672,88 @@ int dmatrix_build(adda_gb300_ctx *c)
 	cudaFree(S);
 	cudaFree(d_tabs);
 	cudaFree(d_index);
-	if (!rc && c->surface) rc = rmatrix_build(c);
-	if (!rc && c->fx) rc = fx_dmatrix(c);
+	return rc;
+}
+
+} // namespace
+
+// The FP64 interaction matrices of a context with a fixed-point matvec stand in one buffer, built in FP64 and turned into
+// fixed point where they stand (both take 16 bytes an entry). A tile shape that selects the FP64 transforms gets the FP64
+// form in a buffer of its own (dmatrix_forms).
+int dmatrix_build(adda_gb300_ctx *c)
+{
+	const bool fx = matvec_fixed(c);
+	// the buffer goes to the form in use
+	if (!fx && !c->D64) {
+		std::swap(c->D64, c->Dfx);
+		std::swap(c->R64, c->Rfx);
+	}
+	if (fx && !c->Dfx) {
+		std::swap(c->D64, c->Dfx);
+		std::swap(c->R64, c->Rfx);
+	}
+	double2 *D = c->D64 ? c->D64 : c->Dfx, *R = c->R64 ? c->R64 : c->Rfx;
+	int rc = tensor_build(c, D, true);
+	if (!rc && c->surface) rc = rmatrix_build(c, R, true);
+	if (!rc && c->Dfx) rc = fx_dmatrix(c, D, R);
 	if (!rc) c->dready = true;
 	return rc;
+}
+
+// the form that the present tile shape reads, where it is missing
+int dmatrix_forms(adda_gb300_ctx *c)
+{
+	const bool fx = matvec_fixed(c);
+	if (!c->dready || (fx ? c->Dfx : c->D64)) return ADDA_GB300_OK;
+	const size_t dlen = (size_t)c->gX * c->DsZ * c->DsY * 6, rlen = c->surface ? (size_t)c->gX * c->gZ * (c->gY / 2 + 1) * 6 : 0;
+	double2 *D = nullptr, *R = nullptr;
+	int rc = ADDA_GB300_OK;
+	if (cudaMalloc(&D, sizeof(double2) * dlen) != cudaSuccess || (rlen && cudaMalloc(&R, sizeof(double2) * rlen) != cudaSuccess)) {
+		cudaGetLastError();
+		set_error("cannot allocate the other form of the interaction matrix");
+		rc = ADDA_GB300_ENOMEM;
+	}
+	if (!rc) {
+		if (fx) {
+			c->Dfx = D;
+			c->Rfx = R;
+			rc = fx_dmatrix(c, c->D64, c->R64);
+		}
+		else {
+			c->D64 = D;
+			c->R64 = R;
+			rc = tensor_build(c, D, false);
+			if (!rc && R) rc = rmatrix_build(c, R, false);
+		}
+		if (rc) {
+			(fx ? c->Dfx : c->D64) = nullptr;
+			(fx ? c->Rfx : c->R64) = nullptr;
+		}
+	}
+	if (rc) {
+		cudaFree(D);
+		cudaFree(R);
+	}
+	return rc;
+}
+
+// the FP64 D (or R, reflected) to the host; where only the fixed-point form stands, rebuilt in its place meanwhile
+int dmatrix_get(adda_gb300_ctx *c, bool reflected, double *out)
+{
+	const size_t n = reflected ? (size_t)c->gX * c->gZ * (c->gY / 2 + 1) * 6 : (size_t)c->gX * c->DsZ * c->DsY * 6;
+	double2 *m = reflected ? c->R64 : c->D64;
+	const bool rebuild = !m;
+	int rc = ADDA_GB300_OK;
+	if (rebuild) {
+		m = reflected ? c->Rfx : c->Dfx;
+		if ((rc = reflected ? rmatrix_build(c, m, false) : tensor_build(c, m, false))) {
+			cudaGetLastError(); // no memory for the build: the matrix still stands in fixed point
+			return rc;
+		}
+	}
+	ADDA_CUDA(cudaMemcpyAsync(out, m, sizeof(double2) * n, cudaMemcpyDeviceToHost, c->stream));
+	ADDA_CUDA(cudaStreamSynchronize(c->stream));
+	return rebuild ? fx_dmatrix(c, reflected ? nullptr : m, reflected ? m : nullptr) : rc;
 }
 
 } // namespace adda

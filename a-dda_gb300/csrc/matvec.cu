@@ -43,6 +43,11 @@ template <typename T> static bool choose_shape(adda_gb300_ctx *c, MvShape &s)
 	return mv::shape_fits<T>(c, s);
 }
 
+bool matvec_fixed(const adda_gb300_ctx *c)
+{
+	return mv::use_fx(c);
+}
+
 int matvec_setup(adda_gb300_ctx *c)
 {
 	if (!choose_shape<double>(c, c->shape[0]) || !choose_shape<float>(c, c->shape[1])) {
@@ -72,8 +77,11 @@ int matvec_set_shape(adda_gb300_ctx *c, bool f32, const MvShape &s)
 		set_error("set_fft_shape: this tile shape is not built for these axis lengths or does not fit shared memory");
 		return ADDA_GB300_EINVAL;
 	}
+	const MvShape old = c->shape[f32 ? 1 : 0];
 	c->shape[f32 ? 1 : 0] = s;
-	return ADDA_GB300_OK;
+	const int rc = f32 ? ADDA_GB300_OK : dmatrix_forms(c);
+	if (rc) c->shape[0] = old;
+	return rc;
 }
 
 template <typename T, typename V>

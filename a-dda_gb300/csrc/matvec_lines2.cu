@@ -14,7 +14,8 @@ size_t fx_exps_ints(const adda_gb300_ctx *c)
 
 namespace mv {
 
-// one row (kx, kz) of D per block: the row's largest exponent, then every component scaled to |v| < 2^60 and split
+// one row (kx, kz) of D per block: the row's largest exponent, then every component scaled to |v| < 2^60 and split. Dfx may
+// be D's own memory: a thread reads an entry before it writes that entry, all of them after the row's largest is known
 __global__ void __launch_bounds__(128) fx_drow(const double2 *D, int4 *Dfx, int *eD, int n)
 {
 	__shared__ int smax;
@@ -77,13 +78,14 @@ int fx_yz_run(adda_gb300_ctx *c, const MvGeom<double> &p, int ck, cudaStream_t s
 
 } // namespace mv
 
-int fx_dmatrix(adda_gb300_ctx *c)
+int fx_dmatrix(adda_gb300_ctx *c, const double2 *D, const double2 *R)
 {
-	mv::fx_drow<<<c->gX * c->DsZ, 128, 0, c->stream>>>(c->D64, (int4 *)c->Dfx, c->fx_eD, c->DsY * 6);
-	ADDA_LAUNCHED();
-	if (c->surface) {
-		mv::fx_drow<<<c->gX * c->gZ, 128, 0, c->stream>>>(c->R64, (int4 *)c->Rfx, c->fx_eD + (size_t)c->gX * c->DsZ,
-			(c->gY / 2 + 1) * 6);
+	if (D) {
+		mv::fx_drow<<<c->gX * c->DsZ, 128, 0, c->stream>>>(D, (int4 *)c->Dfx, c->fx_eD, c->DsY * 6);
+		ADDA_LAUNCHED();
+	}
+	if (R) {
+		mv::fx_drow<<<c->gX * c->gZ, 128, 0, c->stream>>>(R, (int4 *)c->Rfx, c->fx_eD + (size_t)c->gX * c->DsZ, (c->gY / 2 + 1) * 6);
 		ADDA_LAUNCHED();
 	}
 	ADDA_CUDA(cudaStreamSynchronize(c->stream));

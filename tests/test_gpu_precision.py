@@ -221,3 +221,71 @@ def test_cross_sections_do_not_depend_on_the_solve_before():
         assert np.array_equal(d_p.cpu().numpy().view(np.complex128).reshape(2, -1), res["p"])
         assert np.array_equal(np.array([c.cross_sections(prop, pol), c.cross_sections_beam(e)]), np.array(got))
     c.close()
+
+
+@pytest.mark.parametrize("surface", [False, True])
+def test_one_copy_of_the_interaction_matrix(surface):
+    """a context holds the FP64 matrix in one form: 16 + 8 bytes an entry, and the matvec's and vectors' buffers"""
+    import torch
+
+    import adda_gb300 as A
+    s = full_box((3, 126, 126), 1.0)
+    s.grid = (300, 252, 252) if not surface else (150, 252, 252)
+    kw = dict(surface=dict(zsum_shift=1.25, msub=1.5 + 0.1j, relation="img")) if surface else {}
+    A.Context((2, 2, 2), full_box((2, 2, 2), 1.0).pos, None, 0.4, 1.0, (4, 4, 4)).close()
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    c = A.Context(s.box, s.pos, s.mat, s.gridspace, 1.0, s.grid, nrhs_max=1, **kw)
+    c.init_dmatrix()
+    torch.cuda.synchronize()
+    used = free - torch.cuda.mem_get_info()[0]
+    g, b = s.grid, s.box
+    entries = 6 * g[0] * (g[1] // 2 + 1) * (g[2] // 2 + 1) + (6 * g[0] * (g[1] // 2 + 1) * g[2] if surface else 0)
+    slab = 3 * g[2] * b[1]
+    chunk = (4 if surface else 2) * max(48 << 20, 8 * slab * g[0])
+    work = 16 * 3 * g[0] * b[1] * b[2] + chunk + 2 * 16 * 3 * s.n
+    assert 24 * entries > 4 * (64 << 20) and used < 24 * entries * 1.02 + work + (64 << 20)
+    c.close()
+
+
+@pytest.mark.parametrize("surface", [False, True])
+def test_forms_of_the_interaction_matrix(surface):
+    """reading the matrix back, and tile shapes that take the FP64 transforms and back, before and after it is built, leave
+    the matrix and the matvec as they are"""
+    import adda_gb300 as A
+    s = full_box((10, 7, 6), 1.0)
+    kw = dict(surface=dict(zsum_shift=1.25, msub=1.5 + 0.1j, relation="img")) if surface else {}
+
+    def make(shape=None):
+        c = A.Context(s.box, s.pos, s.mat, s.gridspace, 1.0, s.grid, nrhs_max=2, **kw)
+        if shape:
+            c.set_fft_shape(shape, "fp64")
+        c.init_dmatrix()
+        for r in range(2):
+            c.set_cc(r, s.cc[r].reshape(1, 3))
+        return c
+
+    x = random_vec(s.n, 2, 1)
+    c = make()
+    plain, narrow = list(c.fft_shape("fp64")), [1] + list(c.fft_shape("fp64"))[1:]
+    y = c.matvec(x, "fp64")[0]
+    d, r = c.dmatrix(), c.rmatrix() if surface else None
+    assert np.array_equal(c.matvec(x, "fp64")[0], y) and np.array_equal(c.dmatrix(), d)
+    c.set_fft_shape(narrow, "fp64")
+    y64 = c.matvec(x, "fp64")[0]
+    assert 0 < np.abs(y64 - y).max() < 1e-14 * np.abs(y).max()
+    c.set_fft_shape(plain, "fp64")
+    assert np.array_equal(c.matvec(x, "fp64")[0], y)
+    c.init_dmatrix()
+    assert np.array_equal(c.matvec(x, "fp64")[0], y) and np.array_equal(c.dmatrix(), d)
+    n = make(narrow)
+    assert np.array_equal(n.matvec(x, "fp64")[0], y64) and np.array_equal(n.dmatrix(), d)
+    n.set_fft_shape(plain, "fp64")
+    assert np.array_equal(n.matvec(x, "fp64")[0], y) and np.array_equal(n.dmatrix(), d)
+    if surface:
+        assert np.array_equal(c.rmatrix(), r) and np.array_equal(n.rmatrix(), r)
+    n.set_fft_shape(narrow, "fp64")
+    n.init_dmatrix()
+    assert np.array_equal(n.matvec(x, "fp64")[0], y64)
+    c.close()
+    n.close()
