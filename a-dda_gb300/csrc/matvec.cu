@@ -48,6 +48,21 @@ bool matvec_fixed(const adda_gb300_ctx *c)
 	return mv::use_fx(c);
 }
 
+// shared-memory opt-in (which also loads them) of the FP64 kernels that the present tile shape takes: at the context's
+// creation and when a shape is set, not inside a matvec. A process's first FP64 matvec of a 128^3 sphere took 10 ms longer
+// where the fixed-point kernels were left to it, and its first context 20 ms longer with all lengths of the others.
+static int prepare_f64(adda_gb300_ctx *c)
+{
+	int rc;
+	if (!mv::use_fx(c)) {
+		rc = mv::set_attrs_tv<double, double2>(c);
+		return rc ? rc : mv::setup_yz<double>(c);
+	}
+	const mv::MvP<double, double2> p{}; // no RHS
+	if ((rc = mv::fx_scatter_run(c, p, c->stream)) || (rc = mv::fx_yz_run(c, p, 1, c->stream))) return rc;
+	return mv::fx_gather_run(c, p, MvEpi{}, c->stream);
+}
+
 int matvec_setup(adda_gb300_ctx *c)
 {
 	if (!choose_shape<double>(c, c->shape[0]) || !choose_shape<float>(c, c->shape[1])) {
@@ -55,9 +70,8 @@ int matvec_setup(adda_gb300_ctx *c)
 			: "FFT grid too large for the shared-memory tiles (at most 2048 per axis)");
 		return ADDA_GB300_EINVAL;
 	}
-	int rc = mv::set_attrs_tv<double, double2>();
-	if (rc || (rc = mv::setup_yz<double>()) || (rc = mv::setup_yz<float>())) return rc;
-	return matvec_setup_f32(c);
+	const int rc = prepare_f64(c);
+	return rc ? rc : matvec_setup_f32(c);
 }
 
 bool matvec_shape_ok(const adda_gb300_ctx *c, bool f32, const MvShape &s)
@@ -79,8 +93,9 @@ int matvec_set_shape(adda_gb300_ctx *c, bool f32, const MvShape &s)
 	}
 	const MvShape old = c->shape[f32 ? 1 : 0];
 	c->shape[f32 ? 1 : 0] = s;
-	const int rc = f32 ? ADDA_GB300_OK : dmatrix_forms(c);
-	if (rc) c->shape[0] = old;
+	int rc = f32 ? ADDA_GB300_OK : prepare_f64(c);
+	if (!rc && !f32) rc = dmatrix_forms(c);
+	if (rc) c->shape[f32] = old;
 	return rc;
 }
 

@@ -827,22 +827,20 @@ template <typename T, int NS> int set_attrs_yz()
 }
 #undef ADDA_SET
 
-template <typename T, typename V> int set_attrs_tv()
+// ... of those that a context's axes take, in all widths
+template <typename T, typename V> int set_attrs_tv(const adda_gb300_ctx *c)
 {
-	int rc;
-	if ((rc = set_attrs_k13<T, V, 0>()) || (rc = set_attrs_k13<T, V, 64>()) || (rc = set_attrs_k13<T, V, 128>()) ||
-		(rc = set_attrs_k13<T, V, 256>()) || (rc = set_attrs_k13<T, V, 512>()))
-		return rc;
-	return ADDA_GB300_OK;
+	int rc = ADDA_GB300_OK;
+	ADDA_NS_SWITCH(c->gX, (rc = set_attrs_k13<T, V, NS>()));
+	return rc;
 }
 
-template <typename T> int setup_yz()
+template <typename T> int setup_yz(const adda_gb300_ctx *c)
 {
-	int rc;
-	if ((rc = set_attrs_yz<T, 0>()) || (rc = set_attrs_yz<T, 64>()) || (rc = set_attrs_yz<T, 128>()) ||
-		(rc = set_attrs_yz<T, 256>()) || (rc = set_attrs_yz<T, 512>()))
-		return rc;
-	return ADDA_GB300_OK;
+	int rc = ADDA_GB300_OK;
+	ADDA_NS_SWITCH(c->gZ, (rc = set_attrs_yz<T, NS>()));
+	if (!rc && static_len(c->gY) != static_len(c->gZ)) ADDA_NS_SWITCH(c->gY, (rc = set_attrs_yz<T, NS>()));
+	return rc;
 }
 
 // the stages on two-pass transforms (matvec_lines2.cuh, compiled in matvec_lines2*.cu; measured there against the
@@ -952,8 +950,8 @@ template <typename T> int launch_yz(adda_gb300_ctx *c, MvGeom<T> p, int ck, cons
 #ifndef ADDA_MATVEC_YZ_TU
 extern template int launch_yz<float>(adda_gb300_ctx *, MvGeom<float>, int, const MvShape &, cudaStream_t);
 extern template int launch_yz<double>(adda_gb300_ctx *, MvGeom<double>, int, const MvShape &, cudaStream_t);
-extern template int setup_yz<float>();
-extern template int setup_yz<double>();
+extern template int setup_yz<float>(const adda_gb300_ctx *);
+extern template int setup_yz<double>(const adda_gb300_ctx *);
 #endif
 
 template <typename T, typename V>

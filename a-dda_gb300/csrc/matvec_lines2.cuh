@@ -674,17 +674,23 @@ template <class A> inline Lines2<A> make_lines2(const adda_gb300_ctx *c)
 	}
 	return q;
 }
-// launch of a kernel; shared memory near the default limit (48 KB with the static part) and above is opted in to, once
-// per kernel and device
-template <auto KERN, typename... Ar>
-inline int l2_launch(const adda_gb300_ctx *c, dim3 g, int nt, size_t sm, cudaStream_t st, const Ar &...args)
+// shared memory up to SMEM_CAP for a kernel (and its code on the device), once per kernel and device
+template <auto KERN> inline int l2_opt_in(const adda_gb300_ctx *c)
 {
 	static std::atomic<unsigned long long> opted{0};
 	const unsigned long long bit = 1ull << (c->device & 63);
-	if (sm > 32 * 1024 && !(opted.load(std::memory_order_acquire) & bit)) {
+	if (!(opted.load(std::memory_order_acquire) & bit)) {
 		ADDA_CUDA(cudaFuncSetAttribute(KERN, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_CAP));
 		opted.fetch_or(bit, std::memory_order_release);
 	}
+	return ADDA_GB300_OK;
+}
+// launch of a kernel; a grid without blocks (no RHS) only opts it in, at the context's creation (matvec_prepare)
+template <auto KERN, typename... Ar>
+inline int l2_launch(const adda_gb300_ctx *c, dim3 g, int nt, size_t sm, cudaStream_t st, const Ar &...args)
+{
+	const int rc = l2_opt_in<KERN>(c);
+	if (rc || !(g.x && g.z)) return rc;
 	launch_next(KERN, g, dim3(nt), sm, st, args...);
 	ADDA_LAUNCHED();
 	return ADDA_GB300_OK;

@@ -9,8 +9,8 @@ namespace mv {
 
 template int launch_yz<float>(adda_gb300_ctx *, MvGeom<float>, int, const MvShape &, cudaStream_t);
 template int launch_yz<double>(adda_gb300_ctx *, MvGeom<double>, int, const MvShape &, cudaStream_t);
-template int setup_yz<float>();
-template int setup_yz<double>();
+template int setup_yz<float>(const adda_gb300_ctx *);
+template int setup_yz<double>(const adda_gb300_ctx *);
 
 } // namespace mv
 } // namespace adda
