@@ -4,8 +4,9 @@
 //
 // GB300 issues an FP64 instruction every 76 cycles per warp scheduler, so FP64 work that every thread or every block
 // repeats costs more than the vectors' traffic on small particles. Hence:
-//   - sums over a warp are taken in 64-bit fixed point relative to the warp's largest value (exact to 2^-57 of it):
-//     50 integer instructions a sum against 5 FP64 additions (380 cycles);
+//   - sums over a warp are taken in 64-bit fixed point relative to the warp's largest value: 32 values rounded to a unit of
+//     2^-57 to 2^-56 of it, so below 2^-52 of it together and as often up as down (5 FP64 additions: 5 * 2^-53 of the sum);
+//     54 integer instructions a sum against 380 cycles;
 //   - a kernel's scalar coefficients are converted to double-float once per block by one warp (Coefs), not by every
 //     thread;
 //   - the scalar steps are not launches of their own: the last block to finish (last_block) sums the partial sums in a
@@ -34,7 +35,8 @@ __device__ __forceinline__ long long sum_fx(double v, int emax)
 {
 	const int hi = __double2hiint(v), ex = (hi >> 20) & 0x7ff, sh = emax - max(ex, 1);
 	long long m = ((long long)((hi & 0xfffff) | (ex ? 0x100000 : 0)) << 32) | (unsigned)__double2loint(v);
-	m = sh > 62 ? 0 : (m << (SUM_TOP - 53)) >> sh;
+	// rounded: cutting off would take up to 31 units off a sum of squares
+	m = sh > 62 ? 0 : (((m << (SUM_TOP - 52)) >> sh) + 1) >> 1;
 	return hi < 0 ? -m : m;
 }
 __device__ __forceinline__ int sum_key(DF v) { return __float_as_int(v.h) & 0x7fffffff; }
@@ -45,6 +47,8 @@ __device__ __forceinline__ long long sum_fx(float v, int emax)
 {
 	const int b = __float_as_int(v), ex = (b >> 23) & 0xff, sh = emax - max(ex, 1);
 	const long long m = (long long)((b & 0x7fffff) | (ex ? 0x800000 : 0)) << (SUM_TOP - 24);
+	// cut off: only below 2^-33 of the warp's largest value, or in a double-float's low part, which has either sign; a
+	// double-float itself ends at 2^-48
 	const long long q = sh > 62 ? 0 : m >> sh;
 	return b < 0 ? -q : q;
 }

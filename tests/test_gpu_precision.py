@@ -15,13 +15,14 @@ TOL = 9e-16
 LD, CLD = np.longdouble, np.clongdouble
 
 
-def matvec_direct(s, cc, x):
-    """x - S G S x by a direct sum over the dipoles in extended precision, [n, 3]"""
+def matvec_direct(s, cc, x, pick=None):
+    """x - S G S x by a direct sum over the dipoles in extended precision, [n, 3] or at the picked dipoles"""
     S = np.sqrt(cc.reshape(-1)[:3].astype(CLD))
     v = x * S
-    pos, out = s.pos.astype(LD), np.empty((s.n, 3), CLD)
+    pick = range(s.n) if pick is None else pick
+    pos, out = s.pos.astype(LD), np.empty((len(pick), 3), CLD)
     kd = LD(s.wavenum) * LD(s.gridspace)
-    for i in range(s.n):
+    for k, i in enumerate(pick):
         d = pos[i] - pos
         d[i] = 1
         r = np.sqrt((d * d).sum(1))
@@ -29,7 +30,7 @@ def matvec_direct(s, cc, x):
         e = np.exp(1j * kr.astype(CLD)) / (LD(s.gridspace) * r) ** 3
         e[i] = 0
         a, b = e * (kr * kr - 1 + 1j * kr), e * (3 - kr * kr - 3j * kr) * (q * v).sum(1)
-        out[i] = x[i] - S * (a[:, None] * v + b[:, None] * q).sum(0)
+        out[k] = x[i] - S * (a[:, None] * v + b[:, None] * q).sum(0)
     return out
 
 
@@ -289,3 +290,23 @@ def test_forms_of_the_interaction_matrix(surface):
     assert np.array_equal(n.matvec(x, "fp64")[0], y64)
     c.close()
     n.close()
+
+
+@pytest.mark.parametrize("box", [(16, 16, 8), (32, 4, 30)])
+def test_block_sums_round(box):
+    """|y|^2 of y = x (polarisabilities of 1e-300) where each warp sums one value of 1 and others 2^-17 of it that end just
+    below the sum's unit of 2^-56. Cut off, they would all be short by one: 31 * 2^-56 = 4.3e-16. Bound: the block's and the
+    total's rounding to a double, 2 * 2^-53"""
+    s = full_box(box, 1.0)
+    s.cc = [np.full(3, 1e-300)] * 2
+    c = context(s, R=1)
+    b = next(v for v in range((1 << 26) + 1, 1 << 27, 2) if v * v < 1 << 53 and v * v % 4096 == 4089)
+    x = np.zeros((1, s.n, 3), complex)
+    x[0, :, 0] = b * 2.0 ** -26 * 2.0 ** -8
+    x[0, ::32, 0] = 1
+    y, ip = c.matvec(x.reshape(1, -1), "fp64")
+    y = y.reshape(x.shape)
+    assert np.array_equal(y[..., 0].real, x[..., 0].real) and max(abs(y.imag).max(), abs(y[..., 1:]).max()) < 1e-200
+    want = math.fsum((x.real ** 2).ravel())
+    assert abs(ip[0] - want) <= 2.3e-16 * want
+    c.close()
