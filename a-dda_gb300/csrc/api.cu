@@ -533,7 +533,7 @@ static int tune_chunks(adda_gb300_ctx *c)
 	};
 	// 1. the tile shape, one dimension at a time over the alternatives the build holds (register-K2b threads per
 	// block or generic-K2b pairs per block, then y-lines per K2a/K2c block, then per K1/K3 block), each kept when
-	// faster; candidates that do not fit the axis lengths are skipped
+	// faster; candidates that do not fit the axis lengths, or launch the same kernels, are skipped
 	if (!c->shape_fixed) {
 		float best = 1e30f;
 		if (!time_mv(best)) goto done;
@@ -545,7 +545,7 @@ static int tune_chunks(adda_gb300_ctx *c)
 				if (field == cand[dim][k] || (dim == 0 && !matvec_k2b_reg(c)) || (dim == 1 && matvec_k2b_reg(c)))
 					continue;
 				field = cand[dim][k];
-				if (!matvec_shape_ok(c, true, sh)) continue;
+				if (!matvec_shape_ok(c, true, sh) || matvec_same_kernels(c, sh, keep)) continue;
 				c->shape[1] = sh;
 				float t = 0;
 				if (!time_mv(t)) goto done;

@@ -200,6 +200,7 @@ size_t fx_exps_ints(const adda_gb300_ctx *c); // ints of fx_exps
 int fx_dmatrix(adda_gb300_ctx *c, const double2 *D, const double2 *R); // D, R (each if given) -> Dfx, Rfx, fx_eD
 
 // matvec.cu
+bool matvec_same_kernels(const adda_gb300_ctx *c, const adda::MvShape &a, const adda::MvShape &b); // two FP32 tile shapes
 bool matvec_fixed(const adda_gb300_ctx *c); // FP64 matvecs run in fixed point
 int matvec_setup(adda_gb300_ctx *c); // tile shapes, kernel attributes
 int matvec_set_shape(adda_gb300_ctx *c, bool f32, const MvShape &s); // a tile shape the build holds and that fits

@@ -5,6 +5,18 @@
 
 namespace adda {
 
+bool matvec_same_kernels(const adda_gb300_ctx *c, const MvShape &a, const MvShape &b)
+{
+	// x and z axes with a radix above 16 have one width; the two-pass y kernel as many columns as its threads allow
+	const bool x = a.w1 == b.w1 || (mv::use_l2_x(c, a) && mv::use_l2_x(c, b) && c->p2[0].big);
+	const bool z = a.w2 == b.w2 || (mv::use_l2_z(c, a) && mv::use_l2_z(c, b) && c->p2[2].big);
+	const auto columns = [&](const MvShape &s) {
+		return mv::l2_columns<Ar32>(c->p2[1], c->surface ? std::max(1, s.pairs / 2) : s.pairs);
+	};
+	const bool y = a.pairs == b.pairs || (mv::use_l2_y(c) && columns(a) == columns(b));
+	return x && y && z && a.nt == b.nt;
+}
+
 size_t fx_exps_ints(const adda_gb300_ctx *c)
 {
 	size_t n;

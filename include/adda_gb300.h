@@ -372,12 +372,16 @@ int adda_gb300_time_matvec(adda_gb300_ctx *ctx, int prec, int nrhs, int iters, s
  * pairs per block of the generic y-FFT + D kernel, [3] threads per block of the register y-FFT + D kernel (FP32).
  * The library picks the defaults, narrows them for axes longer than 512 (up to 2048 per axis), and tunes the FP32
  * shape at the first FP32 matvec or solve of a context together with its L2 chunk (the reference plans its FFTs
- * with FFTW_MEASURE likewise, fft.c:739-815). No counterpart call in the reference: its FFTs are FFTW's. */
+ * with FFTW_MEASURE likewise, fft.c:739-815). No counterpart call in the reference: its FFTs are FFTW's.
+ * FP64: the default [0] and [1] stand for the fixed-point kernels where the axes have plans for them; those have tiles of
+ * their own, whatever [2] says, and any other [0] or [1] takes the FP64 transforms (2 to 4 times slower). FP32: axes with a
+ * radix above 16 have one width, whatever [0] and [1] say. */
 int adda_gb300_get_fft_shape(const adda_gb300_ctx *ctx, int prec, int shape[4]);
 /* x-slabs per chunk of the y/z stage (the L2 chunk; FP32: tuned with the shape), or EINVAL */
 int adda_gb300_get_l2_chunk(const adda_gb300_ctx *ctx, int prec);
 /* set a shape (FP32: the tuner then keeps it; the L2 chunk is still tuned); EINVAL for a shape this build does not
- * hold for the context's axis lengths or one whose shared memory does not fit a block. The environment variable
+ * hold for the context's axis lengths or one whose shared memory does not fit a block; ENOMEM where the first FP64 shape
+ * that takes the FP64 transforms finds no memory for its form of the interaction matrix. The environment variable
  * ADDA_GB300_FFT_SHAPE="w1,w2,pairs,threads" does the same for every FP32 context. */
 int adda_gb300_set_fft_shape(adda_gb300_ctx *ctx, int prec, const int shape[4]);
 
