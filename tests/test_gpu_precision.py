@@ -310,3 +310,49 @@ def test_block_sums_round(box):
     want = math.fsum((x.real ** 2).ravel())
     assert abs(ip[0] - want) <= 2.3e-16 * want
     c.close()
+
+
+# ---------------------------------------------------------------------------------------------------------------------
+# The fixed-point transforms at the ends of their range
+
+@pytest.mark.parametrize("n", [64, 256, 384, 400, 500, 512])
+@pytest.mark.parametrize("axis", [0, 1, 2])
+def test_coherent_input_on_a_long_axis(axis, n):
+    """constants and plane waves put a line's spectrum into one element, the largest growth of the forward transform (n / 2
+    terms of one sign: radices 16 x 16, 16 x 24, 20 x 25, 16 x 32, shifts of 2 and 3 bits); a single dipole has a flat
+    spectrum, the largest of the inverse ones (n terms). An overflow would be an error of the order of the result"""
+    from helpers import oracle_for, rel
+    box = [3, 2, 3]
+    box[axis] = n // 2
+    s = cube_setup(box, [2 * b for b in box])
+    s.cc = [s.cc[0]] * 2
+    o, c = oracle_for(s), context(s, R=6)
+    o.set_cc(s.cc[0].reshape(1, 3))
+    pol = np.array([1.0, 1.0j, -1.0])
+    along = s.pos[:, axis].astype(float)
+    x = [np.exp(2j * np.pi * f / n * along)[:, None] * pol for f in (0, n // 4, n // 2 - 1)]
+    for at in (0, n // 4, n // 2 - 1):
+        d = np.zeros((s.n, 3), complex)
+        d[np.flatnonzero(s.pos[:, axis] == at)[0]] = pol
+        x.append(d)
+    x = np.stack(x).reshape(6, -1)
+    for her in (False, True):
+        y = c.matvec(x, "fp64", her)[0]
+        for r in range(6):
+            assert rel(y[r], o.matvec(x[r], her)[0]) < 6e-15, (r, her)
+    o.close()
+    c.close()
+
+
+@pytest.mark.parametrize("box", [(32, 32, 32), (64, 45, 40), (100, 20, 16), (12, 125, 10)])
+@pytest.mark.parametrize("scale", [(1, 1, 1), (1, 1e-4, 1e-8), (1e-8, 1, 1e-4)])
+def test_fp64_matvec_to_rounding(box, scale):
+    """errors of twelve dipoles against a direct sum in extended precision, relative to the result's rms"""
+    s = full_box(box, 1.0)
+    c = context(s, R=1)
+    x = random_vec(s.n, 1, 17).reshape(s.n, 3) * np.array(scale)
+    y = c.matvec(x.reshape(1, -1), "fp64")[0].reshape(s.n, 3)
+    pick = np.random.default_rng(3).choice(s.n, 12, replace=False)
+    err = np.abs(y[pick] - matvec_direct(s, s.cc[0], x, pick)).astype(float)
+    assert np.sqrt((err ** 2).sum(1).mean() / (np.abs(y) ** 2).sum(1).mean()) < TOL
+    c.close()
