@@ -674,23 +674,27 @@ template <class A> inline Lines2<A> make_lines2(const adda_gb300_ctx *c)
 	}
 	return q;
 }
-// shared memory up to SMEM_CAP for a kernel (and its code on the device), once per kernel and device
-template <auto KERN> inline int l2_opt_in(const adda_gb300_ctx *c)
+// once per kernel and device: its code on the device (load), or shared memory up to SMEM_CAP where it wants more than near
+// the default limit (48 KB with the static part)
+template <auto KERN> inline int l2_opt_in(const adda_gb300_ctx *c, bool load)
 {
-	static std::atomic<unsigned long long> opted{0};
+	static std::atomic<unsigned long long> done[2]{};
 	const unsigned long long bit = 1ull << (c->device & 63);
-	if (!(opted.load(std::memory_order_acquire) & bit)) {
-		ADDA_CUDA(cudaFuncSetAttribute(KERN, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_CAP));
-		opted.fetch_or(bit, std::memory_order_release);
-	}
+	if (done[load].load(std::memory_order_acquire) & bit) return ADDA_GB300_OK;
+	cudaFuncAttributes a;
+	if (load) ADDA_CUDA(cudaFuncGetAttributes(&a, KERN));
+	else ADDA_CUDA(cudaFuncSetAttribute(KERN, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_CAP));
+	done[load].fetch_or(bit, std::memory_order_release);
 	return ADDA_GB300_OK;
 }
-// launch of a kernel; a grid without blocks (no RHS) only opts it in, at the context's creation (matvec_prepare)
+// launch of a kernel; a grid without blocks (no RHS) only loads and opts it in, at the context's creation (prepare_f64, matvec_setup_f32)
 template <auto KERN, typename... Ar>
 inline int l2_launch(const adda_gb300_ctx *c, dim3 g, int nt, size_t sm, cudaStream_t st, const Ar &...args)
 {
-	const int rc = l2_opt_in<KERN>(c);
-	if (rc || !(g.x && g.z)) return rc;
+	const bool none = !(g.x && g.z);
+	int rc = none ? l2_opt_in<KERN>(c, true) : ADDA_GB300_OK;
+	if (!rc && sm > 32 * 1024) rc = l2_opt_in<KERN>(c, false);
+	if (rc || none) return rc;
 	launch_next(KERN, g, dim3(nt), sm, st, args...);
 	ADDA_LAUNCHED();
 	return ADDA_GB300_OK;
