@@ -1,9 +1,11 @@
 // fft_lines2.cuh - two-pass transforms of lines whose length is a product of two register radices.
 //
-// A line of n = r1*r2 elements (radices up to 32 of the prime factors 2, 3, 5, 7, 11, 13, so nearly all sizes up to 512
-// that fftFit gives) is transformed as: element i = j + r2*t; thread j < r2 does DFT_r1 over t in registers, multiplies
+// A line of n = r1*r2 elements (radices up to 32 of the prime factors 2, 3, 5, 7, 11, 13) is transformed as: element i = j + r2*t; thread j < r2 does DFT_r1 over t in registers, multiplies
 // by W_n^(j*q) and leaves Y[q][j] in shared memory; thread q < r1 does DFT_r2 over j and holds X[q + r1*p]. One
-// exchange, whatever the radices; they are run-time numbers (block-uniform switches), so one kernel serves all sizes.
+// exchange, whatever the radices; they are run-time numbers (block-uniform switches), so one kernel serves all sizes. Of the
+// even lengths up to 512 that fftFit gives, FP32 has a plan for all but 490, fixed point, which has fewer radices above 16
+// (radix_built), for all but 242, 286, 294, 308, 330, 338, 364, 378, 390, 392, 396, 420, 440, 462, 468, 484, 486, 490 and 504:
+// one axis of those lengths, or above 512, leaves the FP64 matvec to FP64 instructions.
 //
 // Two arithmetics:
 //   Ar32  complex float.
@@ -13,9 +15,11 @@
 //         complex sum 4 against 152.
 //         Range: |component| < 2^FX_TOP on entry, so a sum of n terms stays below n*sqrt(2)*2^FX_TOP; the twiddles
 //         between the passes carry a factor 2^-fx_shift(n), which keeps the results below 2^62.5 and everything that
-//         is multiplied (at most half of a pass's terms) below 2^61.5, the bound of the products. Error: one unit is
-//         2^-56 of the block's largest value on entry and 2^-54 after the first pass, where the signal has grown by
-//         sqrt(r1): no more than the rounding of an FP64 transform.
+//         is multiplied (at most half of a pass's terms; two thirds in a radix-3 butterfly, whose products are real and
+//         have room for that) below 2^61.5, the bound of the products. Error: one unit is 2^-56 of the block's largest
+//         value on entry and 2^-(56 - fx_shift(n)) after the first pass (2^-54 up to 256 elements, 2^-53 up to 512), where
+//         the signal has grown by sqrt(r1), 4 and more there: no more than the rounding of an FP64 transform (1.6e-16 a
+//         matvec of a 128^3 sphere, both).
 #pragma once
 
 #include "common.cuh"

@@ -852,7 +852,7 @@ inline bool use_fx(const adda_gb300_ctx *c)
 {
 	return c->fx && c->shape[0].w1 == Tiles<double>::W1 && c->shape[0].w2 == Tiles<double>::W2;
 }
-// FP32: each stage whose axis has no compile-time kernel (those are faster: 256^3 0.68 ms) but a two-pass plan
+// FP32: each stage whose axis has no compile-time kernel (those are faster: 256^3 0.64 ms) but a two-pass plan
 inline bool use_l2_f32(const adda_gb300_ctx *c, int axis, int n) { return static_len(n) == 0 && c->p2[axis].r1 > 0; }
 inline bool use_l2_x(const adda_gb300_ctx *c, const MvShape &s) { return use_l2_f32(c, 0, c->gX) && s.w1 >= 4; }
 inline bool use_l2_z(const adda_gb300_ctx *c, const MvShape &s) { return use_l2_f32(c, 2, c->gZ) && s.w2 >= 8; }

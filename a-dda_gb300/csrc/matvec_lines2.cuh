@@ -1,6 +1,6 @@
 // matvec_lines2.cuh - the matvec's stages (K1, K2a, K2b, K2c, K3 of matvec_kernels.cuh) on the two-pass transforms of
-// fft_lines2.cuh: every FP64 matvec in 64-bit fixed point, and the FP32 matvec of axis lengths without compile-time
-// kernels. Data flow, buffers and their layouts are the same (fixed point: 16-byte complex integers in the place of
+// fft_lines2.cuh: the FP64 matvec in 64-bit fixed point where all three axes have plans for it (use_fx), and the FP32
+// matvec of axis lengths without compile-time kernels. Data flow, buffers and their layouts are the same (fixed point: 16-byte complex integers in the place of
 // double2).
 //
 // Fixed point: the data between two kernels are integers with an exponent per producing block (FxExp below), so that
@@ -9,11 +9,13 @@
 // bits OR-ed together by the producers, not from a worst case, so the growth of a transform costs no bits.
 //
 // Measured (one matvec): FP64 at grid 256^3, 2 RHS 19.21 ms with FP64 instructions (97 % of the FP64 pipe's rate) ->
-// 4.95 ms; FP32 at 192x154x112, 8 RHS 1.409 -> 0.83 ms, at 96^3 with per-dipole polarisabilities, 2 RHS 0.154 -> 0.089
-// ms, at 32^3, 1 RHS 36 -> 30 us (against the multi-pass transforms in shared memory with a run-time plan). Error
-// against 64 bits unchanged (FP64 1.6e-16). The fixed-point kernels are bound by instruction fetch and the integer
-// pipes (issue active 25-37 %, no_instruction the largest stall with long_scoreboard); 128 registers and 16 resident
-// warps an SM.
+// 4.95 ms; FP32 at 192x154x112, 8 RHS 1.409 -> 0.82 ms, at 96^3 with per-dipole polarisabilities, 2 RHS 0.154 -> 0.081
+// ms, at 32^3, 1 RHS 36 -> 20.7 us (against the multi-pass transforms in shared memory with a run-time plan and plain
+// launches). Error against 64 bits unchanged (FP64 1.6e-16).
+// The fixed-point kernels have 128 registers and 14-15 warps an SM, issue on 19-38 % of the cycles and wait for instruction
+// fetch (no instruction 2.0-2.3 per issue), global loads and, in the z transforms, the barrier between the passes. ptxas
+// reports 520 to 1480 bytes of spill stores for them, over the butterflies of all radices up to 16 that one kernel holds; of
+// the instructions a launch executes 0.04 to 0.9 % are spills.
 #pragma once
 
 #include "fft_lines2.cuh"

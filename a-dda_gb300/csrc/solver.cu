@@ -1361,7 +1361,8 @@ static int ensure_work(adda_gb300_ctx *c, int R, int hist_cap)
 // blocks per RHS of the vector kernels of one solve: FP64 vectors of small particles are bound by the FP64 pipes of the
 // SMs they reach, so they spread out, one element a thread (16^3 sphere, 2 RHS: an iteration 79 -> 68 us); the others
 // take four elements a thread, which amortises the block's coefficients and sums (32^3 cube adjoint solve: 25.0 ms
-// against 26.7)
+// against 26.7). At most 152 * 4 blocks: with 152 * 8 no method was faster (seven methods, FP64, mixed and FP32 vectors, 64^3
+// to 128^3 spheres: 0.98 to 1.00 of the speed)
 static int vector_blocks(size_t n3, bool fp64)
 {
 	const size_t per = fp64 ? NT : 4 * NT;
