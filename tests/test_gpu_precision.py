@@ -356,3 +356,20 @@ def test_fp64_matvec_to_rounding(box, scale):
     err = np.abs(y[pick] - matvec_direct(s, s.cc[0], x, pick)).astype(float)
     assert np.sqrt((err ** 2).sum(1).mean() / (np.abs(y) ** 2).sum(1).mean()) < TOL
     c.close()
+
+
+@pytest.mark.parametrize("n", [9, 15, 21, 25, 27, 35, 49, 63, 77, 105, 121, 125, 143, 169, 195, 225, 243, 315, 375])
+def test_odd_x_grids(n):
+    """an x axis of 2 boxX - 1 points: the two-pass transforms' zero half is a point short of half the line"""
+    from helpers import oracle_for, rel
+    s = cube_setup(((n + 1) // 2, 3, 2), (n, 6, 4))
+    s.cc = [s.cc[0]] * 2
+    o, c = oracle_for(s), context(s, R=2)
+    o.set_cc(s.cc[0].reshape(1, 3))
+    x = random_vec(s.n, 2, n)
+    for prec, tol in (("fp64", 6e-15), ("fp32", 5e-6)):
+        y = c.matvec(x, prec)[0]
+        for r in range(2):
+            assert rel(y[r], o.matvec(x[r])[0]) < tol
+    o.close()
+    c.close()
