@@ -354,7 +354,7 @@ int scattered_fields(adda_gb300_ctx *c, int R, int ndir, const double *dirs, dou
 	const size_t rows = (size_t)c->bX + c->bY + c->bZ;
 	// directions per launch: the tables' budget, a multiple of 32 within the grid's limit
 	const int per = (int)std::max<size_t>(32, std::min<size_t>(32768, FLD_TABLE / (rows * sizeof(int4)) / 32 * 32));
-	const int ld = std::min(per, (ndir + 31) / 32 * 32), groups = ld / 32;
+	const int ld = std::min(per, few ? ndir : (ndir + 31) / 32 * 32), groups = ld / 32;
 	// ranges of dipoles: three waves of resident warps (lines of different length even out); where few directions leave the
 	// chip emptier than that, sqrt(N / 16) dipoles each, at least 16: a dipole costs a lone warp 0.44 us (latency), a range
 	// 0.025 us in fld_finish. Measured with 33 to 80 directions (sum and finish, ranges of 256 -> this): 16x8x8 box 119 ->

@@ -373,3 +373,27 @@ def test_odd_x_grids(n):
             assert rel(y[r], o.matvec(x[r])[0]) < tol
     o.close()
     c.close()
+
+
+@pytest.mark.parametrize("method", ["bicg", "cgnr", "csym", "qmr2", "bcgs2"])
+@pytest.mark.parametrize("grid", [6, 10, 16])
+def test_other_methods_of_few_and_many_blocks(method, grid):
+    """vector kernels of one block, a few and dozens per right-hand side, scalar steps in the last block or as kernels: several
+    right-hand sides of different scale converge independently to the oracle's solution"""
+    from oracle import oracle as O
+
+    from helpers import oracle_for, rel, setup_for
+    s = setup_for(dict(grid=grid, m=1.3 + 0.1j, dpl=10))
+    o, c = oracle_for(s), context(s, R=3)
+    scale = [1.0, 1e-30, 1e30]
+    for r in range(3):
+        c.set_cc(r, s.cc[0].reshape(1, 3))
+    o.set_cc(s.cc[0].reshape(1, 3))
+    want = o.solve(s.einc[0], method=O.QMR_CS, eps=1e-11)["p"]
+    res = c.solve(np.stack([s.einc[0] * k for k in scale]), method=method, prec="fp64", eps=1e-11)
+    for r in range(3):
+        assert res["stats"][r]["status"] == "ok", (r, res["stats"][r])
+        # the relative error is at most the condition number (below 10 for m = 1.3) times the residual
+        assert rel(res["p"][r] / scale[r], want) < 1e-9
+    o.close()
+    c.close()
