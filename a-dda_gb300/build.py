@@ -64,7 +64,7 @@ def build(force=False, verbose=False, out=None, defines=()):
     for f in CU:
         o = os.path.join(out_dir, f + ".o")
         objs.append(o)
-        # compressed for speed: the driver unpacks the kernels when a process makes its first context, which took 128 ms
+        # compressed for speed: CUDA unpacks the kernels when a process makes its first context, which took 128 ms
         # with the default compression against 101 (uncompressed 79, but a library of 135 MB against 52)
         jobs.append([nv, "-c", os.path.join(CSRC, f), "-o", o, "-std=c++17", "-O3", "-lineinfo", "--compress-mode=speed", *ARCH,
                      "-Xcompiler", "-fPIC", "-I", INCLUDE, "-I", CSRC, "--expt-relaxed-constexpr",
